@@ -41,7 +41,7 @@ static __device__ __constant__ cplx c_swap[16] = {{1, 0}, {0, 0}, {0, 0}, {0, 0}
                                            {0, 0}, {1, 0}, {0, 0}, {0, 0}, {0, 0}, {0, 0}, {0, 0}, {1, 0}};
 
 // apply_local_gate_exact! on sites (s1, s1+1).
-static __device__ void tebd_apply(Ctx& c, const DState& s, const cplx* op, int s1) {
+static __device__ __noinline__ void tebd_apply(Ctx& c, const DState& s, const cplx* op, int s1) {
   ProfScope prof_scope_(PF_SWEEP);
   shift_oc(c, s, s1);
   if (c.sm.fail) return;
@@ -62,7 +62,7 @@ static __device__ void tebd_apply(Ctx& c, const DState& s, const cplx* op, int s
 }
 
 // apply_window! with method :TEBD (DigitalTJM.jl:307-334).
-static __device__ void apply_window_tebd(Ctx& c, const DState& s, const DevGate& g) {
+static __device__ __noinline__ void apply_window_tebd(Ctx& c, const DState& s, const DevGate& g) {
   if (g.b > g.a + 1) {
     for (int k = g.b - 1; k >= g.a + 1 && !c.sm.fail; --k) tebd_apply(c, s, c_swap, k);
     if (!c.sm.fail) tebd_apply(c, s, g.mat, g.a);
@@ -78,7 +78,7 @@ static __device__ void apply_window_tebd(Ctx& c, const DState& s, const DevGate&
 // sweep (_tdvp_sweep_circuit_2site!, Algorithms.jl:606-627): each pair by +1
 // with the right site back-evolved by -1 (:631-672), the last pair by +1
 // split to the right (:762-800); the centre ends on b.
-static __device__ void apply_window_tdvp(Ctx& c, const DState& s, const DevGate& g, const WMat* wm) {
+static __device__ __noinline__ void apply_window_tdvp(Ctx& c, const DState& s, const DevGate& g, const WMat* wm) {
   const int s1 = g.a, s2 = g.b, n = s2 - s1 + 1;
   const WMat* h1 = wm;
   const WMat* h2 = wm + n;
@@ -111,7 +111,7 @@ static __device__ void apply_window_tdvp(Ctx& c, const DState& s, const DevGate&
 // dissipator needs a two-site split, every operation of the reference sweeps
 // away from the gate's sites is a gauge move, and only the gate's sites are
 // visited; otherwise the reference sweeps run as they are.
-static __device__ void digital_noise(Ctx& c, const DState& s, int s1, int s2) {
+static __device__ __noinline__ void digital_noise(Ctx& c, const DState& s, int s1, int s2) {
   ProfScope prof_scope_(PF_STOCH);
   const DevParams& P = c.P;
   int nloc = 0;
@@ -290,7 +290,7 @@ static __device__ void digital_noise(Ctx& c, const DState& s, int s1, int s2) {
 // Launch 0: initial state, normalisation and the start sample; launch l >= 1:
 // layer l-1 (its 1-qubit gates first, then each 2-qubit gate followed by the
 // noise step) and the sample after it.
-static __device__ void run_digital_step(Ctx& c, const DigParams& D, int launch) {
+static __device__ __noinline__ void run_digital_step(Ctx& c, const DigParams& D, int launch) {
   ProfScope prof_scope_(PF_STEP);
   const DevParams& P = c.P;
   const int L = P.L;

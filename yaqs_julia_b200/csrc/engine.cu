@@ -38,7 +38,8 @@ __global__ void __launch_bounds__(NT, 2) tjm_step_kernel(const DevParams P, int 
 
 // Digital TJM: position 0 prepares every trajectory, position l >= 1 applies
 // layer l-1 of the circuit (run_digital_tjm, DigitalTJM.jl:363-450).
-__global__ void __launch_bounds__(NT, 2) digital_step_kernel(const DevParams P, const DigParams D, int first,
+__global__ void __launch_bounds__(NT, 2) digital_step_kernel(const DevParams P,
+                                                             const DigParams D, int first,
                                                              int count) {
   extern __shared__ __align__(16) unsigned char smraw[];
   CtaSmem& sm = *reinterpret_cast<CtaSmem*>(align_smem_1024(smraw));

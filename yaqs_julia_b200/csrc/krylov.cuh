@@ -161,7 +161,9 @@ union EngineSmemU {
     WApplySmem w;
   } gw;
   cplx svd[SVD_SMEM_CPLX_K];
+#if YAQS_TC
   TcSmem t;  // the tensor-core pipeline (mixed form), no larger than the GEMM staging
+#endif
 };
 struct EngineSmem {
   RedScratch r;
@@ -169,7 +171,7 @@ struct EngineSmem {
   TcState tc;
   EngineSmemU u;
 };
-#if !YAQS_TC
+#if YAQS_TC
 static_assert(sizeof(TcSmem) <= sizeof(GemmSmem), "the default pipeline must not grow the CTA's shared memory");
 #endif
 
@@ -305,7 +307,7 @@ struct KrylovCfg {
 };
 
 // Warp 0: y = exp(-i dt T) e_1 for the m x m Lanczos matrix in ks.
-static __device__ void dev_tridiag_expm(int m, double dt, KrySmem& ks) {
+static __device__ __noinline__ void dev_tridiag_expm(int m, double dt, KrySmem& ks) {
   ProfScope prof_scope_(PF_TRIDIAG);
   if (ltid() >= 32) return;
   const int j = ltid();

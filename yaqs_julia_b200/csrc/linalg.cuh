@@ -239,7 +239,7 @@ struct SvdResult {
 };
 
 // Orthonormal completion of column k of Y (rows x *) against columns 0..k-1.
-static __device__ void dev_complete_column(cplx* Y, int rows, int k, cplx* y, RedScratch& rs) {
+static __device__ __noinline__ void dev_complete_column(cplx* Y, int rows, int k, cplx* y, RedScratch& rs) {
   for (int c = 0; c < rows; ++c) {
     // pass 1: y = e_c - sum_h conj(Y_h[c]) Y_h
     for (int i = ltid(); i < rows; i += NT) {

@@ -7,7 +7,7 @@
 // ---------------------------------------------------------------------------
 // Device program
 // ---------------------------------------------------------------------------
-static __device__ void copy_state(Ctx& c, const DState& dst, const DState& src) {
+static __device__ __noinline__ void copy_state(Ctx& c, const DState& dst, const DState& src) {
   ProfScope prof_scope_(PF_COPY);
   cta_copy(dst.a, src.a, c.P.mps_size);
   for (int b = ltid(); b <= c.P.L; b += NT) dst.chi[b] = src.chi[b];
@@ -15,7 +15,7 @@ static __device__ void copy_state(Ctx& c, const DState& dst, const DState& src) 
   cta_sync();
 }
 
-static __device__ void sample(Ctx& c, const DState& phi, const DState& psi, int col) {
+static __device__ __noinline__ void sample(Ctx& c, const DState& phi, const DState& psi, int col) {
   copy_state(c, psi, phi);
   tdvp_sweep(c, psi);
   if (c.sm.fail) return;
@@ -26,7 +26,7 @@ static __device__ void sample(Ctx& c, const DState& phi, const DState& psi, int 
   evaluate(c, psi, col);
 }
 
-static __device__ void run_step(Ctx& c, int j) {
+static __device__ __noinline__ void run_step(Ctx& c, int j) {
   ProfScope prof_scope_(PF_STEP);
   const DevParams& P = c.P;
   const int L = P.L;
@@ -79,7 +79,7 @@ static __device__ void run_step(Ctx& c, int j) {
 // executing it, so the wait always ends; it is still bounded (about 100 s)
 // and gives up with ST_TIMEOUT.
 #define DONE_WAIT_POLLS 100000000LL
-static __device__ bool wait_done(const DevParams& P, int t, int need, CtaSmem& sm) {
+static __device__ __noinline__ bool wait_done(const DevParams& P, int t, int need, CtaSmem& sm) {
   if (ltid() == 0) {
     volatile int* d = P.done + t;
     int ok = 0;

@@ -202,7 +202,7 @@ static __device__ void set_chi(Ctx& c, const DState& s, int b, int v) {
 }
 
 // site i: A = Q R, Q -> site i, R absorbed into site i+1.
-static __device__ void qr_right(Ctx& c, const DState& s, int i) {
+static __device__ __noinline__ void qr_right(Ctx& c, const DState& s, int i) {
   const int l = s.chi[i], r = s.chi[i + 1], m = 2 * l, rn = min(m, r);
   const int r2 = s.chi[i + 2];
   cplx* A = site_ptr(c, s, i);
@@ -221,7 +221,7 @@ static __device__ void qr_right(Ctx& c, const DState& s, int i) {
 }
 
 // site i: A = L Q, Q -> site i, L absorbed into site i-1.
-static __device__ void lq_left(Ctx& c, const DState& s, int i) {
+static __device__ __noinline__ void lq_left(Ctx& c, const DState& s, int i) {
   const int l = s.chi[i], r = s.chi[i + 1], n2 = 2 * r, rn = min(l, n2);
   const int lp = s.chi[i - 1];
   cplx* A = site_ptr(c, s, i);
@@ -247,7 +247,7 @@ static __device__ void lq_left(Ctx& c, const DState& s, int i) {
   set_chi(c, s, i, rn);
 }
 
-static __device__ void shift_oc(Ctx& c, const DState& s, int nc) {
+static __device__ __noinline__ void shift_oc(Ctx& c, const DState& s, int nc) {
   int oc = *s.oc;
   cta_sync();
   if (oc == nc) return;
@@ -261,7 +261,7 @@ static __device__ void shift_oc(Ctx& c, const DState& s, int nc) {
   cta_sync();
 }
 
-static __device__ void normalize_state(Ctx& c, const DState& s) {
+static __device__ __noinline__ void normalize_state(Ctx& c, const DState& s) {
   for (int i = c.P.L - 1; i >= 1 && !c.sm.fail; --i) lq_left(c, s, i);
   cplx* A = site_ptr(c, s, 0);
   const long long n = (long long)s.chi[0] * 2 * s.chi[1];
@@ -305,7 +305,7 @@ static __device__ void finish_normalize(Ctx& c, const DState& s) {
 }
 
 // Re <psi|psi> by full contraction (scalar_product, MPS.jl:528-585).
-static __device__ double scalar_product(Ctx& c, const DState& s) {
+static __device__ __noinline__ double scalar_product(Ctx& c, const DState& s) {
   ProfScope prof_scope_(PF_SCALAR);
   cplx* Ea = c.ws + c.P.lay.tA;
   cplx* Eb = c.ws + c.P.lay.tB;
@@ -342,7 +342,7 @@ static __device__ void identity_env(Ctx& c, cplx* E, int dim, int w) {
 }
 
 // EL[i+1] from EL[i], A_i and the map Wenv of W_i (update_left_environment)
-static __device__ void update_left_w(Ctx& c, const DState& s, int i, const WMat& Wenv) {
+static __device__ __noinline__ void update_left_w(Ctx& c, const DState& s, int i, const WMat& Wenv) {
   ProfScope prof_scope_(PF_ENV);
   const int l = s.chi[i], r = s.chi[i + 1], wl = c.P.w[i], wr = c.P.w[i + 1];
   const cplx* A = site_ptr(c, s, i);
@@ -389,7 +389,7 @@ static __device__ void update_left_w(Ctx& c, const DState& s, int i, const WMat&
 static __device__ void update_left(Ctx& c, const DState& s, int i) { update_left_w(c, s, i, c.P.wm_envL[i]); }
 
 // ER[i] from ER[i+1], A_i and the map Wenv of W_i (update_right_environment)
-static __device__ void update_right_w(Ctx& c, const DState& s, int i, const WMat& Wenv) {
+static __device__ __noinline__ void update_right_w(Ctx& c, const DState& s, int i, const WMat& Wenv) {
   ProfScope prof_scope_(PF_ENV);
   const int l = s.chi[i], r = s.chi[i + 1], wl = c.P.w[i], wr = c.P.w[i + 1];
   const cplx* A = site_ptr(c, s, i);
@@ -502,7 +502,7 @@ static __device__ HeffOp make_heff(Ctx& c, int l, int D, int r, int bl, int br, 
   return h;
 }
 
-static __device__ void evolve(Ctx& c, cplx* x, int l, int D, int r, int bl, int br, const WMat& W, double dt) {
+static __device__ __noinline__ void evolve(Ctx& c, cplx* x, int l, int D, int r, int bl, int br, const WMat& W, double dt) {
   const HeffOp h = make_heff(c, l, D, r, bl, br, W);
   int mv = dev_expm_krylov(h, x, dt, c.P.kc, c.ws + c.P.lay.Q, c.P.kry_n, c.sm.e);
   if (ltid() == 0) {
@@ -513,7 +513,7 @@ static __device__ void evolve(Ctx& c, cplx* x, int l, int D, int r, int bl, int 
 }
 
 // Theta (l,4,r) of sites i,i+1 into buffer th.
-static __device__ void merge(Ctx& c, const DState& s, int i, cplx* th) {
+static __device__ __noinline__ void merge(Ctx& c, const DState& s, int i, cplx* th) {
   const int l = s.chi[i], m = s.chi[i + 1], r = s.chi[i + 2];
   cta_gemm(gemm_args(2 * l, 2 * r, m, site_ptr(c, s, i), 1, 2 * l, site_ptr(c, s, i + 1), 1, m, th, 1, 2 * l),
            c.sm.e.u.gw.g);
@@ -551,7 +551,7 @@ static __device__ void fix_nonfinite(Ctx& c, cplx* th, long long n) {
 // otherwise right (U | S Vt, U orthonormal, Algorithms.jl:656-663).  The
 // scaled factor is computed as a product with theta and is exactly zero for
 // null singular values.
-static __device__ void split(Ctx& c, const DState& s, int i, cplx* th, int l, int r, int rule, bool s_left) {
+static __device__ __noinline__ void split(Ctx& c, const DState& s, int i, cplx* th, int l, int r, int rule, bool s_left) {
   const int m = 2 * l, n = 2 * r;
   fix_nonfinite(c, th, (long long)m * n);
   SvdWork w = svd_work(c);
@@ -598,7 +598,7 @@ static __device__ void split(Ctx& c, const DState& s, int i, cplx* th, int l, in
 }
 
 // _init_envs (Algorithms.jl:802-819) after moving the centre to site 0.
-static __device__ void init_envs(Ctx& c, const DState& s) {
+static __device__ __noinline__ void init_envs(Ctx& c, const DState& s) {
   const int L = c.P.L;
   shift_oc(c, s, 0);
   identity_env(c, envR(c, L), s.chi[L], c.P.w[L]);
@@ -613,7 +613,7 @@ static __device__ void evolve_bond(Ctx& c, cplx* C, int k, int r, int b, double 
 
 // Site i = Q R (thin QR): Q -> site i, EL[i+1] from it, R evolved by dtb on
 // bond i+1 and absorbed into site i+1 (Algorithms.jl:491-505).
-static __device__ void qr_bond_forward(Ctx& c, const DState& s, int i, double dtb) {
+static __device__ __noinline__ void qr_bond_forward(Ctx& c, const DState& s, int i, double dtb) {
   const int l = s.chi[i], r = s.chi[i + 1], m = 2 * l, rn = min(m, r);
   const int r2 = s.chi[i + 2];
   cplx* A = site_ptr(c, s, i);
@@ -637,7 +637,7 @@ static __device__ void qr_bond_forward(Ctx& c, const DState& s, int i, double dt
 
 // Site i = L Q (thin LQ): Q -> site i, ER[i] from it, L evolved by dtb on
 // bond i and absorbed into site i-1 (Algorithms.jl:515-529).
-static __device__ void lq_bond_backward(Ctx& c, const DState& s, int i, double dtb) {
+static __device__ __noinline__ void lq_bond_backward(Ctx& c, const DState& s, int i, double dtb) {
   const int l = s.chi[i], r = s.chi[i + 1], n2 = 2 * r, rn = min(l, n2);
   const int lp = s.chi[i - 1];
   cplx* A = site_ptr(c, s, i);
@@ -676,7 +676,7 @@ static __device__ void evolve_site1(Ctx& c, const DState& s, int i, double dts) 
 }
 
 // _tdvp_sweep_hamiltonian_1site! (Algorithms.jl:472-533).
-static __device__ void tdvp_sweep_1site(Ctx& c, const DState& s) {
+static __device__ __noinline__ void tdvp_sweep_1site(Ctx& c, const DState& s) {
   const int L = c.P.L;
   const double dt = c.P.dt;
   init_envs(c, s);
@@ -698,7 +698,7 @@ static __device__ void tdvp_sweep_1site(Ctx& c, const DState& s) {
 // keeping min(rank, max_bond_dim) values), a 1-site update with bond
 // back-evolution once it has reached it; once a 1-site step reaches the
 // last bond the last site (first site on the way back) is updated alone.
-static __device__ void tdvp_sweep_dynamic(Ctx& c, const DState& s) {
+static __device__ __noinline__ void tdvp_sweep_dynamic(Ctx& c, const DState& s) {
   const int L = c.P.L;
   const double dt = c.P.dt;
   cplx* th = c.ws + c.P.lay.th;
@@ -747,7 +747,7 @@ static __device__ void tdvp_sweep_dynamic(Ctx& c, const DState& s) {
   cta_sync();
 }
 
-static __device__ void tdvp_sweep_2site(Ctx& c, const DState& s) {
+static __device__ __noinline__ void tdvp_sweep_2site(Ctx& c, const DState& s) {
   const int L = c.P.L;
   const double dt = c.P.dt;
   cplx* th = c.ws + c.P.lay.th;
@@ -826,7 +826,7 @@ static __device__ double local_norm2(Ctx& c, const cplx* A, int l, int d, int r,
 }
 
 // Re sum conj(A) (op A)
-static __device__ double local_expect(Ctx& c, const cplx* A, int l, int d, int r, const cplx* op) {
+static __device__ __noinline__ double local_expect(Ctx& c, const cplx* A, int l, int d, int r, const cplx* op) {
   double sacc = 0.0;
   for (int e = ltid(); e < l * r; e += NT) {
     long long a = e % l, b = e / l;
@@ -853,7 +853,7 @@ static __device__ __forceinline__ bool proc_on(const DevProc& pr, int f1, int f2
   return pr.nsites == 1 ? (pr.s0 == f1 || pr.s0 == f2) : ((pr.s0 == f1 && pr.s1 == f2) || (pr.s0 == f2 && pr.s1 == f1));
 }
 
-static __device__ void apply_dissipation(Ctx& c, const DState& s, bool full, double dt, int f1 = -1, int f2 = -1) {
+static __device__ __noinline__ void apply_dissipation(Ctx& c, const DState& s, bool full, double dt, int f1 = -1, int f2 = -1) {
   ProfScope prof_scope_(PF_DISS);
   const int L = c.P.L;
   bool all_zero = c.P.all_zero != 0;
@@ -932,7 +932,7 @@ static __device__ void apply_dissipation(Ctx& c, const DState& s, bool full, dou
 // ---------------------------------------------------------------------------
 // Stochastic process (StochasticProcess.jl:219-330)
 // ---------------------------------------------------------------------------
-static __device__ void stochastic_process(Ctx& c, const DState& s, double dt, int f1 = -1, int f2 = -1) {
+static __device__ __noinline__ void stochastic_process(Ctx& c, const DState& s, double dt, int f1 = -1, int f2 = -1) {
   ProfScope prof_scope_(PF_STOCH);
   const int L = c.P.L;
   const double dp = 1.0 - scalar_product(c, s);
@@ -1073,7 +1073,7 @@ static __device__ double env_expect(Ctx& c, const cplx* A, const cplx* T, int l,
 // sweeps) or else in the SVD scratch (B, X, Yo, Zo, adjacent); returns false,
 // having written nothing, when no observable is 1-site, the chain is not
 // tight, or neither region holds them.  CTA-collective.
-static __device__ bool local_by_envs(Ctx& c, const DState& s, int col) {
+static __device__ __noinline__ bool local_by_envs(Ctx& c, const DState& s, int col) {
   const DevParams& P = c.P;
   const int L = P.L;
   bool any1 = false;
@@ -1144,7 +1144,7 @@ static __device__ bool local_by_envs(Ctx& c, const DState& s, int col) {
   return true;
 }
 
-static __device__ void evaluate(Ctx& c, const DState& s, int col) {
+static __device__ __noinline__ void evaluate(Ctx& c, const DState& s, int col) {
   ProfScope prof_scope_(PF_EVAL);
   const int ncols = c.P.ncols;
   const bool local_done = local_by_envs(c, s, col);
