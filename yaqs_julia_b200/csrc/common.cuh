@@ -97,6 +97,29 @@ static __device__ __forceinline__ double warp_max(double v) {
   return v;
 }
 
+// Warp sums of NV (a power of two) values at once: at each of the first
+// log2(NV) butterfly steps a lane keeps half of its values and hands the
+// others to its partner, so 16 values take 16 shuffles instead of 80.  Every
+// sum adds the same pairs in the same tree as warp_sum, bit for bit.  Lane l
+// ends with the sum of value l >> (5 - log2(NV)) in x[0].
+template <int NV>
+static __device__ __forceinline__ void warp_sum_multi(double (&x)[NV]) {
+  const int lane = ltid() & 31;
+  int o = 16;
+#pragma unroll
+  for (int n = NV; n > 1; n >>= 1) {
+    const bool up = (lane & o) != 0;
+#pragma unroll
+    for (int k = 0; k < n / 2; ++k) {
+      const double keep = up ? x[k + n / 2] : x[k], give = up ? x[k] : x[k + n / 2];
+      x[k] = keep + __shfl_xor_sync(0xffffffffu, give, o);
+    }
+    o >>= 1;
+  }
+#pragma unroll
+  for (; o > 0; o >>= 1) x[0] += __shfl_xor_sync(0xffffffffu, x[0], o);
+}
+
 // Shared scratch used by the reductions (NW*16+16 doubles).
 struct RedScratch {
   double v[NW * 16 + 16];
@@ -111,11 +134,16 @@ struct RedScratch {
 template <int NV>
 static __device__ __forceinline__ void block_sum_n(double (&x)[NV], RedScratch& rs) {
   const int lane = ltid() & 31, wid = ltid() >> 5;
+  if (NV == 16) {
+    warp_sum_multi<NV>(x);
+    if ((lane & 1) == 0) rs.v[wid * NV + (lane >> 1)] = x[0];
+  } else {
 #pragma unroll
-  for (int k = 0; k < NV; ++k) x[k] = warp_sum(x[k]);
-  if (lane == 0) {
+    for (int k = 0; k < NV; ++k) x[k] = warp_sum(x[k]);
+    if (lane == 0) {
 #pragma unroll
-    for (int k = 0; k < NV; ++k) rs.v[wid * NV + k] = x[k];
+      for (int k = 0; k < NV; ++k) rs.v[wid * NV + k] = x[k];
+    }
   }
   cta_sync();
   if (NV <= 4) {

@@ -306,7 +306,15 @@ struct KrylovCfg {
   double exit_tol;
 };
 
-// Warp 0: y = exp(-i dt T) e_1 for the m x m Lanczos matrix in ks.
+// Warp 0: y = exp(-i dt T) e_1 for the m x m Lanczos matrix in ks, by Taylor
+// series over substeps of norm <= 1/2, each stopped after the first term with
+// |term|^2 < 1e-40.
+//
+// One serial chain on one warp while the others wait (12-31 % of a small
+// chain's step when every term ended in a warp reduction and a division), so
+// terms go in groups of four: their sizes are reduced together, the first
+// small one is found by a ballot and the sum up to it is taken.  h / n comes
+// from a table filled once.
 static __device__ __noinline__ void dev_tridiag_expm(int m, double dt, KrySmem& ks) {
   ProfScope prof_scope_(PF_TRIDIAG);
   if (ltid() >= 32) return;
@@ -320,25 +328,50 @@ static __device__ __noinline__ void dev_tridiag_expm(int m, double dt, KrySmem& 
   int ns = (int)ceil(tn / 0.5);
   if (ns < 1) ns = 1;
   const double h = dt / ns;
+  double* rcp = reinterpret_cast<double*>(ks.y);  // h / n; y is written at the end
+  rcp[j] = h / j;
+  rcp[32 + j] = h / (32 + j);
+  __syncwarp();
   cplx v = make_double2(j == 0 ? 1.0 : 0.0, 0.0);
   for (int s = 0; s < ns; ++s) {
     cplx term = v, acc = v;
-    for (int n = 1; n < 60; ++n) {
-      // term <- (-i h T) term / n
-      cplx tl = make_double2(__shfl_up_sync(0xffffffffu, term.x, 1), __shfl_up_sync(0xffffffffu, term.y, 1));
-      cplx tr = make_double2(__shfl_down_sync(0xffffffffu, term.x, 1), __shfl_down_sync(0xffffffffu, term.y, 1));
-      cplx tt = make_double2(a * term.x + bl * tl.x + br * tr.x, a * term.y + bl * tl.y + br * tr.y);
-      if (!on) tt = make_double2(0.0, 0.0);
-      // multiply by -i h / n:  (x + i y) * (-i c) = c y - i c x
-      const double c = h / n;
-      term = make_double2(c * tt.y, -c * tt.x);
-      acc = cadd(acc, term);
-      double tnorm = warp_sum(cabs2(term));
-      if (tnorm < 1e-40) break;
+    for (int n0 = 1; n0 < 60; n0 += 4) {
+      cplx at[4];
+      double size[4];
+#pragma unroll
+      for (int u = 0; u < 4; ++u) {
+        // term <- (-i h T) term / n
+        cplx tl = make_double2(__shfl_up_sync(0xffffffffu, term.x, 1), __shfl_up_sync(0xffffffffu, term.y, 1));
+        cplx tr = make_double2(__shfl_down_sync(0xffffffffu, term.x, 1), __shfl_down_sync(0xffffffffu, term.y, 1));
+        cplx tt = make_double2(a * term.x + bl * tl.x + br * tr.x, a * term.y + bl * tl.y + br * tr.y);
+        if (!on) tt = make_double2(0.0, 0.0);
+        // multiply by -i h / n:  (x + i y) * (-i c) = c y - i c x
+        const double c = rcp[n0 + u];
+        term = make_double2(c * tt.y, -c * tt.x);
+        acc = cadd(acc, term);
+        at[u] = acc;
+        size[u] = cabs2(term);
+      }
+      warp_sum_multi<4>(size);  // lane l holds the size of term l / 8 of the group
+      const unsigned small = __ballot_sync(0xffffffffu, size[0] < 1e-40);
+      if (small) {
+        const int u = (__ffs(small) - 1) >> 3;
+        acc = u == 0 ? at[0] : u == 1 ? at[1] : u == 2 ? at[2] : at[3];
+        break;
+      }
+      if (n0 == 57) acc = at[2];  // 59 terms at most
     }
     v = acc;
   }
+  __syncwarp();
   if (on) ks.y[j] = v;
+}
+
+// v - c a, its roundings spelled out so that every path subtracts a basis
+// vector with the same bits.
+static __device__ __forceinline__ cplx csub_mul(cplx v, cplx c, cplx a) {
+  return make_double2(__dsub_rn(v.x, __fma_rn(c.x, a.x, -__dmul_rn(c.y, a.y))),
+                      __dsub_rn(v.y, __fma_rn(c.y, a.x, __dmul_rn(c.x, a.y))));
 }
 
 // h_j = <q_j, w> (j < k) into ks.h and |w|^2 in the same pass over w: the
@@ -407,8 +440,8 @@ static __device__ double basis_combine(const cplx* Q, long long qs, const cplx* 
       for (int e = 0; e < 8; ++e) {
         if (j0 + e < k) {
           const cplx ce = c[j0 + e];
-          v0 = csub(v0, cmul(ce, a0[e]));
-          v1 = csub(v1, cmul(ce, a1[e]));
+          v0 = csub_mul(v0, ce, a0[e]);
+          v1 = csub_mul(v1, ce, a1[e]);
         }
       }
     }
@@ -431,10 +464,263 @@ static __device__ double lanczos_subtract(const cplx* Q, long long qs, cplx* w, 
   return basis_combine(Q, qs, w, w, n, k, sm.k.h, 1.0, norm, sm);
 }
 
+// ---------------------------------------------------------------------------
+// Small problems: the whole Krylov solve in shared memory
+// ---------------------------------------------------------------------------
+// A solve on n = chil D chir <= SMALL_N values is bound by latency, not by
+// work: every H_eff product of the general path stages 64-wide tiles of
+// operands that fill a corner of one, and its dot products read vectors that
+// another thread has just written through L2.  Here the environments, the
+// intermediates and as many Krylov vectors as fit live in the CTA's staging
+// buffer, the products run on 8 x 8 blocks dealt to the warps straight from
+// it, and a Lanczos step takes seven barriers instead of about thirty.
+// Every sum is formed in the general path's order (four-deep MMA steps from
+// k = 0, the same reduction trees), so both give the same bits: where a
+// 2-site sweep truncates between equal Schmidt values, rounding decides, and
+// a chain must not change its records by crossing this limit.
+// SMALL_N is one value per thread; wider solves fill the tiles of the general
+// path.  Measured with the sweep on L = 6 Ising, chi 16, 200 trajectories, 51
+// time indices: 445 ms with the general path alone, 268 ms with this one.
+#define SMALL_N 256
+#define SMALL_MIN_VECS 4  // Krylov vectors that have to fit beside the operands
+
+struct SmallPlan {
+  int oR, oT1, oT2, oVal, oIdx, oRed, oQ;  // offsets in the buffer; L at 0
+  int nfit;                                // Krylov vectors held in the buffer
+};
+
+static __device__ __forceinline__ bool small_plan(const HeffOp& h, SmallPlan& p) {
+  const int n = h.chil * h.D * h.chir;
+  if (n > SMALL_N || h.mixed || h.W.no * h.chil * h.chir > 8 * SMALL_N) return false;
+  const int cap = (int)(sizeof(EngineSmemU) / sizeof(cplx));
+  int off = h.chil * h.wl * h.chil;
+  p.oR = off;
+  off += h.chir * h.wr * h.chir;
+  p.oT1 = off;
+  off += h.chil * h.wl * h.D * h.chir;
+  p.oT2 = p.oT1;  // in place: with wl == wr a pair's inputs and outputs share their addresses
+  if (h.wl != h.wr) {
+    p.oT2 = off;
+    off += h.chil * h.wr * h.D * h.chir;
+  }
+  p.oVal = off;
+  off += h.W.ident ? 0 : h.W.nnz;
+  p.oIdx = off;  // row pointers, then columns
+  off += h.W.ident ? 0 : (h.W.no + 1 + h.W.nnz + 3) / 4;
+  p.oRed = off;
+  off += 5 * NW * 8;  // 16 partial sums of each warp for five groups of vectors (33 sums)
+  p.oQ = off;
+  p.nfit = (cap - off) / n;
+  return cap > off && p.nfit >= SMALL_MIN_VECS;
+}
+
+// C(M x N) = A B from shared memory: A (m,k) at A[m + k ak], B (k,n) at
+// B[k bk + n bn], C (m,n) at C[m + n M].  Warps take 8 x 8 blocks.
+static __device__ __forceinline__ void small_gemm(int M, int N, int K, const cplx* A, int ak, const cplx* B, int bk,
+                                                  int bn, cplx* C) {
+  const int lane = ltid() & 31, wid = ltid() >> 5;
+  const int gq = lane >> 2, tq = lane & 3;
+  const int mb = (M + 7) >> 3, nb = (N + 7) >> 3;
+  for (int q = wid; q < mb * nb; q += NW) {
+    const int m0 = (q % mb) * 8, n0 = (q / mb) * 8;
+    const bool rm = m0 + gq < M, rn = n0 + gq < N;
+    const cplx* a0 = A + m0 + gq;
+    const cplx* b0 = B + (n0 + gq) * bn;
+    double cr[2] = {0.0, 0.0}, ci[2] = {0.0, 0.0};
+#pragma unroll 4
+    for (int k0 = 0; k0 < K; k0 += 4) {
+      const int k = k0 + tq;
+      cplx a = make_double2(0.0, 0.0), b = make_double2(0.0, 0.0);
+      if (rm && k < K) a = a0[k * ak];
+      if (rn && k < K) b = b0[k * bk];
+      dmma884(cr[0], cr[1], a.x, b.x);
+      dmma884(ci[0], ci[1], a.x, b.y);
+      dmma884(cr[0], cr[1], -a.y, b.y);
+      dmma884(ci[0], ci[1], a.y, b.x);
+    }
+    if (rm) {
+#pragma unroll
+      for (int e = 0; e < 2; ++e)
+        if (n0 + 2 * tq + e < N) C[m0 + gq + (n0 + 2 * tq + e) * M] = make_double2(cr[e], ci[e]);
+    }
+  }
+}
+
+// w = H_eff x, all in shared memory (w may lie in global memory).
+static __device__ __forceinline__ void small_heff(const HeffOp& h, const SmallPlan& p, cplx* buf, const cplx* x,
+                                                  cplx* w) {
+  const int chil = h.chil, D = h.D, chir = h.chir, wl = h.wl, wr = h.wr;
+  cplx* T1 = buf + p.oT1;
+  small_gemm(chil * wl, D * chir, chil, buf, chil * wl, x, 1, chil, T1);
+  cta_sync();
+  const cplx* T2 = T1;
+  if (!h.W.ident) {
+    cplx* T2w = buf + p.oT2;
+    T2 = T2w;
+    // T2[a, p', m', c] = sum W[(p', m'), (m, p)] T1[a, m, p, c], every output
+    // formed before any is stored (in place)
+    const int npair = chil * chir, items = npair * h.W.no;
+    const cplx* val = buf + p.oVal;
+    const int* rowp = reinterpret_cast<const int*>(buf + p.oIdx);
+    const int* col = rowp + h.W.no + 1;
+    cplx acc[8 * SMALL_N / NT];  // D wr chil chir <= 8 n
+#pragma unroll
+    for (int u = 0; u < 8 * SMALL_N / NT; ++u) {
+      const int e = ltid() + NT * u;
+      acc[u] = make_double2(0.0, 0.0);
+      if (e < items) {
+        const int pr = e % npair, o = e / npair, a = pr % chil, c = pr / chil;
+        const cplx* in = T1 + a + c * chil * wl * D;
+        for (int z = rowp[o]; z < rowp[o + 1]; ++z) wfma(acc[u], val[z], in[col[z] * chil]);
+      }
+    }
+    cta_sync();
+#pragma unroll
+    for (int u = 0; u < 8 * SMALL_N / NT; ++u) {
+      const int e = ltid() + NT * u;
+      if (e < items) {
+        const int pr = e % npair, o = e / npair, a = pr % chil, c = pr / chil;
+        T2w[a + chil * (o + D * wr * c)] = acc[u];
+      }
+    }
+    cta_sync();
+  }
+  small_gemm(chil * D, chir, wr * chir, T2, chil * D, buf + p.oR, chir, 1, w);
+  cta_sync();
+}
+
+// h_j = <q_j, w> (j < k) into ks.h; returns |w|^2.  The group of eight that a
+// vector is summed in does not enter its sum, so the groups share two
+// barriers.
+static __device__ __forceinline__ double small_dots(const cplx* sQ, int nfit, const cplx* Q, long long qs,
+                                                    const cplx* w, int n, int k, double* red, KrySmem& ks) {
+  const int tid = ltid(), lane = tid & 31, wid = tid >> 5;
+  const int groups = (k + 8) / 8;  // k vectors and the norm
+  for (int g = 0; g < groups; ++g) {
+    double d[16];
+#pragma unroll
+    for (int e = 0; e < 16; ++e) d[e] = 0.0;
+    for (int i = tid; i < n; i += NT) {
+      const cplx w0 = w[i];
+#pragma unroll
+      for (int e = 0; e < 8; ++e) {
+        const int j = 8 * g + e;
+        if (j < k) {
+          const cplx q = j < nfit ? sQ[j * n + i] : Q[qs * j + i];
+          const cplx p = cmulc(q, w0);
+          d[2 * e] += p.x;
+          d[2 * e + 1] += p.y;
+        } else if (j == k) {
+          d[2 * e] += cabs2(w0);
+        }
+      }
+    }
+    warp_sum_multi<16>(d);
+    if ((lane & 1) == 0) red[(g * NW + wid) * 16 + (lane >> 1)] = d[0];
+  }
+  cta_sync();
+  for (int t = tid; t < groups * 16; t += NT) {
+    const int g = t >> 4, e = t & 15, j = 8 * g + (e >> 1);
+    double s = 0.0;
+#pragma unroll
+    for (int w2 = 0; w2 < NW; ++w2) s += red[(g * NW + w2) * 16 + e];
+    double* hj = reinterpret_cast<double*>(ks.h + j);
+    if (j <= k) hj[e & 1] = s;  // the norm lands in h[k].x
+  }
+  cta_sync();
+  return ks.h[k].x;
+}
+
+// dev_expm_krylov for a solve that fits small_plan.
+static __device__ __noinline__ int dev_expm_small(const HeffOp& h, const SmallPlan& p, cplx* x, double dt,
+                                                  const KrylovCfg& kc, cplx* Q, long long qs, EngineSmem& sm) {
+  cplx* buf = reinterpret_cast<cplx*>(&sm.u);
+  cplx* sQ = buf + p.oQ;
+  double* red = reinterpret_cast<double*>(buf + p.oRed);
+  KrySmem& ks = sm.k;
+  const int tid = ltid();
+  const int n = h.chil * h.D * h.chir, nfit = p.nfit;
+  const double beta0 = sqrt(cta_norm2(x, n, sm.r));
+  if (beta0 == 0.0) return 0;
+  const double tau = fabs(dt);
+  for (int e = tid; e < h.chil * h.wl * h.chil; e += NT) buf[e] = h.L[e];
+  for (int e = tid; e < h.chir * h.wr * h.chir; e += NT) buf[p.oR + e] = h.R[e];
+  if (!h.W.ident) {
+    int* idx = reinterpret_cast<int*>(buf + p.oIdx);
+    for (int e = tid; e <= h.W.no; e += NT) idx[e] = h.W.rowp[e];
+    for (int e = tid; e < h.W.nnz; e += NT) {
+      idx[h.W.no + 1 + e] = h.W.col[e];
+      buf[p.oVal + e] = h.W.val[e];
+    }
+  }
+  for (int i = tid; i < n; i += NT) sQ[i] = cscale(x[i], 1.0 / beta0);
+  cta_sync();
+  auto vec = [&](int j) { return j < nfit ? sQ + j * n : Q + qs * j; };
+  // out = s (w - sum_{j<k} h_j q_j); this thread's part of |out|^2
+  auto combine = [&](const cplx* w, cplx* out, int k, double s) {
+    double part = 0.0;
+    for (int i = tid; i < n; i += NT) {
+      cplx v = w ? w[i] : make_double2(0.0, 0.0);
+      for (int j = 0; j < k; ++j) v = csub_mul(v, ks.h[j], j < nfit ? sQ[j * n + i] : Q[qs * j + i]);
+      v = cscale(v, s);
+      out[i] = v;
+      part += cabs2(v);
+    }
+    return part;
+  };
+  double bound = 1.0;
+  int m = 0, mv = 0;
+  for (int k = 1; k <= kc.kdim; ++k) {
+    cplx* w = vec(k);
+    small_heff(h, p, buf, vec(k - 1), w);
+    ++mv;
+    ProfScope orth_scope_(PF_ORTH);
+    const double nw2 = small_dots(sQ, nfit, Q, qs, w, n, k, red, ks);
+    double hh = 0.0;
+    for (int j = 0; j < k; ++j) hh += cabs2(ks.h[j]);
+    double a_k = ks.h[k - 1].x;
+    const double r2 = nw2 - hh;
+    const bool accept = r2 >= 0.5 * nw2;
+    double b_k;
+    if (accept) {
+      b_k = sqrt(r2);
+    } else {
+      combine(w, w, k, 1.0);
+      small_dots(sQ, nfit, Q, qs, w, n, k, red, ks);
+      a_k += ks.h[k - 1].x;
+      b_k = sqrt(block_sum(combine(w, w, k, 1.0), sm.r));
+    }
+    if (tid == 0) ks.alpha[k - 1] = a_k;
+    m = k;
+    if (b_k <= tau * kc.tol) break;
+    if (k == kc.kdim) break;
+    bound *= b_k * tau / k;
+    if (kc.exit_tol > 0.0 && bound <= kc.exit_tol) break;
+    if (tid == 0) ks.beta[k - 1] = b_k;
+    const double inv = 1.0 / b_k;
+    if (accept) {
+      combine(w, w, k, inv);
+    } else {
+      for (int i = tid; i < n; i += NT) w[i] = cscale(w[i], inv);
+    }
+    cta_sync();
+  }
+  cta_sync();
+  dev_tridiag_expm(m, dt, ks);
+  cta_sync();
+  if (tid < m) ks.h[tid] = make_double2(-ks.y[tid].x, -ks.y[tid].y);  // x = beta0 sum_j y_j q_j
+  cta_sync();
+  combine(nullptr, x, m, beta0);
+  cta_sync();
+  return mv;
+}
+
 // In place: x <- exp(-i dt H_eff) x.  Q holds kdim+1 vectors of stride qs.
 // Returns the number of H_eff products.  CTA-collective.
 static __device__ __noinline__ int dev_expm_krylov(const HeffOp& h, cplx* x, double dt, const KrylovCfg& kc, cplx* Q,
                                             long long qs, EngineSmem& sm) {
+  SmallPlan sp;
+  if (small_plan(h, sp)) return dev_expm_small(h, sp, x, dt, kc, Q, qs, sm);
   const int tid = ltid();
   const long long n = (long long)h.chil * h.D * h.chir;
   const double beta0 = sqrt(cta_norm2(x, n, sm.r));
