@@ -41,14 +41,15 @@ static __device__ __forceinline__ void cta_sync() { __syncthreads(); }
 #endif
 
 // Optional per-slot phase timers (clock64 cycles), enabled when the host sets
-// g_prof to a [slots][PROF_N] buffer.  Thread 0 of a program accumulates the
+// g_prof to a [slots][PROF_N] buffer.  The pointer is constant memory: every
+// routine tests it on entry and exit, timed or not.  Thread 0 of a program accumulates the
 // elapsed time of each instrumented routine.
 #define PROF_N 16
 enum {
   PF_GEMM = 0, PF_WAPPLY = 1, PF_ORTH = 2, PF_TRIDIAG = 3, PF_SVD = 4, PF_SVDVEC = 5, PF_QR = 6, PF_QRQ = 7,
   PF_SCALAR = 8, PF_ENV = 9, PF_DISS = 10, PF_STOCH = 11, PF_EVAL = 12, PF_SWEEP = 13, PF_STEP = 14, PF_COPY = 15
 };
-static __device__ unsigned long long* g_prof = nullptr;  // one per translation unit
+static __constant__ unsigned long long* g_prof = nullptr;  // one per translation unit
 struct ProfScope {
   long long t0;
   int id;

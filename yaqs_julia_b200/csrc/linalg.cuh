@@ -219,6 +219,28 @@ static __device__ __forceinline__ void dev_qr_extract_r(const cplx* H, int m, in
   cta_sync();
 }
 
+// Thin QR of M (m x n, col-major), load(e) its element e: store_q(e, q), e < m k,
+// stores from Q (m x k) at q, Rout becomes R (k x n), k = min(m, n).  H and Qg
+// are work matrices in global memory; a problem that fits runs in the shared buffer sb
+// (cap values) instead, Q beside the factored matrix if both do: every
+// column step reads what other threads wrote in the step before, which
+// through L2 costs its latency each time.
+template <class Load, class Store>
+static __device__ __forceinline__ void dev_qr_thin(int m, int n, Load load, cplx* H, Store store_q, cplx* Qg, cplx* Rout,
+                                                   cplx* sb, int cap, LinalgSmem& ls, RedScratch& rs) {
+  const int k = min(m, n);
+  cplx* h = m * n <= cap ? sb : H;
+  cplx* q = (m * n + m * k <= cap) ? sb + m * n : Qg;
+  cta_sync();  // the shared buffer's last readers are done
+  for (int e = ltid(); e < m * n; e += NT) h[e] = load(e);
+  cta_sync();
+  dev_qr_factor(h, m, n, ls, rs);
+  dev_qr_formq(h, m, n, q, ls);
+  dev_qr_extract_r(h, m, n, Rout);
+  for (int e = ltid(); e < m * k; e += NT) store_q(e, q);
+  cta_sync();
+}
+
 // ---------------------------------------------------------------------------
 // One-sided Jacobi SVD
 // ---------------------------------------------------------------------------
@@ -391,7 +413,9 @@ static __device__ __forceinline__ void svd_stage(cplx* sb, int ld, const SvdWork
 // Sigma.  Jacobi runs in the block-cyclic order (per sweep: every diagonal
 // block with a round-robin pass, then every pair of blocks in round-robin
 // order with b rounds of disjoint cross pairs) on blocks staged in the
-// shared buffer sb (SVD_SMEM_CPLX elements).  Leaves the sorted singular
+// shared buffer sb (SVD_SMEM_CPLX elements), or on all of B held there when
+// it fits: the sweeps then touch no global memory, where each block pair
+// used to be read and written back every time it was rotated.  Leaves the sorted singular
 // values in w.sig (nulls set to 0).  CTA-collective; returns metadata.
 enum { SVD_LEFT = 0, SVD_RIGHT = 1 };
 static __device__ __noinline__ SvdResult dev_svd(const cplx* M, int m, int n, int side, SvdWork& w, LinalgSmem& ls,
@@ -407,7 +431,12 @@ static __device__ __noinline__ SvdResult dev_svd(const cplx* M, int m, int n, in
   res.q = q;
   res.p = p;
   res.sweeps = 0;
-  cplx* H = w.X;
+  // A problem that fits the shared buffer stays there: the factored matrix
+  // (at the end of the buffer, or in global memory) and B for all sweeps.
+  const bool resident = q * p <= SVD_SMEM_CPLX;
+  const bool h_shared = mm * nn <= SVD_SMEM_CPLX;
+  const bool both = resident && mm * nn + q * p <= SVD_SMEM_CPLX;
+  cplx* H = h_shared ? sb + (SVD_SMEM_CPLX - mm * nn) : w.X;
   for (int e = tid; e < mm * nn; e += NT) {
     int r = (int)(e % mm), c = (int)(e / mm);
     H[e] = res.tr ? M[e] : cconj(M[c + (long long)m * r]);
@@ -415,11 +444,16 @@ static __device__ __noinline__ SvdResult dev_svd(const cplx* M, int m, int n, in
   cta_sync();
   dev_qr_factor(H, mm, nn, ls, rs);
   // B = R^H (nn x k): B[r, c] = conj(R[c, r]) for c <= r
+  cplx* B0 = both ? sb : w.B;
   for (int e = tid; e < q * p; e += NT) {
     int r = (int)(e % q), c = (int)(e / q);
-    w.B[e] = (c <= r) ? cconj(H[c + (long long)mm * r]) : make_double2(0.0, 0.0);
+    B0[e] = (c <= r) ? cconj(H[c + (long long)mm * r]) : make_double2(0.0, 0.0);
   }
   cta_sync();
+  if (resident && !both) {
+    cta_copy(sb, w.B, (long long)q * p);
+    cta_sync();
+  }
   const double tol = 2.220446049250313e-16 * q;
   const int ld = q;
   const int b = svd_block_size(q, p);
@@ -431,9 +465,10 @@ static __device__ __noinline__ SvdResult dev_svd(const cplx* M, int m, int n, in
     cta_sync();
     for (int I = 0; I < nb; ++I) {
       const int c0 = I * b, nc = min(b, p - c0);
-      svd_stage(sb, ld, w, q, c0, nc, 0, 0, false);
+      if (!resident) svd_stage(sb, ld, w, q, c0, nc, 0, 0, false);
+      cplx* cols = resident ? sb + ld * c0 : sb;
       for (int round = 0; round < be2 - 1; ++round) {
-        smem_rotate_round(sb, ld, q, q, be2 / 2,
+        smem_rotate_round(cols, ld, q, q, be2 / 2,
                           [&](int pr, int& i, int& j) {
                             int ta = pr, tb = be2 - 1 - pr;
                             int a = ta == 0 ? 0 : ((ta - 1 - round + 2 * (be2 - 1)) % (be2 - 1)) + 1;
@@ -444,7 +479,7 @@ static __device__ __noinline__ SvdResult dev_svd(const cplx* M, int m, int n, in
                           },
                           tol, &ls.rot_count);
       }
-      svd_stage(sb, ld, w, q, c0, nc, 0, 0, true);
+      if (!resident) svd_stage(sb, ld, w, q, c0, nc, 0, 0, true);
     }
     for (int round = 0; round < nbe - 1; ++round) {
       for (int pr = 0; pr < nbe / 2; ++pr) {
@@ -454,27 +489,33 @@ static __device__ __noinline__ SvdResult dev_svd(const cplx* M, int m, int n, in
         int I = min(A, Bk), J = max(A, Bk);
         if (J >= nb) continue;
         const int c0 = I * b, n0 = min(b, p - c0), c1 = J * b, n1 = min(b, p - c1);
-        svd_stage(sb, ld, w, q, c0, n0, c1, n1, false);
+        if (!resident) svd_stage(sb, ld, w, q, c0, n0, c1, n1, false);
+        cplx* cols = resident ? sb + ld * c0 : sb;
+        const int joff = resident ? c1 - c0 : n0;
         for (int t = 0; t < b; ++t) {
-          smem_rotate_round(sb, ld, q, q, b,
+          smem_rotate_round(cols, ld, q, q, b,
                             [&](int kk, int& i, int& j) {
                               int jj = (kk + t) % b;
                               if (kk >= n0 || jj >= n1) {
                                 i = j = -1;
                               } else {
                                 i = kk;
-                                j = n0 + jj;
+                                j = joff + jj;
                               }
                             },
                             tol, &ls.rot_count);
         }
-        svd_stage(sb, ld, w, q, c0, n0, c1, n1, true);
+        if (!resident) svd_stage(sb, ld, w, q, c0, n0, c1, n1, true);
       }
     }
     int rc = ls.rot_count;
     cta_sync();
     res.sweeps = sweep + 1;
     if (rc == 0) break;
+  }
+  if (resident) {
+    cta_copy(w.B, sb, (long long)q * p);
+    cta_sync();
   }
   // singular values
   const int lane = tid & 31, wid = tid >> 5;

@@ -201,6 +201,21 @@ static __device__ void set_chi(Ctx& c, const DState& s, int b, int v) {
   cta_sync();
 }
 
+// A (m x r) = Q R: Q replaces A, R to Rb.  H, Qg: work buffers.
+static __device__ __noinline__ void right_factor(Ctx& c, cplx* A, int m, int r, cplx* H, cplx* Qg, cplx* Rb) {
+  dev_qr_thin(m, r, [&](int e) { return A[e]; }, H, [&](int e, const cplx* q) { A[e] = q[e]; }, Qg, Rb, c.sm.e.u.svd,
+              (int)(sizeof(EngineSmemU) / sizeof(cplx)), c.sm.la, c.sm.e.r);
+}
+
+// A (l x n2) = L Q: Q replaces A (rn x n2, rn = min(l, n2)), L^H = R of
+// A^H = Q R to Rb.  H, Qg: work buffers.
+static __device__ __noinline__ void left_factor(Ctx& c, cplx* A, int l, int n2, cplx* H, cplx* Qg, cplx* Rb) {
+  const int rn = min(l, n2);
+  dev_qr_thin(n2, l, [&](int e) { return cconj(A[e / n2 + l * (e % n2)]); }, H,
+              [&](int e, const cplx* q) { A[e] = cconj(q[e / rn + n2 * (e % rn)]); }, Qg, Rb, c.sm.e.u.svd,
+              (int)(sizeof(EngineSmemU) / sizeof(cplx)), c.sm.la, c.sm.e.r);
+}
+
 // site i: A = Q R, Q -> site i, R absorbed into site i+1.
 static __device__ __noinline__ void qr_right(Ctx& c, const DState& s, int i) {
   const int l = s.chi[i], r = s.chi[i + 1], m = 2 * l, rn = min(m, r);
@@ -210,11 +225,7 @@ static __device__ __noinline__ void qr_right(Ctx& c, const DState& s, int i) {
   cplx* H = c.ws + c.P.lay.tA;
   cplx* Rb = c.ws + c.P.lay.tB;
   cplx* T = c.ws + c.P.lay.tC;
-  cta_copy(H, A, (long long)m * r);
-  cta_sync();
-  dev_qr_factor(H, m, r, c.sm.la, c.sm.e.r);
-  dev_qr_formq(H, m, r, A, c.sm.la);
-  dev_qr_extract_r(H, m, r, Rb);
+  right_factor(c, A, m, r, H, T, Rb);
   cta_gemm(gemm_args(rn, 2 * r2, r, Rb, 1, rn, An, 1, r, T, 1, rn), c.sm.e.u.gw.g);
   cta_copy(An, T, (long long)rn * 2 * r2);
   set_chi(c, s, i + 1, rn);
@@ -229,18 +240,7 @@ static __device__ __noinline__ void lq_left(Ctx& c, const DState& s, int i) {
   cplx* H = c.ws + c.P.lay.tA;
   cplx* Qh = c.ws + c.P.lay.tB;
   cplx* Rb = c.ws + c.P.lay.tC;
-  for (int e = ltid(); e < n2 * l; e += NT) {
-    int cc = (int)(e % n2), ii = (int)(e / n2);
-    H[e] = cconj(A[ii + (long long)l * cc]);
-  }
-  cta_sync();
-  dev_qr_factor(H, n2, l, c.sm.la, c.sm.e.r);
-  dev_qr_formq(H, n2, l, Qh, c.sm.la);
-  dev_qr_extract_r(H, n2, l, Rb);
-  for (int e = ltid(); e < rn * n2; e += NT) {
-    int k = (int)(e % rn), cc = (int)(e / rn);
-    A[e] = cconj(Qh[cc + (long long)n2 * k]);
-  }
+  left_factor(c, A, l, n2, H, Qh, Rb);
   cta_sync();
   cta_gemm(gemm_args(2 * lp, rn, l, Ap, 1, 2 * lp, Rb, rn, 1, H, 1, 2 * lp, false, true), c.sm.e.u.gw.g);
   cta_copy(Ap, H, (long long)2 * lp * rn);
@@ -621,11 +621,7 @@ static __device__ __noinline__ void qr_bond_forward(Ctx& c, const DState& s, int
   cplx* H = c.ws + c.P.lay.tA;
   cplx* Rb = c.ws + c.P.lay.tB;
   cplx* T = c.ws + c.P.lay.tC;
-  cta_copy(H, A, (long long)m * r);
-  cta_sync();
-  dev_qr_factor(H, m, r, c.sm.la, c.sm.e.r);
-  dev_qr_formq(H, m, r, A, c.sm.la);
-  dev_qr_extract_r(H, m, r, Rb);
+  right_factor(c, A, m, r, H, T, Rb);
   set_chi(c, s, i + 1, rn);
   if (c.sm.fail) return;
   update_left(c, s, i);
@@ -645,18 +641,7 @@ static __device__ __noinline__ void lq_bond_backward(Ctx& c, const DState& s, in
   cplx* H = c.ws + c.P.lay.tA;
   cplx* Qh = c.ws + c.P.lay.tB;
   cplx* Rb = c.ws + c.P.lay.tC;
-  for (int e = ltid(); e < n2 * l; e += NT) {
-    int cc = (int)(e % n2), ii = (int)(e / n2);
-    H[e] = cconj(A[ii + (long long)l * cc]);
-  }
-  cta_sync();
-  dev_qr_factor(H, n2, l, c.sm.la, c.sm.e.r);
-  dev_qr_formq(H, n2, l, Qh, c.sm.la);
-  dev_qr_extract_r(H, n2, l, Rb);
-  for (int e = ltid(); e < rn * n2; e += NT) {
-    int k = (int)(e % rn), cc = (int)(e / rn);
-    A[e] = cconj(Qh[cc + (long long)n2 * k]);
-  }
+  left_factor(c, A, l, n2, H, Qh, Rb);
   cplx* Lm = H;  // L = R^H (l x rn)
   for (int e = ltid(); e < l * rn; e += NT) {
     int a = (int)(e % l), k = (int)(e / l);
