@@ -473,66 +473,61 @@ static __device__ double lanczos_subtract(const cplx* Q, long long qs, cplx* w, 
 // another thread has just written through L2.  Here the environments, the
 // intermediates and as many Krylov vectors as fit live in the CTA's staging
 // buffer, the products run on 8 x 8 blocks dealt to the warps straight from
-// it, and a Lanczos step takes seven barriers instead of about thirty.
+// it, and a Lanczos step takes four barriers (eight with a refinement)
+// instead of about thirty.  Loops are kept rolled: with most of its time spent
+// in code that runs a few dozen times, a solve waits for instruction fetches
+// before it waits for anything else.
 // Every sum is formed in the general path's order (four-deep MMA steps from
 // k = 0, the same reduction trees), so both give the same bits: where a
 // 2-site sweep truncates between equal Schmidt values, rounding decides, and
 // a chain must not change its records by crossing this limit.
 // SMALL_N is one value per thread; wider solves fill the tiles of the general
 // path.  Measured with the sweep on L = 6 Ising, chi 16, 200 trajectories, 51
-// time indices: 445 ms with the general path alone, 268 ms with this one.
+// time indices: 445 ms with the general path alone, 180 ms with this one.
 #define SMALL_N 256
 #define SMALL_MIN_VECS 4  // Krylov vectors that have to fit beside the operands
 
 struct SmallPlan {
-  int oR, oT1, oT2, oVal, oIdx, oRed, oQ;  // offsets in the buffer; L at 0
-  int nfit;                                // Krylov vectors held in the buffer
+  int oR, oT1, oVal, oIdx, oQ;  // offsets in the buffer; L at 0
+  int nfit;                     // Krylov vectors held in the buffer
 };
 
 static __device__ __forceinline__ bool small_plan(const HeffOp& h, SmallPlan& p) {
   const int n = h.chil * h.D * h.chir;
-  if (n > SMALL_N || h.mixed || h.W.no * h.chil * h.chir > 8 * SMALL_N) return false;
+  if (n > SMALL_N || h.mixed) return false;
   const int cap = (int)(sizeof(EngineSmemU) / sizeof(cplx));
   int off = h.chil * h.wl * h.chil;
   p.oR = off;
   off += h.chir * h.wr * h.chir;
   p.oT1 = off;
   off += h.chil * h.wl * h.D * h.chir;
-  p.oT2 = p.oT1;  // in place: with wl == wr a pair's inputs and outputs share their addresses
-  if (h.wl != h.wr) {
-    p.oT2 = off;
-    off += h.chil * h.wr * h.D * h.chir;
-  }
   p.oVal = off;
   off += h.W.ident ? 0 : h.W.nnz;
   p.oIdx = off;  // row pointers, then columns
   off += h.W.ident ? 0 : (h.W.no + 1 + h.W.nnz + 3) / 4;
-  p.oRed = off;
-  off += 5 * NW * 8;  // 16 partial sums of each warp for five groups of vectors (33 sums)
   p.oQ = off;
   p.nfit = (cap - off) / n;
   return cap > off && p.nfit >= SMALL_MIN_VECS;
 }
 
-// C(M x N) = A B from shared memory: A (m,k) at A[m + k ak], B (k,n) at
-// B[k bk + n bn], C (m,n) at C[m + n M].  Warps take 8 x 8 blocks.
-static __device__ __forceinline__ void small_gemm(int M, int N, int K, const cplx* A, int ak, const cplx* B, int bk,
-                                                  int bn, cplx* C) {
+// C(M x N) = A B on 8 x 8 blocks dealt to the warps: fa(row, k) and fb(k, col)
+// give the operands inside the matrix, C (m,n) at C[m + n M].
+template <class FA, class FB>
+static __device__ __forceinline__ void small_gemm(int M, int N, int K, FA fa, FB fb, cplx* C) {
   const int lane = ltid() & 31, wid = ltid() >> 5;
   const int gq = lane >> 2, tq = lane & 3;
   const int mb = (M + 7) >> 3, nb = (N + 7) >> 3;
+#pragma unroll 1
   for (int q = wid; q < mb * nb; q += NW) {
-    const int m0 = (q % mb) * 8, n0 = (q / mb) * 8;
-    const bool rm = m0 + gq < M, rn = n0 + gq < N;
-    const cplx* a0 = A + m0 + gq;
-    const cplx* b0 = B + (n0 + gq) * bn;
+    const int nq = q / mb, row = (q - nq * mb) * 8 + gq, n0 = nq * 8;
+    const bool rm = row < M, rn = n0 + gq < N;
+    auto arow = fa(row);
     double cr[2] = {0.0, 0.0}, ci[2] = {0.0, 0.0};
-#pragma unroll 4
-    for (int k0 = 0; k0 < K; k0 += 4) {
-      const int k = k0 + tq;
+#pragma unroll 1
+    for (int k = tq; k - tq < K; k += 4) {
       cplx a = make_double2(0.0, 0.0), b = make_double2(0.0, 0.0);
-      if (rm && k < K) a = a0[k * ak];
-      if (rn && k < K) b = b0[k * bk];
+      if (rm && k < K) a = arow(k);
+      if (rn && k < K) b = fb(k, n0 + gq);
       dmma884(cr[0], cr[1], a.x, b.x);
       dmma884(ci[0], ci[1], a.x, b.y);
       dmma884(cr[0], cr[1], -a.y, b.y);
@@ -541,91 +536,80 @@ static __device__ __forceinline__ void small_gemm(int M, int N, int K, const cpl
     if (rm) {
 #pragma unroll
       for (int e = 0; e < 2; ++e)
-        if (n0 + 2 * tq + e < N) C[m0 + gq + (n0 + 2 * tq + e) * M] = make_double2(cr[e], ci[e]);
+        if (n0 + 2 * tq + e < N) C[row + (n0 + 2 * tq + e) * M] = make_double2(cr[e], ci[e]);
     }
   }
 }
 
-// w = H_eff x, all in shared memory (w may lie in global memory).
+// w = H_eff x, all in shared memory (w may lie in global memory).  The MPO
+// map is applied while the second product loads its left operand: every
+// value is loaded by one block column only (chir <= 8) or a few, and T2 and
+// its barriers go away.
 static __device__ __forceinline__ void small_heff(const HeffOp& h, const SmallPlan& p, cplx* buf, const cplx* x,
                                                   cplx* w) {
   const int chil = h.chil, D = h.D, chir = h.chir, wl = h.wl, wr = h.wr;
   cplx* T1 = buf + p.oT1;
-  small_gemm(chil * wl, D * chir, chil, buf, chil * wl, x, 1, chil, T1);
+  const int ml = chil * wl;
+  small_gemm(ml, D * chir, chil, [&](int row) { return [=](int k) { return buf[row + k * ml]; }; },
+             [&](int k, int n) { return x[k + n * chil]; }, T1);
   cta_sync();
-  const cplx* T2 = T1;
-  if (!h.W.ident) {
-    cplx* T2w = buf + p.oT2;
-    T2 = T2w;
-    // T2[a, p', m', c] = sum W[(p', m'), (m, p)] T1[a, m, p, c], every output
-    // formed before any is stored (in place)
-    const int npair = chil * chir, items = npair * h.W.no;
-    const cplx* val = buf + p.oVal;
-    const int* rowp = reinterpret_cast<const int*>(buf + p.oIdx);
-    const int* col = rowp + h.W.no + 1;
-    cplx acc[8 * SMALL_N / NT];  // D wr chil chir <= 8 n
-#pragma unroll
-    for (int u = 0; u < 8 * SMALL_N / NT; ++u) {
-      const int e = ltid() + NT * u;
-      acc[u] = make_double2(0.0, 0.0);
-      if (e < items) {
-        const int pr = e % npair, o = e / npair, a = pr % chil, c = pr / chil;
-        const cplx* in = T1 + a + c * chil * wl * D;
-        for (int z = rowp[o]; z < rowp[o + 1]; ++z) wfma(acc[u], val[z], in[col[z] * chil]);
-      }
-    }
-    cta_sync();
-#pragma unroll
-    for (int u = 0; u < 8 * SMALL_N / NT; ++u) {
-      const int e = ltid() + NT * u;
-      if (e < items) {
-        const int pr = e % npair, o = e / npair, a = pr % chil, c = pr / chil;
-        T2w[a + chil * (o + D * wr * c)] = acc[u];
-      }
-    }
-    cta_sync();
-  }
-  small_gemm(chil * D, chir, wr * chir, T2, chil * D, buf + p.oR, chir, 1, w);
+  const cplx* R = buf + p.oR;
+  const cplx* val = buf + p.oVal;
+  const int* rowp = reinterpret_cast<const int*>(buf + p.oIdx);
+  const int* col = rowp + h.W.no + 1;
+  const bool ident = h.W.ident != 0;
+  small_gemm(chil * D, chir, wr * chir,
+             [&](int row) {
+               const int pp = row / chil, a = row - pp * chil;
+               return [=](int k) {
+                 if (ident) return T1[a + k * chil];
+                 // T2[a, p', m', c] = sum W[(p', m'), (m, p)] T1[a, m, p, c], k = m' + wr c
+                 const int c = k / wr, o = pp + D * (k - c * wr);
+                 const cplx* in = T1 + a + c * ml * D;
+                 cplx acc = make_double2(0.0, 0.0);
+#pragma unroll 1
+                 for (int z = rowp[o]; z < rowp[o + 1]; ++z) wfma(acc, val[z], in[col[z] * chil]);
+                 return acc;
+               };
+             },
+             [&](int k, int n) { return R[n + k * chir]; }, w);
   cta_sync();
 }
 
-// h_j = <q_j, w> (j < k) into ks.h; returns |w|^2.  The group of eight that a
-// vector is summed in does not enter its sum, so the groups share two
-// barriers.
-static __device__ __forceinline__ double small_dots(const cplx* sQ, int nfit, const cplx* Q, long long qs,
-                                                    const cplx* w, int n, int k, double* red, KrySmem& ks) {
-  const int tid = ltid(), lane = tid & 31, wid = tid >> 5;
-  const int groups = (k + 8) / 8;  // k vectors and the norm
-  for (int g = 0; g < groups; ++g) {
-    double d[16];
+// h_j = <q_j, w> (j < k) into ks.h; returns |w|^2.  A warp forms one sum: the
+// tree over the lanes of each 32 values, then these in order, which is how
+// the general path's threads, warps and block add them.
+static __device__ __noinline__ double small_dots(const cplx* sQ, int nfit, const cplx* Q, long long qs, const cplx* w,
+                                                 int n, int k, KrySmem& ks) {
+  const int lane = ltid() & 31, wid = ltid() >> 5;
+#pragma unroll 1
+  for (int j = wid; j <= k; j += NW) {  // j = k: the norm
+    const cplx* q = j < nfit ? sQ + j * n : Q + qs * j;
+    double sx = 0.0, sy = 0.0;
+#pragma unroll 1
+    for (int i0 = 0; i0 < n; i0 += 64) {
+      double d[4] = {0.0, 0.0, 0.0, 0.0};
 #pragma unroll
-    for (int e = 0; e < 16; ++e) d[e] = 0.0;
-    for (int i = tid; i < n; i += NT) {
-      const cplx w0 = w[i];
-#pragma unroll
-      for (int e = 0; e < 8; ++e) {
-        const int j = 8 * g + e;
-        if (j < k) {
-          const cplx q = j < nfit ? sQ[j * n + i] : Q[qs * j + i];
-          const cplx p = cmulc(q, w0);
-          d[2 * e] += p.x;
-          d[2 * e + 1] += p.y;
-        } else if (j == k) {
-          d[2 * e] += cabs2(w0);
+      for (int u = 0; u < 2; ++u) {
+        const int i = i0 + 32 * u + lane;
+        if (i < n) {
+          const cplx w0 = w[i];
+          if (j < k) {
+            const cplx v = cmulc(q[i], w0);
+            d[2 * u] = v.x;
+            d[2 * u + 1] = v.y;
+          } else {
+            d[2 * u] = cabs2(w0);
+          }
         }
       }
+      warp_sum_multi<4>(d);  // lane l holds sum l / 8
+      sx += __shfl_sync(0xffffffffu, d[0], 0);
+      sy += __shfl_sync(0xffffffffu, d[0], 8);
+      sx += __shfl_sync(0xffffffffu, d[0], 16);
+      sy += __shfl_sync(0xffffffffu, d[0], 24);
     }
-    warp_sum_multi<16>(d);
-    if ((lane & 1) == 0) red[(g * NW + wid) * 16 + (lane >> 1)] = d[0];
-  }
-  cta_sync();
-  for (int t = tid; t < groups * 16; t += NT) {
-    const int g = t >> 4, e = t & 15, j = 8 * g + (e >> 1);
-    double s = 0.0;
-#pragma unroll
-    for (int w2 = 0; w2 < NW; ++w2) s += red[(g * NW + w2) * 16 + e];
-    double* hj = reinterpret_cast<double*>(ks.h + j);
-    if (j <= k) hj[e & 1] = s;  // the norm lands in h[k].x
+    if (lane == 0) ks.h[j] = make_double2(sx, sy);
   }
   cta_sync();
   return ks.h[k].x;
@@ -636,7 +620,6 @@ static __device__ __noinline__ int dev_expm_small(const HeffOp& h, const SmallPl
                                                   const KrylovCfg& kc, cplx* Q, long long qs, EngineSmem& sm) {
   cplx* buf = reinterpret_cast<cplx*>(&sm.u);
   cplx* sQ = buf + p.oQ;
-  double* red = reinterpret_cast<double*>(buf + p.oRed);
   KrySmem& ks = sm.k;
   const int tid = ltid();
   const int n = h.chil * h.D * h.chir, nfit = p.nfit;
@@ -661,6 +644,7 @@ static __device__ __noinline__ int dev_expm_small(const HeffOp& h, const SmallPl
     double part = 0.0;
     for (int i = tid; i < n; i += NT) {
       cplx v = w ? w[i] : make_double2(0.0, 0.0);
+#pragma unroll 2
       for (int j = 0; j < k; ++j) v = csub_mul(v, ks.h[j], j < nfit ? sQ[j * n + i] : Q[qs * j + i]);
       v = cscale(v, s);
       out[i] = v;
@@ -675,7 +659,7 @@ static __device__ __noinline__ int dev_expm_small(const HeffOp& h, const SmallPl
     small_heff(h, p, buf, vec(k - 1), w);
     ++mv;
     ProfScope orth_scope_(PF_ORTH);
-    const double nw2 = small_dots(sQ, nfit, Q, qs, w, n, k, red, ks);
+    const double nw2 = small_dots(sQ, nfit, Q, qs, w, n, k, ks);
     double hh = 0.0;
     for (int j = 0; j < k; ++j) hh += cabs2(ks.h[j]);
     double a_k = ks.h[k - 1].x;
@@ -686,7 +670,8 @@ static __device__ __noinline__ int dev_expm_small(const HeffOp& h, const SmallPl
       b_k = sqrt(r2);
     } else {
       combine(w, w, k, 1.0);
-      small_dots(sQ, nfit, Q, qs, w, n, k, red, ks);
+      cta_sync();
+      small_dots(sQ, nfit, Q, qs, w, n, k, ks);
       a_k += ks.h[k - 1].x;
       b_k = sqrt(block_sum(combine(w, w, k, 1.0), sm.r));
     }
