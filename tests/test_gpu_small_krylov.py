@@ -22,7 +22,7 @@ def _f(a):
 
 @pytest.mark.parametrize("chil,D,chir,wl,wr", [(1, 2, 1, 1, 1), (2, 4, 1, 5, 1), (1, 2, 3, 1, 8), (7, 2, 9, 3, 5),
                                                (8, 4, 8, 5, 5), (11, 2, 11, 4, 4), (16, 2, 8, 3, 3), (13, 2, 10, 3, 3),
-                                               (16, 2, 8, 1, 16), (4, 4, 4, 8, 8)])
+                                               (16, 2, 8, 1, 16), (4, 4, 4, 5, 5)])
 def test_small_solve_matches_oracle(oracle, chil, D, chir, wl, wr):
     from yaqs_julia_b200 import _lib
     ctx = _lib.default_context()

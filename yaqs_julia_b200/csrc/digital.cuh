@@ -117,7 +117,8 @@ static __device__ __noinline__ void digital_noise(Ctx& c, const DState& s, int s
   int nloc = 0;
   bool all_zero = true, split_diss = false, scalar_only = true, has_lr = false;
   double fdiss = 1.0;
-  for (int k = 0; k < P.nprocs; ++k) {
+  ProcIter itn(P, s1, s2);
+  for (int k; (k = itn.next()) >= 0;) {
     const DevProc& pr = P.procs[k];
     if (!proc_on(pr, s1, s2)) continue;
     ++nloc;
@@ -156,7 +157,8 @@ static __device__ __noinline__ void digital_noise(Ctx& c, const DState& s, int s
       return;
     }
     double total = 0.0;
-    for (int k = 0; k < P.nprocs; ++k)
+    ProcIter itt(P, s1, s2);
+    for (int k; (k = itt.next()) >= 0;)
       if (proc_on(P.procs[k], s1, s2)) total += P.procs[k].gamma * nrm;
     if (total == 0.0) {
       normalize_center(c, s);
@@ -167,9 +169,10 @@ static __device__ __noinline__ void digital_noise(Ctx& c, const DState& s, int s
     int chosen = -1, first = -1;
     const int sites[2] = {s1, s2};
     for (int si = 0; si < 2 && chosen < 0; ++si)
-      for (int k = 0; k < P.nprocs && chosen < 0; ++k) {
+      for (int z = P.p0_off[sites[si]]; z < P.p0_off[sites[si] + 1] && chosen < 0; ++z) {
+        const int k = P.p0_idx[z];
         const DevProc& pr = P.procs[k];
-        if (!proc_on(pr, s1, s2) || pr.s0 != sites[si]) continue;
+        if (!proc_on(pr, s1, s2)) continue;
         if (first < 0) first = k;
         acc += pr.gamma * nrm / total;
         if (r <= acc) chosen = k;
@@ -188,9 +191,9 @@ static __device__ __noinline__ void digital_noise(Ctx& c, const DState& s, int s
     for (int si = 0; si < 2 && !c.sm.fail; ++si) {
       const int i = sites[si];
       shift_oc(c, s, i);
-      for (int k = 0; k < P.nprocs; ++k) {
-        const DevProc& pr = P.procs[k];
-        if (!proc_on(pr, s1, s2) || pr.nsites != 1 || pr.s0 != i) continue;
+      for (int z = P.p0_off[i]; z < P.p0_off[i + 1]; ++z) {
+        const DevProc& pr = P.procs[P.p0_idx[z]];
+        if (!proc_on(pr, s1, s2) || pr.nsites != 1) continue;
         cplx* A = site_ptr(c, s, i);
         if (pr.pauli_name) {
           cta_scale(A, (long long)s.chi[i] * 2 * s.chi[i + 1], exp(-0.5 * pr.gamma));
@@ -200,9 +203,9 @@ static __device__ __noinline__ void digital_noise(Ctx& c, const DState& s, int s
         }
       }
       if (si == 0) {  // 2-site Pauli processes on (s1, s2) scale site s2
-        for (int k = 0; k < P.nprocs; ++k) {
-          const DevProc& pr = P.procs[k];
-          if (!proc_on(pr, s1, s2) || pr.nsites != 2 || pr.s1 != i) continue;
+        for (int z = P.p1_off[i]; z < P.p1_off[i + 1]; ++z) {
+          const DevProc& pr = P.procs[P.p1_idx[z]];
+          if (!proc_on(pr, s1, s2)) continue;
           cta_scale(site_ptr(c, s, i), (long long)s.chi[i] * 2 * s.chi[i + 1], exp(-0.5 * pr.drate));
           cta_sync();
         }
@@ -226,9 +229,10 @@ static __device__ __noinline__ void digital_noise(Ctx& c, const DState& s, int s
   for (int si = 0; si < 2 && !c.sm.fail; ++si) {
     const int site = sites[si];
     shift_oc(c, s, site);
-    for (int k = 0; k < P.nprocs; ++k) {
+    for (int z = P.p0_off[site]; z < P.p0_off[site + 1]; ++z) {
+      const int k = P.p0_idx[z];
       const DevProc& pr = P.procs[k];
-      if (!proc_on(pr, s1, s2) || pr.nsites != 1 || pr.s0 != site) continue;
+      if (!proc_on(pr, s1, s2) || pr.nsites != 1) continue;
       double nr = local_norm2(c, site_ptr(c, s, site), s.chi[site], 2, s.chi[site + 1], pr.pauli_proc ? nullptr : pr.mat);
       if (ltid() == 0) {
         cand[nc] = pr.gamma * nr;
@@ -237,9 +241,10 @@ static __device__ __noinline__ void digital_noise(Ctx& c, const DState& s, int s
       ++nc;
     }
     if (site < P.L - 1) {
-      for (int k = 0; k < P.nprocs; ++k) {
+      for (int z = P.p0_off[site]; z < P.p0_off[site + 1]; ++z) {
+        const int k = P.p0_idx[z];
         const DevProc& pr = P.procs[k];
-        if (!proc_on(pr, s1, s2) || pr.nsites != 2 || pr.s0 != site) continue;
+        if (!proc_on(pr, s1, s2) || pr.nsites != 2) continue;
         double nr;
         if (pr.pauli_proc) {
           nr = local_norm2(c, site_ptr(c, s, site), s.chi[site], 2, s.chi[site + 1], nullptr);

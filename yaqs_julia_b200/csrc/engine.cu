@@ -71,6 +71,8 @@ __global__ void __launch_bounds__(NT, 1) svd_kernel(int m, int n, const cplx* M,
   w.sig = reinterpret_cast<double*>(w0 + 4 * big + max(m, n));
   w.ord = iwork + (long long)b * SVD_MAX_COLS;
   const cplx* Mb = M + (long long)m * n * b;
+  if (ltid() == 0) sm.la.blocked = 0;
+  cta_sync();
   SvdResult r = dev_svd(Mb, m, n, SVD_LEFT, w, sm.la, sm.e.r, sm.e.u.svd);
   dev_svd_vectors(r, k, w, sm.e.r);
   cplx* Ub = U + (long long)m * k * b;
@@ -687,6 +689,40 @@ static int setup_run(yaqs_ctx* ctx, yaqs_run* run, const std::vector<int>& cap, 
   CUDA_TRY(ctx, cudaMemcpy(d_obs, ho.data(), ho.size() * sizeof(DevObs), cudaMemcpyHostToDevice));
   P.procs = d_procs;
   P.obs = d_obs;
+  {  // processes and 1-site observables by site
+    std::vector<int> idx;
+    std::vector<size_t> at;
+    auto by_site = [&](size_t n, auto site_of) {  // site_of(k): its site, or -1
+      at.push_back(idx.size());
+      std::vector<int> off(1, 0), list;
+      for (int i = 0; i < L; ++i) {
+        for (size_t k = 0; k < n; ++k)
+          if (site_of(k) == i) list.push_back((int)k);
+        off.push_back((int)list.size());
+      }
+      idx.insert(idx.end(), off.begin(), off.end());
+      idx.insert(idx.end(), list.begin(), list.end());
+    };
+    const size_t np = (size_t)P.nprocs;
+    by_site(np, [&](size_t k) { return hp[k].s0; });
+    by_site(np, [&](size_t k) { return hp[k].nsites == 2 ? hp[k].s1 : -1; });
+    by_site((size_t)n_obs, [&](size_t k) { return ho[k].kind == OBS_LOCAL1 ? ho[k].s0 : -1; });
+    int* d_idx;
+    CUDA_TRY(ctx, dm.alloc(&d_idx, idx.size()));
+    CUDA_TRY(ctx, cudaMemcpy(d_idx, idx.data(), idx.size() * sizeof(int), cudaMemcpyHostToDevice));
+    P.p0_off = d_idx + at[0];
+    P.p1_off = d_idx + at[1];
+    P.ob_off = d_idx + at[2];
+    P.p0_idx = P.p0_off + L + 1;
+    P.p1_idx = P.p1_off + L + 1;
+    P.ob_idx = P.ob_off + L + 1;
+    P.scalar_all = 1;
+    P.has_lr = 0;
+    for (size_t k = 0; k < np; ++k) {
+      if (!hp[k].pauli_name) P.scalar_all = 0;
+      if (hp[k].lr) P.has_lr = 1;
+    }
+  }
 
   // initial state arena (compact tensors at the site slots)
   std::vector<hcd> arena((size_t)mps_size, 0.0);
@@ -1072,6 +1108,9 @@ static int analog_begin_impl(yaqs_ctx* ctx, const yaqs_mps_desc* psi0, const yaq
   P.mixed = mixed ? 1 : 0;
   P.tc = use_tc ? 1 : 0;
   P.tdvp_mode = cfg->tdvp_mode;
+  // a 2-site sweep may cut between equal Schmidt values, where rounding
+  // decides; it keeps the order of its sums
+  P.blocked = cfg->tdvp_mode != YAQS_TDVP_2SITE ? 1 : 0;
   P.sample_ts = cfg->sample_timesteps != 0;
   P.max_bond = cfg->max_bond_dim;
   P.nobs = n_obs;
@@ -1545,6 +1584,7 @@ int digital_begin(yaqs_ctx* ctx, const yaqs_mps_desc* psi0, const yaqs_gate_desc
   memset(&P, 0, sizeof(P));
   P.L = L;
   P.n_times = n_layers + 1;
+  P.blocked = 1;
   P.max_bond = cfg->max_bond_dim;
   P.nobs = n_obs;
   P.nprocs = nprocs;

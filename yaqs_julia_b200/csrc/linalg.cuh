@@ -24,6 +24,7 @@ struct LinalgSmem {
   cplx tau[SVD_MAX_COLS];
   int rot_count;
   int flag;
+  int blocked;  // this run may reorder sums: panel QR and short rotations
 };
 
 // ---------------------------------------------------------------------------
@@ -219,6 +220,240 @@ static __device__ __forceinline__ void dev_qr_extract_r(const cplx* H, int m, in
   cta_sync();
 }
 
+// ---------------------------------------------------------------------------
+// Panel Householder QR
+// ---------------------------------------------------------------------------
+// The column loop above is a chain of four barriers and a pass over the
+// trailing matrix in L2 per column: 128 x 64 took about 860 us with its Q.
+// Here QR_PANEL columns are factored in shared memory, one barrier a column
+// (each warp forms the reflector for itself), and every other column is
+// loaded once a panel into the registers of one warp, which applies all
+// reflectors of the panel to it without a barrier.  Q is formed the same way
+// from the last panel to the first.  The sums run in another order than the
+// column loop's, so it serves the runs that do not cut between equal Schmidt
+// values of a 2-site TDVP split (see SMALL_N in krylov.cuh): circuits, and
+// the one-site and dynamic sweeps.
+#define QR_PANEL 16
+#define QR_PANEL_MAX_ROWS 256
+
+// Applies the reflectors ja <= j < jb (their tails below the diagonal of the
+// panel V, ld m, column ja first) to the columns c0 <= c < c1 of X: ascending
+// with conj(tau) (Q^H X), or descending with tau (Q X).  Columns c < ident
+// start as unit vectors e_c.  Each warp takes CG columns of 32 CH rows.
+template <int CH, int CG>
+static __device__ __noinline__ void qr_apply(cplx* X, int ld, int c0, int c1, const cplx* V, int m, int ja, int jb,
+                                             bool ascending, int ident, const cplx* tau) {
+  constexpr int NV = 2 * CG;
+  constexpr int SH = NV == 2 ? 4 : NV == 4 ? 3 : NV == 8 ? 2 : 1;  // lane of value v: v << SH
+  const int lane = ltid() & 31, wid = ltid() >> 5;
+#pragma unroll 1
+  for (int cb = c0 + wid * CG; cb < c1; cb += NW * CG) {
+    cplx x[CG][CH];
+#pragma unroll
+    for (int g = 0; g < CG; ++g)
+#pragma unroll
+      for (int q = 0; q < CH; ++q) {
+        const int i = lane + 32 * q, c = cb + g;
+        x[g][q] = make_double2(0.0, 0.0);
+        if (c < c1 && i < m) {
+          if (c < ident)
+            x[g][q].x = i == c ? 1.0 : 0.0;
+          else
+            x[g][q] = X[i + ld * c];
+        }
+      }
+#pragma unroll 1
+    for (int jj = ja; jj < jb; ++jj) {
+      const int j = ascending ? jj : jb - 1 - (jj - ja);
+      cplx t = tau[j];
+      if (ascending) t.y = -t.y;
+      cplx v[CH];
+      double d[NV];
+#pragma unroll
+      for (int e = 0; e < NV; ++e) d[e] = 0.0;
+#pragma unroll
+      for (int q = 0; q < CH; ++q) {
+        const int i = lane + 32 * q;
+        v[q] = make_double2(i == j ? 1.0 : 0.0, 0.0);
+        if (i > j && i < m) v[q] = V[i + m * (j - ja)];
+#pragma unroll
+        for (int g = 0; g < CG; ++g) {
+          cplx a = make_double2(d[2 * g], d[2 * g + 1]);
+          cfmac(a, v[q], x[g][q]);
+          d[2 * g] = a.x;
+          d[2 * g + 1] = a.y;
+        }
+      }
+      warp_sum_multi<NV>(d);
+#pragma unroll
+      for (int g = 0; g < CG; ++g) {
+        const cplx a = cmul(make_double2(__shfl_sync(0xffffffffu, d[0], (2 * g) << SH),
+                                         __shfl_sync(0xffffffffu, d[0], (2 * g + 1) << SH)),
+                            t);
+        const cplx na = make_double2(-a.x, -a.y);
+#pragma unroll
+        for (int q = 0; q < CH; ++q) cfma(x[g][q], na, v[q]);
+      }
+    }
+#pragma unroll
+    for (int g = 0; g < CG; ++g)
+#pragma unroll
+      for (int q = 0; q < CH; ++q) {
+        const int i = lane + 32 * q;
+        if (cb + g < c1 && i < m) X[i + ld * (cb + g)] = x[g][q];
+      }
+  }
+}
+
+// Householder factorisation of the columns ja .. jb-1 of the panel V (m x
+// (pe - ja) in shared memory, ld m) with the columns up to pe updated.
+template <int CH>
+static __device__ __noinline__ void qr_panel(cplx* V, int m, int ja, int jb, int pe, double null_abs, cplx* tau) {
+  const int lane = ltid() & 31, wid = ltid() >> 5;
+  cplx v[CH];
+  double diag = 0.0;
+  int pending = -1;  // column whose reflector warp 0 still holds
+#pragma unroll 1
+  for (int j = ja; j < jb; ++j) {
+    if (wid == 0 && pending >= 0) {
+      cplx* pc = V + m * (pending - ja);
+#pragma unroll
+      for (int q = 0; q < CH; ++q) {
+        const int i = lane + 32 * q;
+        if (i > pending && i < m) pc[i] = v[q];
+        if (i == pending) pc[i] = make_double2(diag, 0.0);
+      }
+    }
+    const cplx* col = V + m * (j - ja);
+    double s = 0.0;
+#pragma unroll
+    for (int q = 0; q < CH; ++q) {
+      const int i = lane + 32 * q;
+      v[q] = i > j && i < m ? col[i] : make_double2(0.0, 0.0);
+      s += cabs2(v[q]);
+    }
+    const double xn2 = warp_sum(s);
+    const cplx alpha = col[j];
+    const double full = sqrt(cabs2(alpha) + xn2);
+    cplx t = make_double2(0.0, 0.0);
+    pending = j;
+    if (full <= null_abs || (xn2 == 0.0 && alpha.y == 0.0)) {
+#pragma unroll
+      for (int q = 0; q < CH; ++q) v[q] = make_double2(0.0, 0.0);
+      diag = alpha.x;
+      // alpha keeps its (null) imaginary part in place of a real diagonal
+      if (alpha.y != 0.0) pending = -2 - j;
+    } else {
+      const double beta = (alpha.x >= 0.0) ? -full : full;
+      const double rb = 1.0 / beta;
+      t = make_double2((beta - alpha.x) * rb, -alpha.y * rb);
+      const cplx amb = make_double2(alpha.x - beta, alpha.y);
+      const double rd = 1.0 / cabs2(amb);
+      const cplx scale = make_double2(amb.x * rd, -amb.y * rd);
+#pragma unroll
+      for (int q = 0; q < CH; ++q) v[q] = cmul(v[q], scale);
+      diag = beta;
+      const cplx ct = cconj(t);
+#pragma unroll 1
+      for (int c = j + 1 + wid; c < pe; c += NW) {
+        cplx* xc = V + m * (c - ja);
+        cplx x[CH];
+        cplx a = make_double2(0.0, 0.0);
+        const cplx xj = xc[j];
+#pragma unroll
+        for (int q = 0; q < CH; ++q) {
+          const int i = lane + 32 * q;
+          x[q] = i > j && i < m ? xc[i] : make_double2(0.0, 0.0);
+          cfmac(a, v[q], x[q]);
+        }
+        double d[2] = {a.x, a.y};
+        warp_sum_multi<2>(d);
+        a = cadd(xj, make_double2(__shfl_sync(0xffffffffu, d[0], 0), __shfl_sync(0xffffffffu, d[0], 16)));
+        a = cmul(a, ct);
+        const cplx na = make_double2(-a.x, -a.y);
+#pragma unroll
+        for (int q = 0; q < CH; ++q) {
+          const int i = lane + 32 * q;
+          if (i > j && i < m) {
+            cfma(x[q], na, v[q]);
+            xc[i] = x[q];
+          }
+        }
+        if (lane == 0) xc[j] = csub(xj, a);
+      }
+    }
+    if (wid == 0 && lane == 0) tau[j] = t;
+    if (pending < -1) {  // null column with a complex head: zero its tail, leave the head
+      cta_sync();        // every warp has read it
+      if (wid == 0)
+        for (int i = j + 1 + lane; i < m; i += 32) V[i + m * (j - ja)] = make_double2(0.0, 0.0);
+      pending = -1;
+    }
+    cta_sync();
+  }
+  if (wid == 0 && pending >= 0) {
+    cplx* pc = V + m * (pending - ja);
+#pragma unroll
+    for (int q = 0; q < CH; ++q) {
+      const int i = lane + 32 * q;
+      if (i > pending && i < m) pc[i] = v[q];
+      if (i == pending) pc[i] = make_double2(diag, 0.0);
+    }
+  }
+  cta_sync();
+}
+
+static __device__ __forceinline__ void qr_apply_rows(cplx* X, int ld, int c0, int c1, const cplx* V, int m, int ja,
+                                                     int jb, bool ascending, int ident, const cplx* tau) {
+  if (m <= 32)
+    qr_apply<1, 4>(X, ld, c0, c1, V, m, ja, jb, ascending, ident, tau);
+  else if (m <= 64)
+    qr_apply<2, 2>(X, ld, c0, c1, V, m, ja, jb, ascending, ident, tau);
+  else if (m <= 128)
+    qr_apply<4, 2>(X, ld, c0, c1, V, m, ja, jb, ascending, ident, tau);
+  else
+    qr_apply<8, 1>(X, ld, c0, c1, V, m, ja, jb, ascending, ident, tau);
+}
+
+// dev_qr_factor by panels: H (m x n) in place, m <= QR_PANEL_MAX_ROWS; sb
+// holds m x QR_PANEL values.  CTA-collective.
+static __device__ __noinline__ void dev_qr_factor_panel(cplx* H, int m, int n, cplx* sb, LinalgSmem& ls, RedScratch& rs) {
+  ProfScope prof_scope_(PF_QR);
+  const int kq = min(m, n);
+  const double null_abs = QR_NULL_TOL * sqrt(cta_norm2(H, (long long)m * n, rs));
+  for (int ja = 0; ja < kq; ja += QR_PANEL) {
+    const int pe = min(ja + QR_PANEL, n), jb = min(ja + QR_PANEL, kq);
+    cplx* P = H + m * ja;
+    for (int e = ltid(); e < m * (pe - ja); e += NT) sb[e] = P[e];
+    cta_sync();
+    if (m <= 32)
+      qr_panel<1>(sb, m, ja, jb, pe, null_abs, ls.tau);
+    else if (m <= 64)
+      qr_panel<2>(sb, m, ja, jb, pe, null_abs, ls.tau);
+    else if (m <= 128)
+      qr_panel<4>(sb, m, ja, jb, pe, null_abs, ls.tau);
+    else
+      qr_panel<8>(sb, m, ja, jb, pe, null_abs, ls.tau);
+    for (int e = ltid(); e < m * (pe - ja); e += NT) P[e] = sb[e];
+    qr_apply_rows(H, m, pe, n, sb, m, ja, jb, true, 0, ls.tau);
+    cta_sync();
+  }
+}
+
+// dev_qr_formq by panels.  CTA-collective.
+static __device__ __noinline__ void dev_qr_formq_panel(const cplx* H, int m, int n, cplx* Q, cplx* sb, LinalgSmem& ls) {
+  ProfScope prof_scope_(PF_QRQ);
+  const int kq = min(m, n), last = (kq - 1) / QR_PANEL * QR_PANEL;
+  for (int ja = last; ja >= 0; ja -= QR_PANEL) {
+    const int jb = min(ja + QR_PANEL, kq);
+    if (kq > QR_PANEL || n > QR_PANEL)  // otherwise the panel is still there
+      for (int e = ltid(); e < m * (jb - ja); e += NT) sb[e] = H[m * ja + e];
+    cta_sync();
+    qr_apply_rows(Q, m, ja, kq, sb, m, ja, jb, false, jb, ls.tau);
+    cta_sync();
+  }
+}
+
 // Thin QR of M (m x n, col-major), load(e) its element e: store_q(e, q), e < m k,
 // stores from Q (m x k) at q, Rout becomes R (k x n), k = min(m, n).  H and Qg
 // are work matrices in global memory; a problem that fits runs in the shared buffer sb
@@ -229,6 +464,17 @@ template <class Load, class Store>
 static __device__ __forceinline__ void dev_qr_thin(int m, int n, Load load, cplx* H, Store store_q, cplx* Qg, cplx* Rout,
                                                    cplx* sb, int cap, LinalgSmem& ls, RedScratch& rs) {
   const int k = min(m, n);
+  if (ls.blocked && m <= QR_PANEL_MAX_ROWS) {
+    cta_sync();
+    for (int e = ltid(); e < m * n; e += NT) H[e] = load(e);
+    cta_sync();
+    dev_qr_factor_panel(H, m, n, sb, ls, rs);
+    dev_qr_formq_panel(H, m, n, Qg, sb, ls);
+    dev_qr_extract_r(H, m, n, Rout);
+    for (int e = ltid(); e < m * k; e += NT) store_q(e, Qg);
+    cta_sync();
+    return;
+  }
   cplx* h = m * n <= cap ? sb : H;
   cplx* q = (m * n + m * k <= cap) ? sb + m * n : Qg;
   cta_sync();  // the shared buffer's last readers are done
@@ -389,6 +635,82 @@ static __device__ __forceinline__ void smem_rotate_round(cplx* sb, int ld, int q
   cta_sync();
 }
 
+// The same round with LP lanes a pair, the four sums reduced together and the
+// rotation from two reciprocal square roots: with R = sqrt(d^2 + 4 |g|^2),
+//   cos^2 = (1 + |d| / R) / 2,  sin / |g| = 1 / (R cos)
+// instead of a chain of rsqrt, sqrt, division and rsqrt.  A round is one
+// dependent chain of loads, shuffles and these, so its length is its cost.
+// For the runs that may reorder sums.
+template <int LP, class PairFn>
+static __device__ __forceinline__ void smem_rotate_short(cplx* sb, int ld, int q, int npairs, PairFn pairs, double tol2,
+                                                         int* rot) {
+  const int hl = ltid() & (LP - 1), grp = ltid() / LP;
+  const int base = (ltid() & 31) & ~(LP - 1);
+  const unsigned mask = ((LP == 32 ? 0u : (1u << (LP & 31))) - 1u) << base;
+#pragma unroll 1
+  for (int k = grp; k < npairs; k += NT / LP) {
+    int i, j;
+    pairs(k, i, j);
+    if (i < 0 || j < 0) continue;
+    cplx* bi = sb + ld * i;
+    cplx* bj = sb + ld * j;
+    double d4[4] = {0.0, 0.0, 0.0, 0.0};  // |b_i|^2, |b_j|^2, b_i^H b_j
+#pragma unroll 2
+    for (int r = hl; r < q; r += LP) {
+      const cplx x = bi[r], y = bj[r];
+      d4[0] = fma(x.x, x.x, fma(x.y, x.y, d4[0]));
+      d4[1] = fma(y.x, y.x, fma(y.y, y.y, d4[1]));
+      d4[2] = fma(x.x, y.x, fma(x.y, y.y, d4[2]));
+      d4[3] = fma(x.x, y.y, fma(-x.y, y.x, d4[3]));
+    }
+    {  // butterfly over the pair's lanes, halving the values twice
+      bool up = (hl & (LP / 2)) != 0;
+#pragma unroll
+      for (int e = 0; e < 2; ++e) {
+        const double keep = up ? d4[e + 2] : d4[e], give = up ? d4[e] : d4[e + 2];
+        d4[e] = keep + __shfl_xor_sync(mask, give, LP / 2);
+      }
+      up = (hl & (LP / 4)) != 0;
+      const double keep = up ? d4[1] : d4[0], give = up ? d4[0] : d4[1];
+      d4[0] = keep + __shfl_xor_sync(mask, give, LP / 4);
+#pragma unroll
+      for (int o = LP / 8; o > 0; o >>= 1) d4[0] += __shfl_xor_sync(mask, d4[0], o);
+    }
+    const double al = __shfl_sync(mask, d4[0], base), be = __shfl_sync(mask, d4[0], base + LP / 4);
+    const double gx = __shfl_sync(mask, d4[0], base + LP / 2), gy = __shfl_sync(mask, d4[0], base + 3 * LP / 4);
+    const double g2 = fma(gx, gx, gy * gy);
+    if (!(g2 > tol2 * (al * be))) continue;
+    if (hl == 0) *rot = 1;  // any rotation keeps the sweeps going
+    const double d = be - al;
+    const double h = rsqrt(fma(d, d, 4.0 * g2));
+    const double c2 = fma(0.5 * fabs(d), h, 0.5);
+    const double rc = rsqrt(c2);
+    const double c = c2 * rc, f = d < 0.0 ? -h * rc : h * rc;
+    const cplx se = make_double2(f * gx, f * gy);
+#pragma unroll 2
+    for (int r = hl; r < q; r += LP) {
+      const cplx x = bi[r], y = bj[r];
+      // b_i <- c b_i - conj(se) b_j,  b_j <- se b_i + c b_j
+      bi[r] = make_double2(fma(c, x.x, fma(-se.x, y.x, -se.y * y.y)), fma(c, x.y, fma(-se.x, y.y, se.y * y.x)));
+      bj[r] = make_double2(fma(c, y.x, fma(se.x, x.x, -se.y * x.y)), fma(c, y.y, fma(se.x, x.y, se.y * x.x)));
+    }
+  }
+  cta_sync();
+}
+
+// One round of a sweep in the form the run takes; a pair gets 16 lanes where
+// the round's pairs leave that many, else 8.
+template <class PairFn>
+static __device__ __forceinline__ void rotate_round(cplx* sb, int ld, int q, int npairs, PairFn pairs, double tol,
+                                                    LinalgSmem& ls, bool blocked) {
+  if (!blocked)
+    smem_rotate_round(sb, ld, q, q, npairs, pairs, tol, &ls.rot_count);
+  else if (npairs * 16 <= NT)
+    smem_rotate_short<16>(sb, ld, q, npairs, pairs, tol * tol, &ls.rot_count);
+  else
+    smem_rotate_short<8>(sb, ld, q, npairs, pairs, tol * tol, &ls.rot_count);
+}
+
 // Stage columns [c0, c0+nc0) and [c1, c1+nc1) of B into sb (ld = q), or
 // write them back.
 static __device__ __forceinline__ void svd_stage(cplx* sb, int ld, const SvdWork& w, int q, int c0, int nc0, int c1, int nc1,
@@ -434,15 +756,19 @@ static __device__ __noinline__ SvdResult dev_svd(const cplx* M, int m, int n, in
   // A problem that fits the shared buffer stays there: the factored matrix
   // (at the end of the buffer, or in global memory) and B for all sweeps.
   const bool resident = q * p <= SVD_SMEM_CPLX;
-  const bool h_shared = mm * nn <= SVD_SMEM_CPLX;
-  const bool both = resident && mm * nn + q * p <= SVD_SMEM_CPLX;
+  const bool panel = ls.blocked && mm <= QR_PANEL_MAX_ROWS;
+  const bool h_shared = !panel && mm * nn <= SVD_SMEM_CPLX;
+  const bool both = resident && (panel || mm * nn + q * p <= SVD_SMEM_CPLX);
   cplx* H = h_shared ? sb + (SVD_SMEM_CPLX - mm * nn) : w.X;
   for (int e = tid; e < mm * nn; e += NT) {
     int r = (int)(e % mm), c = (int)(e / mm);
     H[e] = res.tr ? M[e] : cconj(M[c + (long long)m * r]);
   }
   cta_sync();
-  dev_qr_factor(H, mm, nn, ls, rs);
+  if (panel)
+    dev_qr_factor_panel(H, mm, nn, sb, ls, rs);
+  else
+    dev_qr_factor(H, mm, nn, ls, rs);
   // B = R^H (nn x k): B[r, c] = conj(R[c, r]) for c <= r
   cplx* B0 = both ? sb : w.B;
   for (int e = tid; e < q * p; e += NT) {
@@ -455,6 +781,7 @@ static __device__ __noinline__ SvdResult dev_svd(const cplx* M, int m, int n, in
     cta_sync();
   }
   const double tol = 2.220446049250313e-16 * q;
+  const bool blocked = ls.blocked != 0;
   const int ld = q;
   const int b = svd_block_size(q, p);
   const int nb = (p + b - 1) / b;
@@ -468,16 +795,18 @@ static __device__ __noinline__ SvdResult dev_svd(const cplx* M, int m, int n, in
       if (!resident) svd_stage(sb, ld, w, q, c0, nc, 0, 0, false);
       cplx* cols = resident ? sb + ld * c0 : sb;
       for (int round = 0; round < be2 - 1; ++round) {
-        smem_rotate_round(cols, ld, q, q, be2 / 2,
-                          [&](int pr, int& i, int& j) {
-                            int ta = pr, tb = be2 - 1 - pr;
-                            int a = ta == 0 ? 0 : ((ta - 1 - round + 2 * (be2 - 1)) % (be2 - 1)) + 1;
-                            int c = tb == 0 ? 0 : ((tb - 1 - round + 2 * (be2 - 1)) % (be2 - 1)) + 1;
-                            i = min(a, c);
-                            j = max(a, c);
-                            if (j >= nc) i = j = -1;
-                          },
-                          tol, &ls.rot_count);
+        rotate_round(cols, ld, q, be2 / 2,
+                     [&](int pr, int& i, int& j) {
+                       // round-robin: place t holds column ((t - 1 - round) mod (be2 - 1)) + 1, place 0 column 0
+                       const int ta = pr, tb = be2 - 1 - pr;
+                       int a = ta == 0 ? 0 : ta - round, c = tb == 0 ? 0 : tb - round;
+                       if (ta != 0 && a < 1) a += be2 - 1;
+                       if (tb != 0 && c < 1) c += be2 - 1;
+                       i = min(a, c);
+                       j = max(a, c);
+                       if (j >= nc) i = j = -1;
+                     },
+                     tol, ls, blocked);
       }
       if (!resident) svd_stage(sb, ld, w, q, c0, nc, 0, 0, true);
     }
@@ -493,17 +822,17 @@ static __device__ __noinline__ SvdResult dev_svd(const cplx* M, int m, int n, in
         cplx* cols = resident ? sb + ld * c0 : sb;
         const int joff = resident ? c1 - c0 : n0;
         for (int t = 0; t < b; ++t) {
-          smem_rotate_round(cols, ld, q, q, b,
-                            [&](int kk, int& i, int& j) {
-                              int jj = (kk + t) % b;
-                              if (kk >= n0 || jj >= n1) {
-                                i = j = -1;
-                              } else {
-                                i = kk;
-                                j = joff + jj;
-                              }
-                            },
-                            tol, &ls.rot_count);
+          rotate_round(cols, ld, q, b,
+                       [&](int kk, int& i, int& j) {
+                         const int jj = kk + t < b ? kk + t : kk + t - b;
+                         if (kk >= n0 || jj >= n1) {
+                           i = j = -1;
+                         } else {
+                           i = kk;
+                           j = joff + jj;
+                         }
+                       },
+                       tol, ls, blocked);
         }
         if (!resident) svd_stage(sb, ld, w, q, c0, n0, c1, n1, true);
       }

@@ -106,6 +106,7 @@ static __device__ void run_units(const DevParams& P, CtaSmem& sm, int first, int
   int* wsi = P.wsi + (long long)slot * P.lay.itotal;
   const int nt = P.num_traj;
   const int total = count * nt;
+  if (ltid() == 0) sm.la.blocked = P.blocked;  // the loop's first barrier publishes it
   for (;;) {
     if (ltid() == 0) sm.bcast_i[7] = atomicAdd(&P.queue[first], 1);
     cta_sync();

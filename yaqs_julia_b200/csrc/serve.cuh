@@ -41,6 +41,7 @@ static __device__ void serve_units(const BatchRun* runs, int nruns, int total_un
     }
     cta_sync();
     const DevParams& P = br.P;
+    if (ltid() == 0) sm.la.blocked = P.blocked;  // published by the barriers before the unit runs
     const int nt = P.num_traj;
     const int local = u - br.unit_begin, k = local / nt, t = local - k * nt, pos = br.first + k;
     cplx* ws = P.ws + (long long)slot * P.lay.total;

@@ -83,6 +83,13 @@ struct DevParams {
   long long kry_n;
   const DevProc* procs;
   const DevObs* obs;
+  // Processes by their left site (both kinds) and 2-site processes by their
+  // right site, 1-site observables by site: entries off[i] .. off[i+1]-1 of
+  // idx are the indices that belong to site i, ascending.
+  const int *p0_off, *p0_idx, *p1_off, *p1_idx, *ob_off, *ob_idx;
+  int blocked;     // panel QR and short Jacobi rounds (LinalgSmem::blocked)
+  int scalar_all;  // every process is a scalar dissipator (pauli_name)
+  int has_lr;      // some process is long-range
   const cplx* psi0;  // arena layout, compact tensors
   const int* chi0;   // [L+1]
   cplx* phi;         // [num_traj][mps_size]
@@ -287,11 +294,11 @@ static __device__ void normalize_center(Ctx& c, const DState& s) {
 // a sweep is a pure gauge move.  Uniform across the CTA.
 static __device__ bool chain_tight(const Ctx& c, const DState& s) {
   bool ok = true;
-  for (int b = 1; b < c.P.L; ++b) {
+  for (int b = 1 + (ltid() & 31); b < c.P.L; b += 32) {
     const int x = s.chi[b];
     if (x > 2 * s.chi[b - 1] || x > 2 * s.chi[b + 1]) ok = false;
   }
-  return ok;
+  return __all_sync(0xffffffffu, ok) != 0;
 }
 
 // normalize! of a state in mixed canonical form around its centre: on a
@@ -838,25 +845,67 @@ static __device__ __forceinline__ bool proc_on(const DevProc& pr, int f1, int f2
   return pr.nsites == 1 ? (pr.s0 == f1 || pr.s0 == f2) : ((pr.s0 == f1 && pr.s1 == f2) || (pr.s0 == f2 && pr.s1 == f1));
 }
 
+// The processes that a noise step may take, in ascending order: all, or those
+// whose left site is one of a gate's sites.
+struct ProcIter {
+  const int *a, *ae, *b, *be;
+  int k, n;
+  __device__ __forceinline__ ProcIter(const DevParams& P, int f1, int f2) {
+    a = ae = b = be = nullptr;
+    k = 0;
+    n = f1 < 0 ? P.nprocs : 0;
+    if (f1 >= 0) {
+      a = P.p0_idx + P.p0_off[f1];
+      ae = P.p0_idx + P.p0_off[f1 + 1];
+      b = P.p0_idx + P.p0_off[f2];
+      be = P.p0_idx + P.p0_off[f2 + 1];
+    }
+  }
+  __device__ __forceinline__ int next() {  // -1 at the end
+    if (n) return k < n ? k++ : -1;
+    if (a < ae && (b >= be || *a < *b)) return *a++;
+    return b < be ? *b++ : -1;
+  }
+};
+
+// prod_k exp(-dt/2 drate_k) over all processes, in order: a warp takes the
+// exponentials 32 at a time.
+static __device__ double scalar_decay(const DevParams& P, double dt) {
+  double f = 1.0;
+  for (int k0 = 0; k0 < P.nprocs; k0 += 32) {
+    const int k = k0 + (ltid() & 31);
+    const double e = k < P.nprocs ? exp(-0.5 * dt * P.procs[k].drate) : 1.0;
+    const int m = min(32, P.nprocs - k0);
+    for (int u = 0; u < m; ++u) f *= __shfl_sync(0xffffffffu, e, u);
+  }
+  return f;
+}
+
 static __device__ __noinline__ void apply_dissipation(Ctx& c, const DState& s, bool full, double dt, int f1 = -1, int f2 = -1) {
   ProfScope prof_scope_(PF_DISS);
   const int L = c.P.L;
   bool all_zero = c.P.all_zero != 0;
   if (f1 >= 0) {
     all_zero = true;
-    for (int k = 0; k < c.P.nprocs; ++k)
+    ProcIter it(c.P, f1, f2);
+    for (int k; (k = it.next()) >= 0;)
       if (proc_on(c.P.procs[k], f1, f2) && c.P.procs[k].gamma != 0.0) all_zero = false;
   }
   // Every dissipator a scalar (Pauli names, Dissipation.jl:14-21, 57-60, 88-91)
   // on a tight chain: the sweep only multiplies the state by their product
   // and moves the centre to site 0 by shape-preserving gauge steps.
-  bool scalar_only = true;
+  bool scalar_only = f1 < 0 ? c.P.scalar_all != 0 : true;
   double fscal = 1.0;
-  for (int k = 0; k < c.P.nprocs; ++k) {
-    const DevProc& pr = c.P.procs[k];
-    if (!proc_on(pr, f1, f2)) continue;
-    if (!pr.pauli_name) scalar_only = false;
-    fscal *= exp(-0.5 * dt * pr.drate);
+  if (f1 < 0) {
+    if (scalar_only) fscal = scalar_decay(c.P, dt);
+  } else {
+    ProcIter it(c.P, f1, f2);
+    for (int k; (k = it.next()) >= 0;) {
+      const DevProc& pr = c.P.procs[k];
+      if (!proc_on(pr, f1, f2)) continue;
+      if (!pr.pauli_name) scalar_only = false;
+      fscal *= exp(-0.5 * dt * pr.drate);
+    }
   }
   if ((!c.P.noise_present || all_zero || scalar_only) && chain_tight(c, s)) {
     shift_oc(c, s, 0);
@@ -879,9 +928,9 @@ static __device__ __noinline__ void apply_dissipation(Ctx& c, const DState& s, b
   }
   cplx* th = c.ws + c.P.lay.th;
   for (int i = L - 1; i >= 0 && !c.sm.fail; --i) {
-    for (int k = 0; k < c.P.nprocs; ++k) {
-      const DevProc& pr = c.P.procs[k];
-      if (pr.nsites == 1 && pr.s0 == i && proc_on(pr, f1, f2)) {
+    for (int z = c.P.p0_off[i]; z < c.P.p0_off[i + 1]; ++z) {
+      const DevProc& pr = c.P.procs[c.P.p0_idx[z]];
+      if (pr.nsites == 1 && proc_on(pr, f1, f2)) {
         cplx* A = site_ptr(c, s, i);
         const long long n = (long long)s.chi[i] * 2 * s.chi[i + 1];
         if (pr.pauli_name) {
@@ -893,9 +942,9 @@ static __device__ __noinline__ void apply_dissipation(Ctx& c, const DState& s, b
       }
     }
     if (i > 0) {
-      for (int k = 0; k < c.P.nprocs && !c.sm.fail; ++k) {
-        const DevProc& pr = c.P.procs[k];
-        if (pr.nsites == 2 && pr.s1 == i && proc_on(pr, f1, f2)) {
+      for (int z = c.P.p1_off[i]; z < c.P.p1_off[i + 1] && !c.sm.fail; ++z) {
+        const DevProc& pr = c.P.procs[c.P.p1_idx[z]];
+        if (proc_on(pr, f1, f2)) {
           if (pr.pauli_name) {  // Pauli names and long-range processes: a scalar at the right site
             cta_scale(site_ptr(c, s, i), (long long)s.chi[i] * 2 * s.chi[i + 1], exp(-0.5 * dt * pr.drate));
             cta_sync();
@@ -922,8 +971,11 @@ static __device__ __noinline__ void stochastic_process(Ctx& c, const DState& s, 
   const int L = c.P.L;
   const double dp = 1.0 - scalar_product(c, s);
   bool jump = false;
-  int ntake = 0;
-  for (int k = 0; k < c.P.nprocs; ++k) ntake += proc_on(c.P.procs[k], f1, f2) ? 1 : 0;
+  int ntake = f1 < 0 ? c.P.nprocs : 0;
+  if (f1 >= 0) {
+    ProcIter it(c.P, f1, f2);
+    for (int k; (k = it.next()) >= 0;) ntake += proc_on(c.P.procs[k], f1, f2) ? 1 : 0;
+  }
   if (ntake > 0) {
     double u1 = draw_uniform(c);
     jump = u1 < dp;
@@ -941,9 +993,10 @@ static __device__ __noinline__ void stochastic_process(Ctx& c, const DState& s, 
   cplx* th = c.ws + c.P.lay.th;
   for (int site = 0; site < L && !c.sm.fail; ++site) {
     shift_oc(c, s, site);
-    for (int k = 0; k < c.P.nprocs; ++k) {
+    for (int z = c.P.p0_off[site]; z < c.P.p0_off[site + 1]; ++z) {
+      const int k = c.P.p0_idx[z];
       const DevProc& pr = c.P.procs[k];
-      if (pr.nsites == 1 && pr.s0 == site && proc_on(pr, f1, f2)) {
+      if (pr.nsites == 1 && proc_on(pr, f1, f2)) {
         double nr = local_norm2(c, site_ptr(c, s, site), s.chi[site], 2, s.chi[site + 1],
                                 pr.pauli_proc ? nullptr : pr.mat);
         if (ltid() == 0) {
@@ -954,9 +1007,10 @@ static __device__ __noinline__ void stochastic_process(Ctx& c, const DState& s, 
       }
     }
     if (site < L - 1) {
-      for (int k = 0; k < c.P.nprocs; ++k) {
+      for (int z = c.P.p0_off[site]; z < c.P.p0_off[site + 1]; ++z) {
+        const int k = c.P.p0_idx[z];
         const DevProc& pr = c.P.procs[k];
-        if (pr.nsites == 2 && !pr.lr && pr.s0 == site && proc_on(pr, f1, f2)) {
+        if (pr.nsites == 2 && !pr.lr && proc_on(pr, f1, f2)) {
           double nr;
           if (pr.pauli_proc) {
             nr = local_norm2(c, site_ptr(c, s, site), s.chi[site], 2, s.chi[site + 1], nullptr);
@@ -975,7 +1029,7 @@ static __device__ __noinline__ void stochastic_process(Ctx& c, const DState& s, 
   }
   // long-range processes after every local candidate (StochasticProcess.jl:169-202);
   // the centre is at site L-1
-  for (int k = 0; k < c.P.nprocs && !c.sm.fail; ++k) {
+  for (int k = 0; c.P.has_lr && k < c.P.nprocs && !c.sm.fail; ++k) {
     const DevProc& pr = c.P.procs[k];
     if (!pr.lr || !proc_on(pr, f1, f2)) continue;
     const double nr = pr.pauli_proc ? local_norm2(c, site_ptr(c, s, L - 1), s.chi[L - 1], 2, s.chi[L], nullptr)
@@ -1061,9 +1115,8 @@ static __device__ double env_expect(Ctx& c, const cplx* A, const cplx* T, int l,
 static __device__ __noinline__ bool local_by_envs(Ctx& c, const DState& s, int col) {
   const DevParams& P = c.P;
   const int L = P.L;
-  bool any1 = false;
-  for (int k = 0; k < P.nobs; ++k) any1 |= P.obs[k].kind == OBS_LOCAL1;
-  if (!any1 || !chain_tight(c, s)) return false;
+  const int nlocal = P.ob_off[L];
+  if (nlocal == 0 || !chain_tight(c, s)) return false;
   long long need = 0;
   for (int b = 1; b <= L; ++b) need += (long long)s.chi[b] * s.chi[b];
   cplx* Rs;
@@ -1100,14 +1153,13 @@ static __device__ __noinline__ bool local_by_envs(Ctx& c, const DState& s, int c
     const int l = s.chi[i], r = s.chi[i + 1];
     const cplx* A = site_ptr(c, s, i);
     off -= (long long)r * r;
-    bool here = false;
-    for (int k = 0; k < P.nobs; ++k) here |= P.obs[k].kind == OBS_LOCAL1 && P.obs[k].s0 == i;
-    if (here) {
+    const int ob0 = P.ob_off[i], ob1 = P.ob_off[i + 1];
+    if (ob0 < ob1) {
       // T1[a,q,r'] = sum_r A[a,q,r] R_{i+1}[r,r'];  T3[a',q,r'] = sum_a E_i[a,a'] T1[a,q,r']
       cta_gemm(gemm_args(2 * l, r, r, A, 1, 2 * l, Rs + off, 1, r, T1, 1, 2 * l), gs);
       cta_gemm(gemm_args(l, 2 * r, l, E0, l, 1, T1, 1, l, T3, 1, l), gs);
-      for (int k = 0; k < P.nobs; ++k) {
-        if (P.obs[k].kind != OBS_LOCAL1 || P.obs[k].s0 != i) continue;
+      for (int z = ob0; z < ob1; ++z) {
+        const int k = P.ob_idx[z];
         const double v = env_expect(c, A, T3, l, r, P.obs[k].mat);
         if (ltid() == 0) vals[k] = v;
       }
@@ -1122,9 +1174,10 @@ static __device__ __noinline__ bool local_by_envs(Ctx& c, const DState& s, int c
     }
   }
   cta_sync();
-  if (ltid() == 0)
-    for (int k = 0; k < P.nobs; ++k)
-      if (P.obs[k].kind == OBS_LOCAL1) P.traj_out[((long long)c.traj * P.nobs + k) * P.ncols + col] = vals[k];
+  for (int z = ltid(); z < nlocal; z += NT) {
+    const int k = P.ob_idx[z];
+    P.traj_out[((long long)c.traj * P.nobs + k) * P.ncols + col] = vals[k];
+  }
   cta_sync();
   return true;
 }
