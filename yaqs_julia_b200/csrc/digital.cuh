@@ -89,6 +89,8 @@ static __device__ __noinline__ void apply_window_tdvp(Ctx& c, const DState& s, c
   if (c.sm.fail) return;
   identity_env(c, envL(c, s1), s.chi[s1], 1);
   identity_env(c, envR(c, s2 + 1), s.chi[s2 + 1], 1);
+  if (ltid() == 0) c.sm.id_left[s1] = c.sm.id_right[s2 + 1] = 1;
+  cta_sync();
   for (int j = n - 1; j >= 1; --j) update_right_w(c, s, s1 + j, eR[j]);
   for (int j = 0; j + 2 < n && !c.sm.fail; ++j) {
     const int i = s1 + j, l = s.chi[i], r = s.chi[i + 2];

@@ -236,6 +236,10 @@ bool make_tc_map(CUtensorMap* out, const void* base, long long pitch, long long 
 struct HostWMat {
   int no = 0, ni = 0;
   int ident = 0;
+  int idc = -1;
+  bool planned = false;
+  HPlan plan{};
+  std::vector<HSeg> seg;
   std::vector<int> rowp, col;
   std::vector<hcd> val;
 };
@@ -259,17 +263,96 @@ HostWMat build_wmat(int no, int ni, F f) {
   return m;
 }
 
+// Channels of every bond in which the left (right) environment next to
+// isometric sites is the identity: reached from the boundary through W = 1
+// alone.  -1 where there is none.
+template <class F>
+void identity_channels(int L, const int* w, F Wat, std::vector<int>& left, std::vector<int>& right) {
+  left.assign(L + 1, -1);
+  right.assign(L + 1, -1);
+  auto is = [&](int i, int m, int mr, bool one) {
+    for (int po = 0; po < 2; ++po)
+      for (int pi = 0; pi < 2; ++pi)
+        if (Wat(i, m, po, pi, mr) != hcd(one && po == pi ? 1.0 : 0.0)) return false;
+    return true;
+  };
+  left[0] = w[0] == 1 ? 0 : -1;
+  for (int i = 0; i < L && left[i] >= 0; ++i)
+    for (int mr = 0; mr < w[i + 1] && left[i + 1] < 0; ++mr) {
+      bool ok = true;
+      for (int m = 0; m < w[i] && ok; ++m) ok = is(i, m, mr, m == left[i]);
+      if (ok) left[i + 1] = mr;
+    }
+  right[L] = w[L] == 1 ? 0 : -1;
+  for (int i = L - 1; i >= 0 && right[i + 1] >= 0; --i)
+    for (int m = 0; m < w[i] && right[i] < 0; ++m) {
+      bool ok = true;
+      for (int mr = 0; mr < w[i + 1] && ok; ++mr) ok = is(i, m, mr, mr == right[i + 1]);
+      if (ok) right[i] = m;
+    }
+}
+
+// The structured product of an effective-Hamiltonian map M[(p' + D m'),
+// (m + wl p)] with identity channels il and ir, kept when it multiplies fewer
+// chi^3 blocks than the general one (wl + wr a physical index).
+void plan_heff(HostWMat& m, int D, int wl, int wr, int il, int ir) {
+  if (il < 0 || ir < 0) return;
+  HPlan& pl = m.plan;
+  pl = HPlan{};
+  pl.il = il;
+  pl.ir = ir;
+  int lo = wl, hi = -1;
+  for (int pp = 0; pp < D; ++pp) {
+    pl.off[pp] = (int)m.seg.size();
+    for (int mp = 0; mp < wr; ++mp) {
+      const int o = pp + D * mp;
+      for (int z = m.rowp[o]; z < m.rowp[o + 1]; ++z) {
+        const int mi = m.col[z] % wl, p = m.col[z] / wl;
+        const cplx v = make_double2(m.val[z].real(), m.val[z].imag());
+        if (mi == il && mp == ir) {
+          pl.loc[pp + D * p] = v;
+          pl.has_loc = 1;
+          continue;
+        }
+        HSeg q{};
+        q.p = p;
+        q.coef = v;
+        q.side = mp == ir ? 0 : mi == il ? 1 : 2;
+        q.m = mp == ir ? mi : mp;
+        q.g = mi;  // rebased below
+        if (q.side == 2) {
+          lo = std::min(lo, mi);
+          hi = std::max(hi, mi);
+        }
+        m.seg.push_back(q);
+      }
+    }
+  }
+  pl.nseg = (int)m.seg.size();
+  for (int pp = D; pp < 5; ++pp) pl.off[pp] = pl.nseg;
+  pl.nt1 = hi >= 0 ? hi - lo + 1 : 0;
+  pl.t1m = hi >= 0 ? lo : 0;
+  for (auto& q : m.seg)
+    if (q.side == 2) q.g -= lo;
+  bool every = true;  // a block without segments would not start the GEMM's pipeline
+  for (int pp = 0; pp < D; ++pp) every = every && pl.off[pp + 1] > pl.off[pp];
+  m.planned = every && pl.nseg <= HEFF_MAX_SEGS && pl.nt1 * D + pl.nseg <= (wl + wr) * D;
+}
+
 // The sparse maps of an MPO (W(i, m, p_out, p_in, m') via Wat) in the order
 // heff1[L], heff2[L-1] (merged two-site W of Algorithms.jl:639-643),
 // envL[L], envR[L].
 template <class F>
 void append_mpo_wmats(int L, const int* w, F Wat, std::vector<HostWMat>& all) {
+  std::vector<int> left, right;
+  identity_channels(L, w, Wat, left, right);
   for (int i = 0; i < L; ++i) {  // heff1: M[(p' + 2 m'), (m + wl p)]
     int wl = w[i], wr = w[i + 1];
     all.push_back(build_wmat(2 * wr, wl * 2, [&](int o, int in) {
       int pp = o % 2, mp = o / 2, m = in % wl, p = in / wl;
       return Wat(i, m, pp, p, mp);
     }));
+    plan_heff(all.back(), 2, wl, wr, left[i], right[i + 1]);
   }
   for (int i = 0; i + 1 < L; ++i) {  // heff2 (merged)
     int wl = w[i], wm = w[i + 1], wr = w[i + 2];
@@ -288,6 +371,7 @@ void append_mpo_wmats(int L, const int* w, F Wat, std::vector<HostWMat>& all) {
       int pp = o % 4, mp = o / 4, m = in % wl, p = in / wl;
       return G[m + (size_t)wl * (pp + 4 * (p + 4 * (size_t)mp))];
     }));
+    plan_heff(all.back(), 4, wl, wr, left[i], right[i + 2]);
   }
   for (int i = 0; i < L; ++i) {  // envL: M[(po + 2 m'), (ml + wl pi)]
     int wl = w[i], wr = w[i + 1];
@@ -295,6 +379,7 @@ void append_mpo_wmats(int L, const int* w, F Wat, std::vector<HostWMat>& all) {
       int po = o % 2, mp = o / 2, ml = in % wl, pi = in / wl;
       return Wat(i, ml, po, pi, mp);
     }));
+    all.back().idc = left[i + 1];
   }
   for (int i = 0; i < L; ++i) {  // envR: M[(po + 2 ml), (pi + 2 mr)]
     int wl = w[i], wr = w[i + 1];
@@ -302,6 +387,7 @@ void append_mpo_wmats(int L, const int* w, F Wat, std::vector<HostWMat>& all) {
       int po = o % 2, ml = o / 2, pi = in % 2, mr = in / 2;
       return Wat(i, ml, po, pi, mr);
     }));
+    all.back().idc = right[i];
   }
 }
 
@@ -362,6 +448,14 @@ int upload_wmats(yaqs_ctx* ctx, DevMem& dm, const std::vector<HostWMat>& all, st
   }
   int* di = nullptr;
   cplx* dv = nullptr;
+  HPlan* dplan = nullptr;  // one slot a map
+  HSeg* dseg = nullptr;
+  std::vector<HPlan> hp;
+  std::vector<HSeg> hs;
+  size_t nseg = 0;
+  for (auto& m : all) nseg += m.planned ? m.seg.size() : 0;
+  CUDA_TRY(ctx, dm.alloc(&dplan, all.size()));
+  CUDA_TRY(ctx, dm.alloc(&dseg, nseg));
   CUDA_TRY(ctx, dm.alloc(&di, nint));
   CUDA_TRY(ctx, dm.alloc(&dv, nval));
   std::vector<int> hi;
@@ -375,6 +469,15 @@ int upload_wmats(yaqs_ctx* ctx, DevMem& dm, const std::vector<HostWMat>& all, st
     w.ni = m.ni;
     w.nnz = (int)m.val.size();
     w.ident = m.ident;
+    w.idc = m.idc;
+    w.plan = m.planned ? dplan + views.size() : nullptr;
+    if (m.planned) {
+      HPlan pl = m.plan;
+      pl.seg = dseg + hs.size();
+      hp.resize(views.size() + 1);
+      hp.back() = pl;
+      hs.insert(hs.end(), m.seg.begin(), m.seg.end());
+    }
     w.rowp = di + hi.size();
     hi.insert(hi.end(), m.rowp.begin(), m.rowp.end());
     w.col = di + hi.size();
@@ -382,6 +485,10 @@ int upload_wmats(yaqs_ctx* ctx, DevMem& dm, const std::vector<HostWMat>& all, st
     w.val = dv + hv.size();
     hv.insert(hv.end(), m.val.begin(), m.val.end());
     views.push_back(w);
+  }
+  if (!hp.empty()) {
+    CUDA_TRY(ctx, cudaMemcpy(dplan, hp.data(), hp.size() * sizeof(HPlan), cudaMemcpyHostToDevice));
+    CUDA_TRY(ctx, cudaMemcpy(dseg, hs.data(), hs.size() * sizeof(HSeg), cudaMemcpyHostToDevice));
   }
   CUDA_TRY(ctx, cudaMemcpy(di, hi.data(), hi.size() * sizeof(int), cudaMemcpyHostToDevice));
   CUDA_TRY(ctx, cudaMemcpy(dv, hv.data(), hv.size() * sizeof(hcd), cudaMemcpyHostToDevice));
@@ -1047,9 +1154,12 @@ static int analog_begin_impl(yaqs_ctx* ctx, const yaqs_mps_desc* psi0, const yaq
   };
   std::vector<HostWMat> all;
   append_mpo_wmats(L, w.data(), Wat, all);
+  std::vector<int> left, right;
+  identity_channels(L, w.data(), Wat, left, right);
   for (int b = 0; b <= L; ++b) {  // bond: identity on the MPO bond, physical dimension 1
     all.push_back(build_wmat(w[b], w[b], [&](int o, int in) { return hcd(o == in ? 1.0 : 0.0, 0.0); }));
     all.back().ident = 1;
+    plan_heff(all.back(), 1, w[b], w[b], left[b], right[b]);
   }
   for (auto& m : all)
     if (m.ni > WAPPLY_MAXI || m.no > WAPPLY_MAXI || (int)m.val.size() > WAPPLY_MAXNNZ)

@@ -21,10 +21,34 @@
 #define WAPPLY_LB 8  // inputs a thread loads back to back
 #define KRYLOV_MAX 32
 
+// Structure of an effective Hamiltonian whose left environment holds the
+// identity in MPO channel il and the right one in channel ir, as an MPO's
+// running-sum form gives them next to isometric sites.  With those blocks
+// taken out the product is, per output physical index p',
+//   y_{p'} = sum_s coef_s A_s B_s + sum_p loc[p', p] x_p
+// over segments L_m x_p (side 0, the term ends on the left), x_p R_m' (side
+// 1, it starts there) and (L_m x)_p R_m' (side 2, it passes through; the
+// products T1 = L_m x for m in [t1m, t1m + nt1) are formed first).
+#define HEFF_MAX_SEGS 64
+struct HSeg {
+  int side, m, p;  // p: physical index of the source
+  int g;           // side 2: row block of T1
+  cplx coef;
+};
+struct HPlan {
+  int il, ir;  // channels that have to be the identity
+  int t1m, nt1, nseg, has_loc;
+  int off[5];     // segments of p' are off[p'] .. off[p' + 1] - 1
+  cplx loc[16];   // [p' + D p]
+  const HSeg* seg;
+};
+
 // Sparse MPO matrix M[o, i] in CSR form (rows are outputs).
 struct WMat {
   int no, ni, nnz;
   int ident;  // identity map with a physical dimension of 1 (bond): T2 is T1
+  int idc;    // environment maps: output channel that is the identity next to isometric sites, -1 for none
+  const HPlan* plan;  // effective-Hamiltonian maps: the structured product, null when it does not pay
   const int* rowp;  // no+1
   const int* col;   // nnz
   const cplx* val;  // nnz
@@ -119,6 +143,8 @@ static __device__ __noinline__ void dev_wapply(const T* in, T* out, const WMat W
 }
 
 struct HeffOp {
+  int blocked = 0;  // the run may reorder sums
+  const HPlan* plan = nullptr;  // set when both identity channels were found in the environments
   const cplx* L;  // (chil, wl, chil)
   const cplx* R;  // (chir, wr, chir)
   WMat W;         // rows p'+D m', cols m + wl p
@@ -169,6 +195,7 @@ struct EngineSmem {
   RedScratch r;
   KrySmem k;
   TcState tc;
+  HSeg hseg[HEFF_MAX_SEGS];  // segments of the solve's plan
   EngineSmemU u;
 };
 #if YAQS_TC
@@ -232,6 +259,66 @@ static __device__ void dev_heff_tc(const HeffOp& h, const cplx* x, cplx* y, Engi
 }
 #endif
 
+// One output block of the structured product as a segmented GEMM.
+struct HeffProv {
+  const HeffOp& h;
+  const HSeg* seg;
+  const cplx* x;
+  int nseg;
+  __device__ __forceinline__ int K(int s) const { return seg[s].side == 0 ? h.chil : h.chir; }
+  __device__ __forceinline__ bool unit(int s) const { return seg[s].coef.x == 1.0 && seg[s].coef.y == 0.0; }
+  __device__ __forceinline__ cplx coef(int s) const { return seg[s].coef; }
+  __device__ __forceinline__ void get(int s, GemmSeg& o) const {
+    const HSeg& q = seg[s];
+    o.am = 1;
+    if (q.side == 0) {
+      o.A = h.L + h.chil * q.m;
+      o.ak = h.chil * h.wl;
+      o.B = x + h.chil * q.p;
+      o.bk = 1;
+      o.bn = h.chil * h.D;
+      o.K = h.chil;
+    } else {
+      const int ld = q.side == 1 ? h.chil : h.chil * h.plan->nt1;
+      o.A = q.side == 1 ? x + h.chil * q.p : h.T1 + h.chil * q.g + ld * q.p;
+      o.ak = ld * h.D;
+      o.B = h.R + h.chir * q.m;
+      o.bk = h.chir * h.wr;
+      o.bn = 1;
+      o.K = h.chir;
+    }
+  }
+};
+
+// y = H_eff x by the plan of h (its segments in sm.hseg).  A Heisenberg site
+// multiplies 8 blocks of chi^3 instead of 10 and neither stores nor maps the
+// (w chi) x (D chi) intermediates: the K slices of all segments run through
+// one ring into one accumulator tile.
+static __device__ __noinline__ void heff_block(const HeffOp& h, const cplx* x, int pp, cplx* y, EngineSmem& sm) {
+  ProfScope prof_scope_(PF_GEMM);
+  const HPlan& pl = *h.plan;
+  const HeffProv pv{h, sm.hseg + pl.off[pp], x, pl.off[pp + 1] - pl.off[pp]};
+  const int ld = h.chil * h.D;
+  const bool loc = pl.has_loc != 0;
+  gemm_core(pv, h.chil, h.chir, false, false,
+            [&](int mm, int nn, cplx v) {
+              const int e = mm + nn * ld;
+              if (loc)
+                for (int p = 0; p < h.D; ++p) cfma(v, pl.loc[pp + h.D * p], x[e + h.chil * p]);
+              y[e + h.chil * pp] = v;
+            },
+            sm.u.gw.g);
+}
+
+static __device__ __forceinline__ void heff_structured(const HeffOp& h, const cplx* x, cplx* y, EngineSmem& sm) {
+  const HPlan& pl = *h.plan;
+  if (pl.nt1 > 0)
+    cta_gemm(gemm_args(h.chil * pl.nt1, h.D * h.chir, h.chil, h.L + h.chil * pl.t1m, 1, h.chil * h.wl, x, 1, h.chil,
+                       h.T1, 1, h.chil * pl.nt1),
+             sm.u.gw.g);
+  for (int pp = 0; pp < h.D; ++pp) heff_block(h, x, pp, y, sm);
+}
+
 // y = H_eff x.  CTA-collective.  In the mixed form x is rounded to FP32, the
 // three contractions run in FP32 (tensor cores for the two GEMMs) and y is
 // written back in FP64.
@@ -243,6 +330,10 @@ static __device__ __noinline__ void dev_heff(const HeffOp& h, const cplx* x, cpl
     return;
   }
 #endif
+  if (h.plan && !h.mixed) {
+    heff_structured(h, x, y, sm);
+    return;
+  }
   if (h.mixed) {
     GemmSmemF& gf = reinterpret_cast<GemmSmemF&>(sm.u.gw.g);
     cta_to_f32(h.xf, x, (long long)chil * D * chir);
@@ -298,6 +389,15 @@ static __device__ __noinline__ void dev_heff(const HeffOp& h, const cplx* x, cpl
 static __device__ __forceinline__ double heff_flops(int chil, int wl, int D, int chir, int wr) {
   return 8.0 * ((double)chil * chil * wl * D * chir + (double)chil * chir * D * D * wl * wr +
                 (double)chil * D * chir * chir * wr);
+}
+
+// Floating-point operations of one product in the form it takes.
+static __device__ __forceinline__ double heff_work(const HeffOp& h) {
+  if (!h.plan || h.mixed) return heff_flops(h.chil, h.wl, h.D, h.chir, h.wr);
+  const double l = h.chil, r = h.chir;
+  double f = l * l * h.plan->nt1 * h.D * r;
+  for (int s = 0; s < h.plan->nseg; ++s) f += h.plan->seg[s].side == 0 ? l * l * r : l * r * r;
+  return 8.0 * f;
 }
 
 struct KrylovCfg {
@@ -700,12 +800,174 @@ static __device__ __noinline__ int dev_expm_small(const HeffOp& h, const SmallPl
   return mv;
 }
 
+// ---------------------------------------------------------------------------
+// Lanczos steps of the runs that may reorder sums
+// ---------------------------------------------------------------------------
+// With w = H q_{k-1}, the projections of w' = w - sigma q_{k-1} - beta q_{k-2}
+// on q_{k-1}, q_{k-2}, ..., q_0 into ks.h (ks.h[j] belongs to q_j) and |w'|^2.
+// sigma and beta are what the recurrence predicts (the first diagonal entry
+// and the last off-diagonal one), so what is left is small beside the residual
+// and one pass leaves it orthogonal: without them the large diagonal entry
+// sent half of the steps through a second projection, two more passes over the
+// basis.  The passes are bound by memory latency and by L2: 7 vectors and two
+// values a thread keep 16 loads in flight.  CTA-collective.
+static __device__ __noinline__ double predicted_dots(const cplx* Q, long long qs, const cplx* w, int n, int k,
+                                                     double sigma, double beta, EngineSmem& sm) {
+  const int tid = ltid(), lane = tid & 31, wid = tid >> 5;
+  const cplx* q0 = Q + qs * (k - 1);
+  const cplx* q1 = k > 1 ? q0 - qs : q0;
+  if (k == 1) beta = 0.0;
+  double nw2 = 0.0;
+  for (int j0 = 0; j0 < k; j0 += 7) {  // vectors q_{k-1-j0}, q_{k-2-j0}, ...
+    double d[16];
+#pragma unroll
+    for (int e = 0; e < 16; ++e) d[e] = 0.0;
+#pragma unroll 1
+    for (int i0 = tid; i0 < n; i0 += 2 * NT) {
+      const int i1 = i0 + NT < n ? i0 + NT : i0;
+      const double on = i0 + NT < n ? 1.0 : 0.0;
+      cplx a0[7], a1[7];
+#pragma unroll
+      for (int e = 0; e < 7; ++e) {
+        const bool live = j0 + e < k;
+        const cplx* q = q0 - qs * (j0 + e);
+        a0[e] = live ? q[i0] : make_double2(0.0, 0.0);
+        a1[e] = live ? q[i1] : make_double2(0.0, 0.0);
+      }
+      cplx w0 = w[i0], w1 = w[i1];
+      const cplx s0 = j0 == 0 ? a0[0] : q0[i0], s1 = j0 == 0 ? a1[0] : q0[i1];
+      const cplx t0 = j0 == 0 && k > 1 ? a0[1] : q1[i0], t1 = j0 == 0 && k > 1 ? a1[1] : q1[i1];
+      w0.x = fma(-beta, t0.x, fma(-sigma, s0.x, w0.x));
+      w0.y = fma(-beta, t0.y, fma(-sigma, s0.y, w0.y));
+      w1.x = on * fma(-beta, t1.x, fma(-sigma, s1.x, w1.x));
+      w1.y = on * fma(-beta, t1.y, fma(-sigma, s1.y, w1.y));
+      d[14] += cabs2(w0) + cabs2(w1);
+#pragma unroll
+      for (int e = 0; e < 7; ++e) {
+        cplx p = make_double2(d[2 * e], d[2 * e + 1]);
+        cfmac(p, a0[e], w0);
+        cfmac(p, a1[e], w1);
+        d[2 * e] = p.x;
+        d[2 * e + 1] = p.y;
+      }
+    }
+    warp_sum_multi<16>(d);
+    if ((lane & 1) == 0) sm.r.v[wid * 16 + (lane >> 1)] = d[0];
+    cta_sync();
+    if (tid < 16) {
+      double v = 0.0;
+      for (int u = 0; u < NW; ++u) v += sm.r.v[u * 16 + tid];
+      sm.r.v[NW * 16 + tid] = v;
+      const int j = k - 1 - j0 - (tid >> 1);
+      if (tid < 14 && j >= 0) reinterpret_cast<double*>(sm.k.h + j)[tid & 1] = v;
+    }
+    cta_sync();
+    if (j0 == 0) nw2 = sm.r.v[NW * 16 + 14];
+  }
+  cta_sync();
+  return nw2;
+}
+
+// out = s (w - sum_{j<k} h_j q_j) with h in ks.h; w null: no w.  One pass,
+// eight vectors and two values a thread at a time.  CTA-collective.
+static __device__ __noinline__ void combine_pass(const cplx* Q, long long qs, const cplx* w, cplx* out, int n, int k,
+                                                 double s, EngineSmem& sm) {
+  const cplx* h = sm.k.h;
+#pragma unroll 1
+  for (int i0 = ltid(); i0 < n; i0 += 2 * NT) {
+    const int i1 = i0 + NT < n ? i0 + NT : i0;
+    cplx v0 = w ? w[i0] : make_double2(0.0, 0.0), v1 = w ? w[i1] : make_double2(0.0, 0.0);
+#pragma unroll 1
+    for (int j0 = 0; j0 < k; j0 += 8) {
+      cplx a0[8], a1[8];
+#pragma unroll
+      for (int e = 0; e < 8; ++e) {
+        const bool live = j0 + e < k;
+        const cplx* q = Q + qs * (j0 + e);
+        a0[e] = live ? q[i0] : make_double2(0.0, 0.0);
+        a1[e] = live ? q[i1] : make_double2(0.0, 0.0);
+      }
+#pragma unroll
+      for (int e = 0; e < 8; ++e) {
+        const cplx c = h[min(j0 + e, KRYLOV_MAX)], nc = make_double2(-c.x, -c.y);
+        cfma(v0, nc, a0[e]);
+        cfma(v1, nc, a1[e]);
+      }
+    }
+    out[i0] = cscale(v0, s);
+    if (i1 != i0) out[i1] = cscale(v1, s);
+  }
+  cta_sync();
+}
+
+// dev_expm_krylov with predicted projections.
+static __device__ __noinline__ int dev_expm_predicted(const HeffOp& h, cplx* x, double dt, const KrylovCfg& kc, cplx* Q,
+                                                      long long qs, EngineSmem& sm) {
+  const int tid = ltid();
+  const int n = h.chil * h.D * h.chir;
+  const double beta0 = sqrt(cta_norm2(x, n, sm.r));
+  if (beta0 == 0.0) return 0;
+  const double tau = fabs(dt);
+  for (int i = tid; i < n; i += NT) Q[i] = cscale(x[i], 1.0 / beta0);
+  if (tid <= KRYLOV_MAX) sm.k.h[tid] = make_double2(0.0, 0.0);  // combine_pass reads whole groups
+  cta_sync();
+  double bound = 1.0, sigma = 0.0, beta = 0.0;
+  int m = 0, mv = 0;
+  for (int k = 1; k <= kc.kdim; ++k) {
+    cplx* w = Q + qs * k;
+    dev_heff(h, Q + qs * (k - 1), w, sm);
+    ++mv;
+    ProfScope orth_scope_(PF_ORTH);
+    const double nw2 = predicted_dots(Q, qs, w, n, k, sigma, beta, sm);
+    double hh = 0.0;
+    for (int j = 0; j < k; ++j) hh += cabs2(sm.k.h[j]);
+    double a_k = sm.k.h[k - 1].x + sigma;
+    const double r2 = nw2 - hh;
+    const bool accept = r2 >= 0.5 * nw2;  // DGKS, on what the prediction left
+    cta_sync();
+    if (tid == 0) {
+      sm.k.h[k - 1].x += sigma;
+      if (k > 1) sm.k.h[k - 2].x += beta;
+    }
+    cta_sync();
+    double b_k;
+    if (accept) {
+      b_k = sqrt(r2);
+    } else {
+      combine_pass(Q, qs, w, w, n, k, 1.0, sm);
+      const double n2 = predicted_dots(Q, qs, w, n, k, 0.0, 0.0, sm);
+      a_k += sm.k.h[k - 1].x;
+      hh = 0.0;
+      for (int j = 0; j < k; ++j) hh += cabs2(sm.k.h[j]);
+      b_k = sqrt(fmax(n2 - hh, 0.0));  // hh is rounding: the first projection took the rest
+    }
+    if (tid == 0) sm.k.alpha[k - 1] = a_k;
+    m = k;
+    if (b_k <= tau * kc.tol) break;
+    if (k == kc.kdim) break;
+    bound *= b_k * tau / k;
+    if (kc.exit_tol > 0.0 && bound <= kc.exit_tol) break;
+    if (tid == 0) sm.k.beta[k - 1] = b_k;
+    combine_pass(Q, qs, w, w, n, k, 1.0 / b_k, sm);
+    if (k == 1) sigma = a_k;
+    beta = b_k;
+  }
+  cta_sync();
+  dev_tridiag_expm(m, dt, sm.k);
+  cta_sync();
+  if (tid < m) sm.k.h[tid] = make_double2(-sm.k.y[tid].x, -sm.k.y[tid].y);  // x = beta0 sum_j y_j q_j
+  cta_sync();
+  combine_pass(Q, qs, nullptr, x, n, m, beta0, sm);
+  return mv;
+}
+
 // In place: x <- exp(-i dt H_eff) x.  Q holds kdim+1 vectors of stride qs.
 // Returns the number of H_eff products.  CTA-collective.
 static __device__ __noinline__ int dev_expm_krylov(const HeffOp& h, cplx* x, double dt, const KrylovCfg& kc, cplx* Q,
                                             long long qs, EngineSmem& sm) {
   SmallPlan sp;
   if (small_plan(h, sp)) return dev_expm_small(h, sp, x, dt, kc, Q, qs, sm);
+  if (h.blocked) return dev_expm_predicted(h, x, dt, kc, Q, qs, sm);
   const int tid = ltid();
   const long long n = (long long)h.chil * h.D * h.chir;
   const double beta0 = sqrt(cta_norm2(x, n, sm.r));

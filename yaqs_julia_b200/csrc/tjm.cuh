@@ -117,6 +117,8 @@ struct CtaSmem {
   double bcast_d[8];
   int fail;
   int canon;  // the state is in mixed canonical form around its centre
+  // 1 + the MPO channel in which an environment was found to be the identity, 0 for none
+  unsigned char id_left[MAX_L + 1], id_right[MAX_L + 1];
 };
 
 // Dynamic shared memory of one trajectory program, with 1024 bytes of slack
@@ -348,6 +350,32 @@ static __device__ void identity_env(Ctx& c, cplx* E, int dim, int w) {
   cta_sync();
 }
 
+// Next to isometric sites one channel of an environment is the identity up to
+// the rounding of the factorisations (the operator has not started yet, or has
+// ended).  Where channel idc of E (dim, w, dim) is that, to within the
+// rounding of the contraction that formed it, it is written as the exact
+// identity and noted for make_heff; a state that is not in canonical form
+// fails the test and takes the general product.  CTA-collective.
+static __device__ __noinline__ void note_identity(Ctx& c, cplx* E, int dim, int w, int idc, unsigned char* note) {
+  bool found = false;
+  if (c.P.blocked && idc >= 0) {
+    double dev = 0.0;
+    for (int k = ltid() >> 5; k < dim; k += NW)
+      for (int a = ltid() & 31; a < dim; a += 32) {
+        const cplx v = E[a + dim * (idc + w * k)];
+        const double d = fmax(fabs(v.x - (a == k ? 1.0 : 0.0)), fabs(v.y));
+        dev = d > dev || d != d ? (d != d ? INFINITY : d) : dev;
+      }
+    found = block_max(dev, c.sm.e.r) <= (c.P.mixed ? 2e-5 : 1e-12);
+    if (found)
+      for (int k = ltid() >> 5; k < dim; k += NW)
+        for (int a = ltid() & 31; a < dim; a += 32)
+          E[a + dim * (idc + w * k)] = make_double2(a == k ? 1.0 : 0.0, 0.0);
+  }
+  if (ltid() == 0) *note = found ? idc + 1 : 0;
+  cta_sync();
+}
+
 // EL[i+1] from EL[i], A_i and the map Wenv of W_i (update_left_environment)
 static __device__ __noinline__ void update_left_w(Ctx& c, const DState& s, int i, const WMat& Wenv) {
   ProfScope prof_scope_(PF_ENV);
@@ -391,6 +419,7 @@ static __device__ __noinline__ void update_left_w(Ctx& c, const DState& s, int i
     cta_gemm(gemm_args(r, wr * r, 2 * l, A, 2 * l, 1, T2, 1, 2 * l, envL(c, i + 1), 1, r, true, false),
              c.sm.e.u.gw.g);
   }
+  note_identity(c, envL(c, i + 1), r, wr, Wenv.idc, c.sm.id_left + i + 1);
 }
 
 static __device__ void update_left(Ctx& c, const DState& s, int i) { update_left_w(c, s, i, c.P.wm_envL[i]); }
@@ -435,6 +464,7 @@ static __device__ __noinline__ void update_right_w(Ctx& c, const DState& s, int 
     dev_wapply<cplx>(T1, T2, Wenv, g, c.sm.e.u.gw.w);
     cta_gemm(gemm_args(l, wl * l, 2 * r, A, 1, l, T2, 1, 2 * r, envR(c, i), 1, l, true, false), c.sm.e.u.gw.g);
   }
+  note_identity(c, envR(c, i), l, wl, Wenv.idc, c.sm.id_right + i);
 }
 
 static __device__ void update_right(Ctx& c, const DState& s, int i) { update_right_w(c, s, i, c.P.wm_envR[i]); }
@@ -472,6 +502,12 @@ static __device__ HeffOp make_heff(Ctx& c, int l, int D, int r, int bl, int br, 
   h.T1 = c.ws + c.P.lay.T1;
   h.T2 = c.ws + c.P.lay.T2;
   h.mixed = c.P.mixed;
+  h.blocked = c.P.blocked;
+  if (W.plan && c.sm.id_left[bl] == W.plan->il + 1 && c.sm.id_right[br] == W.plan->ir + 1) {
+    h.plan = W.plan;
+    for (int e = ltid(); e < W.plan->nseg; e += NT) c.sm.e.hseg[e] = W.plan->seg[e];
+    cta_sync();
+  }
   const bool tc = c.P.tc && !(c.P.tune && c.P.tune[tune_index(l, D, r)] == 1);
   if (tc) {  // environments staged once per Krylov solve as the TMA operands
     const WsLayout& y = c.P.lay;
@@ -515,7 +551,7 @@ static __device__ __noinline__ void evolve(Ctx& c, cplx* x, int l, int D, int r,
   if (ltid() == 0) {
     c.cnt[0] += mv;
     c.cnt[1] += (mv > 0);
-    *c.fl += mv * heff_flops(l, h.wl, D, r, h.wr);
+    *c.fl += mv * heff_work(h);
   }
 }
 
@@ -609,8 +645,10 @@ static __device__ __noinline__ void init_envs(Ctx& c, const DState& s) {
   const int L = c.P.L;
   shift_oc(c, s, 0);
   identity_env(c, envR(c, L), s.chi[L], c.P.w[L]);
-  for (int i = L - 1; i >= 1; --i) update_right(c, s, i);
   identity_env(c, envL(c, 0), s.chi[0], c.P.w[0]);
+  if (ltid() == 0) c.sm.id_right[L] = c.sm.id_left[0] = c.P.blocked ? 1 : 0;  // channel 0 of width 1
+  cta_sync();
+  for (int i = L - 1; i >= 1; --i) update_right(c, s, i);
 }
 
 // exp(-i dtb H_bond) C on bond b (project_bond, Algorithms.jl:222-226), C (k x r).
