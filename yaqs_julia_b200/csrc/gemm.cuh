@@ -8,9 +8,12 @@
 // written as one such GEMM over the reference's column-major layouts.
 //
 // Tiling: 64 x GBN_EFF output tiles (64 x 64 for a 256-thread program, 64 x
-// 32 for a 128-thread one), 8-deep K slices staged in shared memory by
-// cp.async through a four-stage ring (one barrier per slice, zero-filled
-// outside the matrix).  The 8 x 8 blocks of a tile are dealt to the warps in
+// 32 for a 128-thread one), K slices staged in shared memory by cp.async
+// through a ring (one barrier per slice, zero-filled outside the matrix): two
+// stages of 16 for long sums, where the work of a slice has to outweigh its
+// barrier (L = 30, chi 64, FP64: 1158 ms against 1246 with 8-deep slices),
+// four of 8 for sums shorter than 32, which 16-deep ones would pad (digital
+// L = 40: 766 against 799 ms).  The 8 x 8 blocks of a tile are dealt to the warps in
 // rows and columns (warp (wm, wn) owns block rows wm + 2 i and block columns
 // wn + NW/2 j), so a tile that is only partly inside the matrix still spreads
 // over all warps; blocks outside it issue no MMA and stage no data.
@@ -24,8 +27,7 @@
 
 #define GBM 64
 #define GBN 64
-#define GBK 8
-#define GSTAGES 4
+#define GROWS 32  // k rows in the ring: stages x slice depth
 // Output columns of one CTA tile: the warps form a 2 x NW/2 grid.
 #define GBN_EFF (16 * (NW / 2))
 static_assert(NW % 2 == 0 && GBN_EFF <= GBN, "the GEMM needs an even warp count of at most 8");
@@ -34,8 +36,8 @@ static_assert(NW % 2 == 0 && GBN_EFF <= GBN, "the GEMM needs an even warp count 
 // at two columns each, and 66 (34) x 16 bytes puts those in eight different
 // 16-byte bank groups (65 gave two-way conflicts).
 struct GemmSmem {
-  cplx As[GSTAGES][GBK][GBM + 2];
-  cplx Bs[GSTAGES][GBK][GBN_EFF + 2];
+  cplx As[GROWS][GBM + 2];
+  cplx Bs[GROWS][GBN_EFF + 2];
 };
 
 static __device__ __forceinline__ void cp_async16(void* smem, const void* gmem, bool valid) {
@@ -46,8 +48,9 @@ static __device__ __forceinline__ void cp_async16(void* smem, const void* gmem, 
 static __device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;\n" ::: "memory"); }
 static __device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wait_group 0;\n" ::: "memory"); }
 static __device__ __forceinline__ void cp_async_wait_one() { asm volatile("cp.async.wait_group 1;\n" ::: "memory"); }
-static __device__ __forceinline__ void cp_async_wait_ring() {
-  asm volatile("cp.async.wait_group %0;\n" ::"n"(GSTAGES - 2) : "memory");
+template <int N>
+static __device__ __forceinline__ void cp_async_wait() {
+  asm volatile("cp.async.wait_group %0;\n" ::"n"(N) : "memory");
 }
 
 struct GemmArgs {
@@ -119,9 +122,10 @@ static __device__ __forceinline__ double flip_sign(double x, unsigned mask) {
 // chi 64, FP64 (260 trajectories, 2 time indices) went from 1588 to 1453 ms,
 // L = 16 at chi 128 from 600 to 550 ms and L = 6 at chi 16 from 528 to 446 ms,
 // with the same bits.
-template <class Prov, class Epi>
+template <int GBK, class Prov, class Epi>
 static __device__ __forceinline__ void gemm_core(const Prov& pv, int M, int N, bool conjA, bool conjB, Epi epi,
                                                  GemmSmem& sm) {
+  constexpr int GSTAGES = GROWS / GBK;
   const int tid = ltid();
   const int lane = tid & 31, wid = tid >> 5;
   const int wm = wid & 1, wn = wid >> 1;  // 2 x NW/2 warps
@@ -156,7 +160,7 @@ static __device__ __forceinline__ void gemm_core(const Prov& pv, int M, int N, b
             const int ka = ik + ki;
             const bool va = mi < mrem && ka < o.K;
             if (mi < mlim)
-              cp_async16(&sm.As[buf][ki][mi], o.A + (va ? (tm + mi) * o.am + ka * o.ak : 0), va);
+              cp_async16(&sm.As[buf * GBK + ki][mi], o.A + (va ? (tm + mi) * o.am + ka * o.ak : 0), va);
           }
 #pragma unroll
           for (int e = 0; e < GBN_EFF * GBK / NT; ++e) {
@@ -166,7 +170,7 @@ static __device__ __forceinline__ void gemm_core(const Prov& pv, int M, int N, b
             const int kb = ik + kj;
             const bool vb = ni < nrem && kb < o.K;
             if (ni < nlim)
-              cp_async16(&sm.Bs[buf][kj][ni], o.B + (vb ? kb * o.bk + (tn + ni) * o.bn : 0), vb);
+              cp_async16(&sm.Bs[buf * GBK + kj][ni], o.B + (vb ? kb * o.bk + (tn + ni) * o.bn : 0), vb);
           }
           ik += GBK;
           if (ik >= o.K) {
@@ -177,11 +181,11 @@ static __device__ __forceinline__ void gemm_core(const Prov& pv, int M, int N, b
         cp_async_commit();
       };
       cta_sync();  // the ring's last readers (the tile before) are done
-#pragma unroll
+#pragma unroll 1
       for (int p = 0; p < GSTAGES - 1; ++p) issue(p);
       int cs = 0, ck = 0, cK = pv.K(0);
       for (int t = 0; t < nslice; ++t) {
-        cp_async_wait_ring();  // slice t has landed (this thread's part)
+        cp_async_wait<GSTAGES - 2>();  // slice t has landed (this thread's part)
         cta_sync();            // everybody's part; slice t - 1 is consumed
         issue((t + GSTAGES - 1) % GSTAGES);
         const int buf = t % GSTAGES;
@@ -194,7 +198,7 @@ static __device__ __forceinline__ void gemm_core(const Prov& pv, int M, int N, b
           for (int j = 0; j < 2; ++j) {
             const int n0 = (wn + (NW / 2) * j) * 8;
             if (n0 < nrem) {
-              const cplx b = sm.Bs[buf][k4 + tq][n0 + gq];
+              const cplx b = sm.Bs[buf * GBK + k4 + tq][n0 + gq];
               br[j] = b.x;
               bi[j] = flip_sign(b.y, sgB);
               if (!unit) {
@@ -209,16 +213,27 @@ static __device__ __forceinline__ void gemm_core(const Prov& pv, int M, int N, b
           for (int i = 0; i < 4; ++i) {
             const int m0 = (wm + 2 * i) * 8;
             if (m0 >= mrem) break;
-            const cplx a = sm.As[buf][k4 + tq][m0 + gq];
+            const cplx a = sm.As[buf * GBK + k4 + tq][m0 + gq];
             ar[i] = a.x;
             ai[i] = flip_sign(a.y, sgA);
-#pragma unroll
-            for (int j = 0; j < 2; ++j) {
-              if ((wn + (NW / 2) * j) * 8 >= nrem) break;
-              dmma884(cr[i][j][0], cr[i][j][1], ar[i], br[j]);
-              dmma884(ci[i][j][0], ci[i][j][1], ar[i], bi[j]);
-              dmma884(cr[i][j][0], cr[i][j][1], -ai[i], bi[j]);
-              dmma884(ci[i][j][0], ci[i][j][1], ai[i], br[j]);
+            // first products of both blocks before the second ones, which wait
+            // for the same accumulators
+            const bool one = wn * 8 < nrem, two = (wn + NW / 2) * 8 < nrem;
+            if (one) {
+              dmma884(cr[i][0][0], cr[i][0][1], ar[i], br[0]);
+              dmma884(ci[i][0][0], ci[i][0][1], ar[i], bi[0]);
+            }
+            if (two) {
+              dmma884(cr[i][1][0], cr[i][1][1], ar[i], br[1]);
+              dmma884(ci[i][1][0], ci[i][1][1], ar[i], bi[1]);
+            }
+            if (one) {
+              dmma884(cr[i][0][0], cr[i][0][1], -ai[i], bi[0]);
+              dmma884(ci[i][0][0], ci[i][0][1], ai[i], br[0]);
+            }
+            if (two) {
+              dmma884(cr[i][1][0], cr[i][1][1], -ai[i], bi[1]);
+              dmma884(ci[i][1][0], ci[i][1][1], ai[i], br[1]);
             }
           }
         }
@@ -263,14 +278,77 @@ struct OneSeg {
   }
 };
 
-static __device__ __noinline__ void cta_gemm(const GemmArgs g, GemmSmem& sm) {
+template <int GBK>
+static __device__ __noinline__ void cta_gemm_k(const GemmArgs g, GemmSmem& sm) {
   ProfScope prof_scope_(PF_GEMM);
   const OneSeg pv{g, 1};
-  gemm_core(pv, g.M, g.N, g.conjA, g.conjB,
-            [&](int mm, int nn, cplx v) {
-              cplx* c = g.C + (mm * (int)g.cm + nn * (int)g.cn);
-              if (g.accumulate) v = cadd(v, *c);
-              *c = v;
-            },
-            sm);
+  gemm_core<GBK>(pv, g.M, g.N, g.conjA, g.conjB,
+                 [&](int mm, int nn, cplx v) {
+                   cplx* c = g.C + (mm * (int)g.cm + nn * (int)g.cn);
+                   if (g.accumulate) v = cadd(v, *c);
+                   *c = v;
+                 },
+                 sm);
+}
+
+// A product of a few 8 x 8 blocks and a short sum, straight from global memory:
+// two blocks a warp at most, no staging and one barrier.  The tiled form's
+// slices, copies and barriers cost more than such a product.  Same bits.
+#define GDIRECT_K 32
+static __device__ __noinline__ void cta_gemm_direct(const GemmArgs g) {
+  ProfScope prof_scope_(PF_GEMM);
+  const int lane = ltid() & 31, wid = ltid() >> 5;
+  const int gq = lane >> 2, tq = lane & 3;
+  const unsigned sgA = g.conjA ? 0x80000000u : 0u, sgB = g.conjB ? 0x80000000u : 0u;
+  const int mb = (g.M + 7) >> 3, nb = (g.N + 7) >> 3;
+#pragma unroll 1
+  for (int q = wid; q < mb * nb; q += NW) {
+    const int nq = q / mb, row = (q - nq * mb) * 8 + gq, n0 = nq * 8;
+    const bool rm = row < g.M, rn = n0 + gq < g.N;
+    const cplx* A = g.A + (long long)(rm ? row : 0) * g.am;
+    const cplx* B = g.B + (long long)(rn ? n0 + gq : 0) * g.bn;
+    double cr[2] = {0.0, 0.0}, ci[2] = {0.0, 0.0};
+#pragma unroll 1
+    for (int k0 = 0; k0 < g.K; k0 += 16) {
+      cplx a[4], b[4];
+#pragma unroll
+      for (int u = 0; u < 4; ++u) {
+        const int k = k0 + 4 * u + tq;
+        const bool in = k < g.K;
+        a[u] = in && rm ? A[k * g.ak] : make_double2(0.0, 0.0);
+        b[u] = in && rn ? B[k * g.bk] : make_double2(0.0, 0.0);
+      }
+#pragma unroll
+      for (int u = 0; u < 4; ++u) {
+        if (k0 + 4 * u >= g.K) break;
+        const double ai = flip_sign(a[u].y, sgA), bi = flip_sign(b[u].y, sgB);
+        dmma884(cr[0], cr[1], a[u].x, b[u].x);
+        dmma884(ci[0], ci[1], a[u].x, bi);
+        dmma884(cr[0], cr[1], -ai, bi);
+        dmma884(ci[0], ci[1], ai, b[u].x);
+      }
+    }
+    if (rm) {
+#pragma unroll
+      for (int e = 0; e < 2; ++e) {
+        const int n = n0 + 2 * tq + e;
+        if (n < g.N) {
+          cplx* c = g.C + (long long)row * g.cm + (long long)n * g.cn;
+          cplx v = make_double2(cr[e], ci[e]);
+          if (g.accumulate) v = cadd(v, *c);
+          *c = v;
+        }
+      }
+    }
+  }
+  cta_sync();
+}
+
+static __device__ __forceinline__ void cta_gemm(const GemmArgs g, GemmSmem& sm) {
+  if (g.K <= GDIRECT_K && ((g.M + 7) >> 3) * ((g.N + 7) >> 3) <= 2 * NW)
+    cta_gemm_direct(g);
+  else if (g.K >= 32)
+    cta_gemm_k<16>(g, sm);
+  else
+    cta_gemm_k<8>(g, sm);
 }

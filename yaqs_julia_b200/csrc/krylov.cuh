@@ -300,7 +300,7 @@ static __device__ __noinline__ void heff_block(const HeffOp& h, const cplx* x, i
   const HeffProv pv{h, sm.hseg + pl.off[pp], x, pl.off[pp + 1] - pl.off[pp]};
   const int ld = h.chil * h.D;
   const bool loc = pl.has_loc != 0;
-  gemm_core(pv, h.chil, h.chir, false, false,
+  gemm_core<16>(pv, h.chil, h.chir, false, false,
             [&](int mm, int nn, cplx v) {
               const int e = mm + nn * ld;
               if (loc)
