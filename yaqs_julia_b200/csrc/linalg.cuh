@@ -403,6 +403,30 @@ static __device__ __noinline__ void qr_panel(cplx* V, int m, int ja, int jb, int
   cta_sync();
 }
 
+static __device__ __forceinline__ void qr_panel_rows(cplx* V, int m, int ja, int jb, int pe, double null_abs, cplx* tau) {
+  if (m <= 32)
+    qr_panel<1>(V, m, ja, jb, pe, null_abs, tau);
+  else if (m <= 64)
+    qr_panel<2>(V, m, ja, jb, pe, null_abs, tau);
+  else if (m <= 128)
+    qr_panel<4>(V, m, ja, jb, pe, null_abs, tau);
+  else
+    qr_panel<8>(V, m, ja, jb, pe, null_abs, tau);
+}
+
+// m x n values by load(e) into V; returns the null threshold of their factorisation.
+template <class Load>
+static __device__ __forceinline__ double qr_load_panel(int m, int n, Load load, cplx* V, RedScratch& rs) {
+  cta_sync();  // the buffer's last readers are done
+  double s = 0.0;
+  for (int e = ltid(); e < m * n; e += NT) {
+    const cplx v = load(e);
+    V[e] = v;
+    s += cabs2(v);
+  }
+  return QR_NULL_TOL * sqrt(block_sum(s, rs));
+}
+
 static __device__ __forceinline__ void qr_apply_rows(cplx* X, int ld, int c0, int c1, const cplx* V, int m, int ja,
                                                      int jb, bool ascending, int ident, const cplx* tau) {
   if (m <= 32)
@@ -426,14 +450,7 @@ static __device__ __noinline__ void dev_qr_factor_panel(cplx* H, int m, int n, c
     cplx* P = H + m * ja;
     for (int e = ltid(); e < m * (pe - ja); e += NT) sb[e] = P[e];
     cta_sync();
-    if (m <= 32)
-      qr_panel<1>(sb, m, ja, jb, pe, null_abs, ls.tau);
-    else if (m <= 64)
-      qr_panel<2>(sb, m, ja, jb, pe, null_abs, ls.tau);
-    else if (m <= 128)
-      qr_panel<4>(sb, m, ja, jb, pe, null_abs, ls.tau);
-    else
-      qr_panel<8>(sb, m, ja, jb, pe, null_abs, ls.tau);
+    qr_panel_rows(sb, m, ja, jb, pe, null_abs, ls.tau);
     for (int e = ltid(); e < m * (pe - ja); e += NT) P[e] = sb[e];
     qr_apply_rows(H, m, pe, n, sb, m, ja, jb, true, 0, ls.tau);
     cta_sync();
@@ -454,6 +471,27 @@ static __device__ __noinline__ void dev_qr_formq_panel(const cplx* H, int m, int
   }
 }
 
+template <class Load, class Store>
+static __device__ __forceinline__ void qr_one_panel(int m, int n, Load load, Store store_q, cplx* Rout, cplx* sb,
+                                                    LinalgSmem& ls, RedScratch& rs) {
+  const int k = min(m, n);
+  const double null_abs = qr_load_panel(m, n, load, sb, rs);
+  {
+    ProfScope prof_scope_(PF_QR);
+    qr_panel_rows(sb, m, 0, k, n, null_abs, ls.tau);
+  }
+  ProfScope prof_scope_(PF_QRQ);
+  cplx* q = sb + m * n;
+  qr_apply_rows(q, m, 0, k, sb, m, 0, k, false, k, ls.tau);
+  for (int e = ltid(); e < k * n; e += NT) {
+    const int c = e / k, r = e - c * k;
+    Rout[e] = (r <= c) ? sb[r + m * c] : make_double2(0.0, 0.0);
+  }
+  cta_sync();
+  for (int e = ltid(); e < m * k; e += NT) store_q(e, q);
+  cta_sync();
+}
+
 // Thin QR of M (m x n, col-major), load(e) its element e: store_q(e, q), e < m k,
 // stores from Q (m x k) at q, Rout becomes R (k x n), k = min(m, n).  H and Qg
 // are work matrices in global memory; a problem that fits runs in the shared buffer sb
@@ -464,6 +502,11 @@ template <class Load, class Store>
 static __device__ __forceinline__ void dev_qr_thin(int m, int n, Load load, cplx* H, Store store_q, cplx* Qg, cplx* Rout,
                                                    cplx* sb, int cap, LinalgSmem& ls, RedScratch& rs) {
   const int k = min(m, n);
+  if (ls.blocked && n <= QR_PANEL && m <= QR_PANEL_MAX_ROWS && m * (n + k) <= cap) {
+    // one panel: never leaves shared memory, Q beside it
+    qr_one_panel(m, n, load, store_q, Rout, sb, ls, rs);
+    return;
+  }
   if (ls.blocked && m <= QR_PANEL_MAX_ROWS) {
     cta_sync();
     for (int e = ltid(); e < m * n; e += NT) H[e] = load(e);
@@ -757,23 +800,31 @@ static __device__ __noinline__ SvdResult dev_svd(const cplx* M, int m, int n, in
   // (at the end of the buffer, or in global memory) and B for all sweeps.
   const bool resident = q * p <= SVD_SMEM_CPLX;
   const bool panel = ls.blocked && mm <= QR_PANEL_MAX_ROWS;
-  const bool h_shared = !panel && mm * nn <= SVD_SMEM_CPLX;
+  const bool one_panel = panel && nn <= QR_PANEL && mm * nn + q * p <= SVD_SMEM_CPLX;
+  const bool h_shared = one_panel || (!panel && mm * nn <= SVD_SMEM_CPLX);
   const bool both = resident && (panel || mm * nn + q * p <= SVD_SMEM_CPLX);
   cplx* H = h_shared ? sb + (SVD_SMEM_CPLX - mm * nn) : w.X;
-  for (int e = tid; e < mm * nn; e += NT) {
-    int r = (int)(e % mm), c = (int)(e / mm);
-    H[e] = res.tr ? M[e] : cconj(M[c + (long long)m * r]);
+  auto load = [&](int e) {
+    const int c = e / mm, r = e - c * mm;
+    return res.tr ? M[e] : cconj(M[c + m * r]);
+  };
+  if (one_panel) {
+    const double null_abs = qr_load_panel(mm, nn, load, H, rs);
+    ProfScope qr_scope_(PF_QR);
+    qr_panel_rows(H, mm, 0, k, nn, null_abs, ls.tau);
+  } else {
+    for (int e = tid; e < mm * nn; e += NT) H[e] = load(e);
+    cta_sync();
+    if (panel)
+      dev_qr_factor_panel(H, mm, nn, sb, ls, rs);
+    else
+      dev_qr_factor(H, mm, nn, ls, rs);
   }
-  cta_sync();
-  if (panel)
-    dev_qr_factor_panel(H, mm, nn, sb, ls, rs);
-  else
-    dev_qr_factor(H, mm, nn, ls, rs);
   // B = R^H (nn x k): B[r, c] = conj(R[c, r]) for c <= r
   cplx* B0 = both ? sb : w.B;
   for (int e = tid; e < q * p; e += NT) {
-    int r = (int)(e % q), c = (int)(e / q);
-    B0[e] = (c <= r) ? cconj(H[c + (long long)mm * r]) : make_double2(0.0, 0.0);
+    const int c = e / q, r = e - c * q;
+    B0[e] = (c <= r) ? cconj(H[c + mm * r]) : make_double2(0.0, 0.0);
   }
   cta_sync();
   if (resident && !both) {
@@ -842,49 +893,43 @@ static __device__ __noinline__ SvdResult dev_svd(const cplx* M, int m, int n, in
     res.sweeps = sweep + 1;
     if (rc == 0) break;
   }
-  if (resident) {
-    cta_copy(w.B, sb, (long long)q * p);
-    cta_sync();
-  }
-  // singular values
+  // singular values; the factorisation's scalars are done with, their room
+  // holds the unsorted values and the order
+  const cplx* Bv = resident ? sb : w.B;
+  double* sig0 = reinterpret_cast<double*>(ls.tau);
+  int* ord = reinterpret_cast<int*>(sig0 + SVD_MAX_COLS);
+  if (resident) cta_copy(w.B, sb, (long long)q * p);
   const int lane = tid & 31, wid = tid >> 5;
   for (int c = wid; c < p; c += NW) {
-    const cplx* bc = w.B + (long long)q * c;
+    const cplx* bc = Bv + q * c;
     double s = 0.0;
     for (int r = lane; r < q; r += 32) s += cabs2(bc[r]);
     s = warp_sum(s);
-    if (lane == 0) w.sig[c] = sqrt(s);
+    if (lane == 0) sig0[c] = sqrt(s);
   }
   cta_sync();
   // stable descending order
   for (int c = tid; c < p; c += NT) {
-    double sc = w.sig[c];
+    double sc = sig0[c];
     int rank = 0;
     for (int c2 = 0; c2 < p; ++c2) {
-      double s2 = w.sig[c2];
+      double s2 = sig0[c2];
       if (s2 > sc || (s2 == sc && c2 < c)) ++rank;
     }
+    ord[rank] = c;
     w.ord[rank] = c;
   }
   cta_sync();
-  const double smax = p > 0 ? w.sig[w.ord[0]] : 0.0;
-  // rank of non-null values (sorted prefix)
+  // sorted singular values into sig (nulls zeroed); rank = their non-null prefix
+  const double smax = p > 0 ? sig0[ord[0]] : 0.0;
   int cnt = 0;
-  for (int k = tid; k < p; k += NT) {
-    double s = w.sig[w.ord[k]];
-    if (smax > 0.0 && s > SVD_NULL_TOL * smax) ++cnt;
+  for (int k2 = tid; k2 < p; k2 += NT) {
+    const double s = sig0[ord[k2]];
+    const bool live = smax > 0.0 && s > SVD_NULL_TOL * smax;
+    cnt += live ? 1 : 0;
+    w.sig[k2] = live ? s : 0.0;
   }
   res.rank = (int)block_sum((double)cnt, rs);
-  // sorted singular values into sig (nulls zeroed)
-  double sk = 0.0;
-  int myk = tid;
-  if (myk < p) {
-    double s = w.sig[w.ord[myk]];
-    sk = (smax > 0.0 && s > SVD_NULL_TOL * smax) ? s : 0.0;
-  }
-  cta_sync();
-  if (myk < p) w.sig[myk] = sk;
-  cta_sync();
   return res;
 }
 
@@ -897,8 +942,8 @@ static __device__ __noinline__ void dev_svd_vectors(const SvdResult& res, int ne
   need = min(need, p);
   const int ng = min(need, res.rank);
   for (int e = tid; e < q * ng; e += NT) {
-    int r = (int)(e % q), k = (int)(e / q);
-    w.Yo[e] = cscale(w.B[r + (long long)q * w.ord[k]], 1.0 / w.sig[k]);
+    const int k = e / q, r = e - k * q;
+    w.Yo[e] = cscale(w.B[r + q * w.ord[k]], 1.0 / w.sig[k]);
   }
   cta_sync();
   for (int k = res.rank; k < need; ++k) dev_complete_column(w.Yo, q, k, w.y, rs);
