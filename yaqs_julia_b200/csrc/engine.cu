@@ -334,6 +334,32 @@ void plan_heff(HostWMat& m, int D, int wl, int wr, int il, int ir) {
   pl.t1m = hi >= 0 ? lo : 0;
   for (auto& q : m.seg)
     if (q.side == 2) q.g -= lo;
+  // the same by environment block
+  pl.ts_ok = 1;
+  for (TsSide* sd : {&pl.left, &pl.right}) {
+    sd->nb = 0;
+    for (int b = 0; b < TS_MAX_BLOCKS; ++b)
+      for (int pp = 0; pp < 4; ++pp) sd->src[b][pp] = sd->t1[b][pp] = -1;
+  }
+  for (int pp = 0; pp < D; ++pp)
+    for (int z = pl.off[pp]; z < (pp + 1 < D ? pl.off[pp + 1] : pl.nseg); ++z) {
+      const HSeg& q = m.seg[z];
+      TsSide& sd = q.side == 0 ? pl.left : pl.right;
+      int b = 0;
+      while (b < sd.nb && sd.m[b] != q.m) ++b;
+      if (b == TS_MAX_BLOCKS || sd.src[b][pp] >= 0) {
+        pl.ts_ok = 0;
+        break;
+      }
+      if (b == sd.nb) {
+        sd.m[b] = q.m;
+        ++sd.nb;
+      }
+      sd.src[b][pp] = q.p;
+      sd.t1[b][pp] = q.side == 2 ? q.g : -1;
+      sd.coef[b][pp] = make_float2((float)q.coef.x, (float)q.coef.y);
+    }
+  if (pl.left.nb == 0 || pl.right.nb == 0) pl.ts_ok = 0;
   bool every = true;  // a block without segments would not start the GEMM's pipeline
   for (int pp = 0; pp < D; ++pp) every = every && pl.off[pp + 1] > pl.off[pp];
   m.planned = every && pl.nseg <= HEFF_MAX_SEGS && pl.nt1 * D + pl.nseg <= (wl + wr) * D;
@@ -1219,8 +1245,8 @@ static int analog_begin_impl(yaqs_ctx* ctx, const yaqs_mps_desc* psi0, const yaq
   P.tc = use_tc ? 1 : 0;
   P.tdvp_mode = cfg->tdvp_mode;
   // a 2-site sweep may cut between equal Schmidt values, where rounding
-  // decides; it keeps the order of its sums
-  P.blocked = cfg->tdvp_mode != YAQS_TDVP_2SITE ? 1 : 0;
+  // decides; in FP64 it keeps the order of its sums
+  P.blocked = mixed || cfg->tdvp_mode != YAQS_TDVP_2SITE ? 1 : 0;
   P.sample_ts = cfg->sample_timesteps != 0;
   P.max_bond = cfg->max_bond_dim;
   P.nobs = n_obs;

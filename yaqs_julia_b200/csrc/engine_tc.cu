@@ -105,8 +105,15 @@ __global__ void __launch_bounds__(2 * NT, 1) tune_heff_kernel_tc(const DevParams
   for (long long e = ltid(); e < nx; e += NT) x[e] = make_double2(1.0 / (1 + e % 13), 0.25);
   cta_sync();
   const WMat& W = D == 1 ? Q.wm_bond[bl] : D == 2 ? Q.wm_heff1[site] : Q.wm_heff2[site];
+  if (ltid() == 0) {  // the environments stand for ones next to isometric sites
+    sm.id_left[bl] = W.plan ? W.plan->il + 1 : 0;
+    sm.id_right[br] = W.plan ? W.plan->ir + 1 : 0;
+  }
+  cta_sync();
   const HeffOp h = make_heff(c, l, D, r, bl, br, W);
-  for (int k = 0; k < reps; ++k) dev_heff(h, x, y, sm.e);
+  SmallPlan sp;
+  if (!small_plan(h, sp))  // small solves take neither form
+    for (int k = 0; k < reps; ++k) dev_heff(h, x, y, sm.e);
   tc_teardown(sm.e.tc);
 }
 

@@ -35,7 +35,19 @@ struct HSeg {
   int g;           // side 2: row block of T1
   cplx coef;
 };
+// The same terms by environment block for the tensor-core product (tsgemm.cuh):
+// block b multiplies channel m[b] with, per output index p', coef * (slice
+// src of x, or of row block t1 of T1 where t1 >= 0); src < 0: no term.
+#define TS_MAX_BLOCKS 8
+struct TsSide {
+  int nb;
+  int m[TS_MAX_BLOCKS];
+  int src[TS_MAX_BLOCKS][4], t1[TS_MAX_BLOCKS][4];
+  float2 coef[TS_MAX_BLOCKS][4];
+};
 struct HPlan {
+  int ts_ok;  // one term at most per block and p', at least one block on each side
+  TsSide left, right;
   int il, ir;  // channels that have to be the identity
   int t1m, nt1, nseg, has_loc;
   int off[5];     // segments of p' are off[p'] .. off[p' + 1] - 1
@@ -195,7 +207,11 @@ struct EngineSmem {
   RedScratch r;
   KrySmem k;
   TcState tc;
+#if YAQS_TC
+  TsSide ts[2];  // left and right blocks of the solve's plan
+#else
   HSeg hseg[HEFF_MAX_SEGS];  // segments of the solve's plan
+#endif
   EngineSmemU u;
 };
 #if YAQS_TC
@@ -203,6 +219,8 @@ static_assert(sizeof(TcSmem) <= sizeof(GemmSmem), "the default pipeline must not
 #endif
 
 #if YAQS_TC
+#include "tsgemm.cuh"
+
 // Mixed form on tcgen05 (compiled only into the tensor-core kernel,
 // engine_tc.cu: a kernel that contains tcgen05 code is given one CTA per
 // SM).  x is staged as the K-major B operand of the first product, the MPO
@@ -211,6 +229,10 @@ static_assert(sizeof(TcSmem) <= sizeof(GemmSmem), "the default pipeline must not
 // once per Krylov solve.
 static __device__ void dev_heff_tc(const HeffOp& h, const cplx* x, cplx* y, EngineSmem& sm) {
   const int chil = h.chil, D = h.D, chir = h.chir, wl = h.wl, wr = h.wr;
+  if (h.plan) {
+    ts_heff(h, x, y, sm.ts, sm.u.t, sm.tc);
+    return;
+  }
   const long long n = (long long)chil * D * chir;
   // Sx[nn px + k] = x[k + chil nn], 8 loads in flight per thread
   for (long long e0 = ltid(); e0 < n; e0 += 8 * NT) {
@@ -259,6 +281,7 @@ static __device__ void dev_heff_tc(const HeffOp& h, const cplx* x, cplx* y, Engi
 }
 #endif
 
+#if !YAQS_TC
 // One output block of the structured product as a segmented GEMM.
 struct HeffProv {
   const HeffOp& h;
@@ -319,6 +342,8 @@ static __device__ __forceinline__ void heff_structured(const HeffOp& h, const cp
   for (int pp = 0; pp < h.D; ++pp) heff_block(h, x, pp, y, sm);
 }
 
+#endif
+
 // y = H_eff x.  CTA-collective.  In the mixed form x is rounded to FP32, the
 // three contractions run in FP32 (tensor cores for the two GEMMs) and y is
 // written back in FP64.
@@ -330,10 +355,12 @@ static __device__ __noinline__ void dev_heff(const HeffOp& h, const cplx* x, cpl
     return;
   }
 #endif
+#if !YAQS_TC
   if (h.plan && !h.mixed) {
     heff_structured(h, x, y, sm);
     return;
   }
+#endif
   if (h.mixed) {
     GemmSmemF& gf = reinterpret_cast<GemmSmemF&>(sm.u.gw.g);
     cta_to_f32(h.xf, x, (long long)chil * D * chir);
@@ -393,7 +420,7 @@ static __device__ __forceinline__ double heff_flops(int chil, int wl, int D, int
 
 // Floating-point operations of one product in the form it takes.
 static __device__ __forceinline__ double heff_work(const HeffOp& h) {
-  if (!h.plan || h.mixed) return heff_flops(h.chil, h.wl, h.D, h.chir, h.wr);
+  if (!h.plan || (h.mixed && !h.tc)) return heff_flops(h.chil, h.wl, h.D, h.chir, h.wr);
   const double l = h.chil, r = h.chir;
   double f = l * l * h.plan->nt1 * h.D * r;
   for (int s = 0; s < h.plan->nseg; ++s) f += h.plan->seg[s].side == 0 ? l * l * r : l * r * r;
@@ -594,7 +621,7 @@ struct SmallPlan {
 
 static __device__ __forceinline__ bool small_plan(const HeffOp& h, SmallPlan& p) {
   const int n = h.chil * h.D * h.chir;
-  if (n > SMALL_N || h.mixed) return false;
+  if (n > SMALL_N) return false;
   const int cap = (int)(sizeof(EngineSmemU) / sizeof(cplx));
   int off = h.chil * h.wl * h.chil;
   p.oR = off;

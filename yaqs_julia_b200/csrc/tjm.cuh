@@ -503,12 +503,37 @@ static __device__ HeffOp make_heff(Ctx& c, int l, int D, int r, int bl, int br, 
   h.T2 = c.ws + c.P.lay.T2;
   h.mixed = c.P.mixed;
   h.blocked = c.P.blocked;
+  const bool tc = c.P.tc && !(c.P.tune && c.P.tune[tune_index(l, D, r)] == 1);
   if (W.plan && c.sm.id_left[bl] == W.plan->il + 1 && c.sm.id_right[br] == W.plan->ir + 1) {
-    h.plan = W.plan;
-    for (int e = ltid(); e < W.plan->nseg; e += NT) c.sm.e.hseg[e] = W.plan->seg[e];
+#if YAQS_TC
+    if (tc && W.plan->ts_ok) {
+      h.plan = W.plan;
+      const int* src = reinterpret_cast<const int*>(&W.plan->left);
+      int* dst = reinterpret_cast<int*>(c.sm.e.ts);
+      for (int e = ltid(); e < (int)(2 * sizeof(TsSide) / sizeof(int)); e += NT) dst[e] = src[e];
+    }
+#else
+    if (!c.P.mixed) {
+      h.plan = W.plan;
+      for (int e = ltid(); e < W.plan->nseg; e += NT) c.sm.e.hseg[e] = W.plan->seg[e];
+    }
+#endif
     cta_sync();
   }
-  const bool tc = c.P.tc && !(c.P.tune && c.P.tune[tune_index(l, D, r)] == 1);
+  h.T1f = reinterpret_cast<cflt*>(c.ws + c.P.lay.T1f);
+  h.xf = reinterpret_cast<cflt*>(c.ws + c.P.lay.xf);
+  SmallPlan sp;
+  if (small_plan(h, sp)) return h;  // solved in shared memory, FP64
+  if (tc && h.plan) {  // the structured product reads FP32 copies of the environments
+    h.tc = 1;
+    cflt* Lf = reinterpret_cast<cflt*>(c.ws + c.P.lay.Lf);
+    cflt* Rf = reinterpret_cast<cflt*>(c.ws + c.P.lay.Rf);
+    cta_to_f32(Lf, h.L, (long long)l * h.wl * l);
+    cta_to_f32(Rf, h.R, (long long)r * h.wr * r);
+    h.Lf = Lf;
+    h.Rf = Rf;
+    return h;
+  }
   if (tc) {  // environments staged once per Krylov solve as the TMA operands
     const WsLayout& y = c.P.lay;
     h.tc = 1;
