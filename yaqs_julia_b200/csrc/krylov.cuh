@@ -209,6 +209,7 @@ struct EngineSmem {
   TcState tc;
 #if YAQS_TC
   TsSide ts[2];  // left and right blocks of the solve's plan
+  cplx loc[16];  // and its local term
 #else
   HSeg hseg[HEFF_MAX_SEGS];  // segments of the solve's plan
 #endif
@@ -230,7 +231,7 @@ static_assert(sizeof(TcSmem) <= sizeof(GemmSmem), "the default pipeline must not
 static __device__ void dev_heff_tc(const HeffOp& h, const cplx* x, cplx* y, EngineSmem& sm) {
   const int chil = h.chil, D = h.D, chir = h.chir, wl = h.wl, wr = h.wr;
   if (h.plan) {
-    ts_heff(h, x, y, sm.ts, sm.u.t, sm.tc);
+    ts_heff(h, x, y, sm.ts, sm.loc, sm.u.t, sm.tc);
     return;
   }
   const long long n = (long long)chil * D * chir;

@@ -511,6 +511,7 @@ static __device__ HeffOp make_heff(Ctx& c, int l, int D, int r, int bl, int br, 
       const int* src = reinterpret_cast<const int*>(&W.plan->left);
       int* dst = reinterpret_cast<int*>(c.sm.e.ts);
       for (int e = ltid(); e < (int)(2 * sizeof(TsSide) / sizeof(int)); e += NT) dst[e] = src[e];
+      if (ltid() < 16) c.sm.e.loc[ltid()] = W.plan->loc[ltid()];
     }
 #else
     if (!c.P.mixed) {

@@ -52,16 +52,17 @@ static_assert(sizeof(TsSmem) <= sizeof(TcSmem), "the planes must fit the tensor-
 enum { TS_RIGHT = 0, TS_LEFT = 1, TS_T1 = 2 };
 
 // One pass over all its tiles.  CTA-collective; false once a wait gave up.
-//   TS_RIGHT: y = sum + local term;  TS_LEFT: y += sum;  TS_T1: T1f = L_m x.
+//   TS_RIGHT: y = sum;  TS_LEFT: y += sum + local term;  TS_T1: T1f = L_m x.
 template <int MODE>
-static __device__ __noinline__ bool ts_pass(const HeffOp& h, const TsSide& side, const cplx* x, cplx* y, TcSmem& raw,
-                                            TcState& st) {
+static __device__ __noinline__ bool ts_pass(const HeffOp& h, const TsSide& side, const cplx* loc, const cplx* x,
+                                            cplx* y, TcSmem& raw, TcState& st) {
   ProfScope prof_scope_(PF_GEMM);
   TsSmem& s = reinterpret_cast<TsSmem&>(raw);
   const int tid = ltid(), lane = tid & 31, wid = tid >> 5;
   const int chil = h.chil, D = h.D, chir = h.chir;
-  const HPlan& pl = *h.plan;
-  const int M = MODE == TS_RIGHT ? chil * D : MODE == TS_LEFT ? D * chir : chil * pl.nt1;
+  const int nt1 = h.plan->nt1, t1m = h.plan->t1m;
+  const bool has_loc = h.plan->has_loc != 0;
+  const int M = MODE == TS_RIGHT ? chil * D : MODE == TS_LEFT ? D * chir : chil * nt1;
   const int N = MODE == TS_RIGHT ? chir : MODE == TS_LEFT ? chil : D * chir;
   const int K = MODE == TS_RIGHT ? chir : chil;
   const int nb = MODE == TS_T1 ? 1 : side.nb;
@@ -88,7 +89,7 @@ static __device__ __noinline__ bool ts_pass(const HeffOp& h, const TsSide& side,
       auto block = [&](int b) {
         pa = pb = nullptr;
         if (MODE == TS_T1) {
-          if (rok) pa = h.Lf + chil * pl.t1m + row;
+          if (rok) pa = h.Lf + chil * t1m + row;
           ka = chil * h.wl;
           if (cok) pb = h.xf + (n0 + bc) * chil;
           kb = 1;
@@ -96,7 +97,7 @@ static __device__ __noinline__ bool ts_pass(const HeffOp& h, const TsSide& side,
         }
         const int src = rok ? side.src[b][pp] : -1;
         if (MODE == TS_RIGHT) {
-          const int g = rok ? side.t1[b][pp] : -1, ld = g < 0 ? chil : chil * pl.nt1;
+          const int g = rok ? side.t1[b][pp] : -1, ld = g < 0 ? chil : chil * nt1;
           if (src >= 0) pa = (g < 0 ? h.xf : h.T1f + chil * g) + ld * src + r0;
           ka = ld * D;
           if (cok) pb = h.Rf + chir * side.m[b] + n0 + bc;
@@ -177,35 +178,70 @@ static __device__ __noinline__ bool ts_pass(const HeffOp& h, const TsSide& side,
       ok &= mbar_wait(&st.bar_mma[0], phase);
       phase ^= 1;
       tc_fence_after();
-      // epilogue: warp w reads lanes 32 (w % 4) .. +31, warps 0-3 the first 32 columns
+      // epilogue: warp w reads lanes 32 (w % 4) .. +31, warps 0-3 the first 32
+      // columns.  Loads and stores of y are dense and in batches: one element
+      // at a time, each waiting for the one before, they took 200 of the 375 us
+      // of a 64 x 2 x 64 product.
       const int quarter = wid & 3, half = wid >> 2;
-      const int er = m0 + quarter * 32 + lane;
+      const int r_base = m0 + quarter * 32;
       const unsigned lane_addr = st.tmem_base + ((unsigned)(quarter * 32) << 16);
 #pragma unroll 1
       for (int c16 = 0; c16 < 2; ++c16) {
         const int col = half * 32 + c16 * 16;
-        if (col >= nrem) break;  // uniform per warp
+        if (col >= nrem || r_base >= M) break;  // uniform per warp
         float re[16], im[16];
         tmem_ld16(lane_addr + col, re);
         tmem_ld16(lane_addr + TC_BN + col, im);
         tmem_wait_ld();
-        if (er < M) {
-          const int ep = MODE == TS_RIGHT ? er / chil : 0, ea = er - ep * chil;
+        if (MODE != TS_LEFT) {  // lanes run along the output's fast index
+          const int er = r_base + lane;
 #pragma unroll
           for (int j = 0; j < 16; ++j) {
             const int n = n0 + col + j;
-            if (n >= N) continue;
-            if (MODE == TS_T1) {
-              h.T1f[er + (long long)M * n] = make_float2(re[j], im[j]);
-            } else if (MODE == TS_RIGHT) {
-              cplx v = make_double2(re[j], im[j]);
-              if (pl.has_loc)
-                for (int p = 0; p < D; ++p) cfma(v, pl.loc[ep + D * p], x[ea + chil * (p + D * n)]);
-              y[er + chil * D * n] = v;
-            } else {
-              cplx* o = y + n + chil * er;
-              const cplx v = *o;
-              *o = make_double2(v.x + re[j], v.y + im[j]);
+            if (er < M && n < N) {
+              if (MODE == TS_T1)
+                h.T1f[er + M * n] = make_float2(re[j], im[j]);
+              else
+                y[er + M * n] = make_double2(re[j], im[j]);
+            }
+          }
+        } else {
+          // turned in shared memory (the planes are free): the fast index of y is the column
+          float2* turn = reinterpret_cast<float2*>(&s) + wid * (32 * 17);
+          __syncwarp();
+#pragma unroll
+          for (int j = 0; j < 16; ++j) turn[lane * 17 + j] = make_float2(re[j], im[j]);
+          __syncwarp();
+          const int j = lane & 15, n = n0 + col + j;
+#pragma unroll 1
+          for (int i0 = lane >> 4; i0 < 32; i0 += 16) {
+            cplx v[8];
+#pragma unroll
+            for (int u = 0; u < 8; ++u) {
+              const int er = r_base + i0 + 2 * u;
+              v[u] = er < M && n < N ? y[n + chil * er] : make_double2(0.0, 0.0);
+            }
+            if (has_loc) {
+#pragma unroll 1
+              for (int p = 0; p < D; ++p) {
+                cplx xv[8];
+#pragma unroll
+                for (int u = 0; u < 8; ++u) {
+                  const int er = r_base + i0 + 2 * u, bb = er / D;
+                  xv[u] = er < M && n < N ? x[n + chil * (p + D * bb)] : make_double2(0.0, 0.0);
+                }
+#pragma unroll
+                for (int u = 0; u < 8; ++u) {
+                  const int er = r_base + i0 + 2 * u;
+                  cfma(v[u], loc[er % D + D * p], xv[u]);
+                }
+              }
+            }
+#pragma unroll
+            for (int u = 0; u < 8; ++u) {
+              const int er = r_base + i0 + 2 * u;
+              const float2 t = turn[(i0 + 2 * u) * 17 + j];
+              if (er < M && n < N) y[n + chil * er] = make_double2(v[u].x + t.x, v[u].y + t.y);
             }
           }
         }
@@ -223,10 +259,10 @@ static __device__ __noinline__ bool ts_pass(const HeffOp& h, const TsSide& side,
 }
 
 // y = H_eff x by the plan of h; ts[0], ts[1] its left and right blocks.
-static __device__ __forceinline__ void ts_heff(const HeffOp& h, const cplx* x, cplx* y, const TsSide* ts, TcSmem& raw,
-                                               TcState& st) {
+static __device__ __forceinline__ void ts_heff(const HeffOp& h, const cplx* x, cplx* y, const TsSide* ts,
+                                               const cplx* loc, TcSmem& raw, TcState& st) {
   cta_to_f32(h.xf, x, (long long)h.chil * h.D * h.chir);
-  if (h.plan->nt1 > 0) ts_pass<TS_T1>(h, ts[0], x, y, raw, st);
-  ts_pass<TS_RIGHT>(h, ts[1], x, y, raw, st);
-  ts_pass<TS_LEFT>(h, ts[0], x, y, raw, st);
+  if (h.plan->nt1 > 0) ts_pass<TS_T1>(h, ts[0], loc, x, y, raw, st);
+  ts_pass<TS_RIGHT>(h, ts[1], loc, x, y, raw, st);
+  ts_pass<TS_LEFT>(h, ts[0], loc, x, y, raw, st);
 }
