@@ -855,6 +855,10 @@ static int setup_run(yaqs_ctx* ctx, yaqs_run* run, const std::vector<int>& cap, 
       if (!hp[k].pauli_name) P.scalar_all = 0;
       if (hp[k].lr) P.has_lr = 1;
     }
+    // sweeps, splits and normalisations leave canonical states; what may not:
+    // long-range jumps, non-unitary 1-qubit gates (digital_begin) and states
+    // put in from outside (yaqs_run_restore)
+    P.canonical = P.has_lr ? 0 : 1;
   }
 
   // initial state arena (compact tensors at the site slots)
@@ -978,6 +982,30 @@ static double mpo_antihermitian_sq(const yaqs_mpo_desc* H) {
   const double n1 = E1[0].real();
   if (n1 == 0.0) return 0.0;
   return (2.0 * n1 - 2.0 * E2[0].real()) / n1;
+}
+
+// True when the tensors left of site oc are left-isometries and those right of
+// it right-isometries, each to 1e-10 (host arithmetic; tensors packed one
+// after the other, (left, 2, right) column-major).
+static bool canonical_around(int L, const int32_t* chi, int oc, const double* tensors) {
+  const double* t = tensors;
+  for (int i = 0; i < L; ++i) {
+    const int l = chi[i], r = chi[i + 1];
+    const bool left = i < oc;
+    const int d = left ? r : l;
+    for (int x = 0; i != oc && x < d; ++x)
+      for (int y = x; y < d; ++y) {
+        hcd s = 0.0;
+        if (left) {
+          for (int e = 0; e < 2 * l; ++e) s += std::conj(cload(t, e + (size_t)2 * l * x)) * cload(t, e + (size_t)2 * l * y);
+        } else {
+          for (int e = 0; e < 2 * r; ++e) s += cload(t, x + (size_t)l * e) * std::conj(cload(t, y + (size_t)l * e));
+        }
+        if (!(std::abs(s - (x == y ? 1.0 : 0.0)) < 1e-10)) return false;
+      }
+    t += (size_t)4 * l * r;
+  }
+  return true;
 }
 
 // Largest squared relative anti-Hermitian part accepted for a Hamiltonian:
@@ -1416,6 +1444,7 @@ int yaqs_run_restore(yaqs_run* run, int32_t traj, const int32_t* chi, int32_t oc
   if (chi[0] != 1 || chi[L] != 1) return set_err(ctx, YAQS_E_ARG, "boundary bonds must be 1");
   for (int b = 0; b <= L; ++b)
     if (chi[b] < 1 || chi[b] > cap[b]) return set_err(ctx, YAQS_E_ARG, "bond dimension beyond this run's capacity");
+  if (!canonical_around(L, chi, oc, tensors)) run->P.canonical = 0;  // the caller's tensors may be in any gauge
   cplx* base = run->P.phi + (size_t)traj * run->P.mps_size;
   const double* src = tensors;
   for (int i = 0; i < L; ++i) {
@@ -1763,6 +1792,16 @@ int digital_begin(yaqs_ctx* ctx, const yaqs_mps_desc* psi0, const yaqs_gate_desc
       d.wm = -1;
       const int dd = q.kind == YAQS_GATE_2Q ? 4 : 2;
       for (int e = 0; e < dd * dd; ++e) d.mat[e] = make_double2(q.matrix[2 * e], q.matrix[2 * e + 1]);
+      if (dd == 2) {  // applied off the centre: keeps the gauge only when unitary
+        double dev = 0.0;
+        for (int i = 0; i < 2; ++i)
+          for (int j = 0; j < 2; ++j) {
+            hcd v = i == j ? -1.0 : 0.0;
+            for (int k = 0; k < 2; ++k) v += std::conj(cload(q.matrix, k + 2 * i)) * cload(q.matrix, k + 2 * j);
+            dev = std::max(dev, std::abs(v));
+          }
+        if (!(dev < 1e-12)) P.canonical = 0;
+      }
       if (by_tdvp(q)) {
         // construct_window_mpo (DigitalTJM.jl:192-236): coeff g(s1) on the
         // first window site, g(s2) on the last, identities between, bond 1

@@ -112,6 +112,7 @@ __global__ void __launch_bounds__(2 * NT, 1) tune_heff_kernel_tc(const DevParams
   cta_sync();
   const HeffOp h = make_heff(c, l, D, r, bl, br, W);
   SmallPlan sp;
+  if (h.tc && h.plan) cta_to_f32(h.xf, x, nx);
   if (!small_plan(h, sp))  // small solves take neither form
     for (int k = 0; k < reps; ++k) dev_heff(h, x, y, sm.e);
   tc_teardown(sm.e.tc);

@@ -898,8 +898,9 @@ static __device__ __noinline__ double predicted_dots(const cplx* Q, long long qs
 
 // out = s (w - sum_{j<k} h_j q_j) with h in ks.h; w null: no w.  One pass,
 // eight vectors and two values a thread at a time.  CTA-collective.
+// With out32 the result is also stored in FP32.
 static __device__ __noinline__ void combine_pass(const cplx* Q, long long qs, const cplx* w, cplx* out, int n, int k,
-                                                 double s, EngineSmem& sm) {
+                                                 double s, EngineSmem& sm, cflt* out32 = nullptr) {
   const cplx* h = sm.k.h;
 #pragma unroll 1
   for (int i0 = ltid(); i0 < n; i0 += 2 * NT) {
@@ -922,8 +923,14 @@ static __device__ __noinline__ void combine_pass(const cplx* Q, long long qs, co
         cfma(v1, nc, a1[e]);
       }
     }
-    out[i0] = cscale(v0, s);
-    if (i1 != i0) out[i1] = cscale(v1, s);
+    v0 = cscale(v0, s);
+    v1 = cscale(v1, s);
+    out[i0] = v0;
+    if (i1 != i0) out[i1] = v1;
+    if (out32) {
+      out32[i0] = make_float2((float)v0.x, (float)v0.y);
+      if (i1 != i0) out32[i1] = make_float2((float)v1.x, (float)v1.y);
+    }
   }
   cta_sync();
 }
@@ -936,7 +943,13 @@ static __device__ __noinline__ int dev_expm_predicted(const HeffOp& h, cplx* x, 
   const double beta0 = sqrt(cta_norm2(x, n, sm.r));
   if (beta0 == 0.0) return 0;
   const double tau = fabs(dt);
-  for (int i = tid; i < n; i += NT) Q[i] = cscale(x[i], 1.0 / beta0);
+  // the structured mixed product takes its vector in FP32 from here
+  cflt* xf = h.tc && h.plan ? h.xf : nullptr;
+  for (int i = tid; i < n; i += NT) {
+    const cplx v = cscale(x[i], 1.0 / beta0);
+    Q[i] = v;
+    if (xf) xf[i] = make_float2((float)v.x, (float)v.y);
+  }
   if (tid <= KRYLOV_MAX) sm.k.h[tid] = make_double2(0.0, 0.0);  // combine_pass reads whole groups
   cta_sync();
   double bound = 1.0, sigma = 0.0, beta = 0.0;
@@ -976,7 +989,7 @@ static __device__ __noinline__ int dev_expm_predicted(const HeffOp& h, cplx* x, 
     bound *= b_k * tau / k;
     if (kc.exit_tol > 0.0 && bound <= kc.exit_tol) break;
     if (tid == 0) sm.k.beta[k - 1] = b_k;
-    combine_pass(Q, qs, w, w, n, k, 1.0 / b_k, sm);
+    combine_pass(Q, qs, w, w, n, k, 1.0 / b_k, sm, xf);
     if (k == 1) sigma = a_k;
     beta = b_k;
   }

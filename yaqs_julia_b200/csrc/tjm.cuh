@@ -87,6 +87,7 @@ struct DevParams {
   // right site, 1-site observables by site: entries off[i] .. off[i+1]-1 of
   // idx are the indices that belong to site i, ascending.
   const int *p0_off, *p0_idx, *p1_off, *p1_idx, *ob_off, *ob_idx;
+  int canonical;   // recorded states are in mixed canonical form around their centre
   int blocked;     // panel QR and short Jacobi rounds (LinalgSmem::blocked)
   int scalar_all;  // every process is a scalar dissipator (pauli_name)
   int has_lr;      // some process is long-range
@@ -1181,6 +1182,70 @@ static __device__ __noinline__ bool local_by_envs(Ctx& c, const DState& s, int c
   const int L = P.L;
   const int nlocal = P.ob_off[L];
   if (nlocal == 0 || !chain_tight(c, s)) return false;
+  double* vals = reinterpret_cast<double*>(c.ws + P.lay.dbl) + SVD_MAX_COLS;  // one value per observable
+  auto record = [&]() {
+    cta_sync();
+    for (int z = ltid(); z < nlocal; z += NT) {
+      const int k = P.ob_idx[z];
+      P.traj_out[((long long)c.traj * P.nobs + k) * P.ncols + col] = vals[k];
+    }
+    cta_sync();
+  };
+  if (P.canonical) {
+    // Mixed canonical form around the centre: the environments left and right
+    // of it are identities, so each site needs one product for its values and
+    // one to step outwards, two GEMMs instead of six.
+    cplx* Ea = c.ws + P.lay.tA;
+    cplx* Eb = c.ws + P.lay.tB;
+    cplx* T = c.ws + P.lay.tC;
+    GemmSmem& gm = c.sm.e.u.gw.g;
+    auto values = [&](int i, const cplx* A, const cplx* V) {
+      for (int z = P.ob_off[i]; z < P.ob_off[i + 1]; ++z) {
+        const int k = P.ob_idx[z];
+        const double v = env_expect(c, A, V, s.chi[i], s.chi[i + 1], P.obs[k].mat);
+        if (ltid() == 0) vals[k] = v;
+      }
+    };
+    const int oc = *s.oc;
+    cta_sync();
+    // rightwards: V[a',p,r] = sum_a E[a,a'] A[a,p,r], E'[r,r'] = sum V[a',p,r] conj(A[a',p,r'])
+    const cplx* E = nullptr;  // identity
+    for (int i = oc; i < L; ++i) {
+      const int l = s.chi[i], r = s.chi[i + 1];
+      const cplx* A = site_ptr(c, s, i);
+      const cplx* V = A;
+      if (E) {
+        cta_gemm(gemm_args(l, 2 * r, l, E, l, 1, A, 1, l, T, 1, l), gm);
+        V = T;
+      }
+      values(i, A, V);
+      if (i + 1 < L && P.ob_off[i + 1] < P.ob_off[L]) {
+        cplx* En = E == Ea ? Eb : Ea;
+        cta_gemm(gemm_args(r, r, 2 * l, V, 2 * l, 1, A, 1, 2 * l, En, 1, r, false, true), gm);
+        E = En;
+      } else {
+        break;  // no observable further right
+      }
+    }
+    // leftwards: R[x,y] = sum V[x,p,r'] conj(A[y,p,r']) from the centre, V[(a,p),r'] = sum_r A[a,p,r] R[r,r']
+    cplx* R = nullptr;
+    for (int i = oc; i >= 0; --i) {
+      const int l = s.chi[i], r = s.chi[i + 1];
+      const cplx* A = site_ptr(c, s, i);
+      const cplx* V = A;
+      if (R) {
+        cta_gemm(gemm_args(2 * l, r, r, A, 1, 2 * l, R, 1, r, T, 1, 2 * l), gm);
+        V = T;
+        values(i, A, V);
+      }
+      if (P.ob_off[i] == 0) break;  // no observable further left
+      cplx* Rn = R == Ea ? Eb : Ea;
+      cta_gemm(gemm_args(l, l, 2 * r, V, 1, l, A, l, 1, Rn, 1, l, false, true), gm);
+      R = Rn;
+    }
+    record();
+    return true;
+  }
   long long need = 0;
   for (int b = 1; b <= L; ++b) need += (long long)s.chi[b] * s.chi[b];
   cplx* Rs;
@@ -1211,7 +1276,6 @@ static __device__ __noinline__ bool local_by_envs(Ctx& c, const DState& s, int c
     // R_b[x, y] = sum_{p,r'} X[x,p,r'] conj(A[y,p,r'])
     cta_gemm(gemm_args(l, l, 2 * r, T1, 1, l, A, l, 1, Rs + off, 1, l, false, true), gs);
   }
-  double* vals = reinterpret_cast<double*>(c.ws + P.lay.dbl) + SVD_MAX_COLS;  // one value per observable
   off = need;  // R_{i+1} at off - chi_{i+1}^2
   for (int i = 0; i < L; ++i) {
     const int l = s.chi[i], r = s.chi[i + 1];
@@ -1237,12 +1301,7 @@ static __device__ __noinline__ bool local_by_envs(Ctx& c, const DState& s, int c
       E1 = t;
     }
   }
-  cta_sync();
-  for (int z = ltid(); z < nlocal; z += NT) {
-    const int k = P.ob_idx[z];
-    P.traj_out[((long long)c.traj * P.nobs + k) * P.ncols + col] = vals[k];
-  }
-  cta_sync();
+  record();
   return true;
 }
 

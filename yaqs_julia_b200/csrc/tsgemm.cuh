@@ -258,10 +258,10 @@ static __device__ __noinline__ bool ts_pass(const HeffOp& h, const TsSide& side,
   return good;
 }
 
-// y = H_eff x by the plan of h; ts[0], ts[1] its left and right blocks.
+// y = H_eff x by the plan of h; ts[0], ts[1] its left and right blocks.  h.xf
+// holds x in FP32.
 static __device__ __forceinline__ void ts_heff(const HeffOp& h, const cplx* x, cplx* y, const TsSide* ts,
                                                const cplx* loc, TcSmem& raw, TcState& st) {
-  cta_to_f32(h.xf, x, (long long)h.chil * h.D * h.chir);
   if (h.plan->nt1 > 0) ts_pass<TS_T1>(h, ts[0], loc, x, y, raw, st);
   ts_pass<TS_RIGHT>(h, ts[1], loc, x, y, raw, st);
   ts_pass<TS_LEFT>(h, ts[0], loc, x, y, raw, st);
