@@ -352,6 +352,7 @@ int yaqs_server_create(yaqs_ctx* ctx, const yaqs_server_config* cfg, yaqs_server
   srv->ictx.device = ctx->device;
   srv->ictx.sms = ctx->sms;
   CUDA_TRY(ctx, cudaSetDevice(ctx->device));
+  srv->ictx.pool = make_pool(ctx->device);
   // slot shape: the largest analog and digital layouts the config admits
   const int L = cfg->max_L;
   std::vector<int> wmax(L + 1, cfg->max_mpo_width), wone(L + 1, 1);
