@@ -59,6 +59,13 @@ struct ProfScope {
   }
 };
 
+// Routines that are not inlined see shared memory through plain pointers and
+// would load it as generic memory, slower and on the global scoreboard; this
+// tells the compiler where a pointer points.  For routines whose pointer is
+// always shared; dev_svd, which picks between the staging buffer and global
+// memory, came out wrong with it and takes plain pointers.
+#define ASSUME_SHARED(p) __builtin_assume(__isShared((const void*)(p)))
+
 static __device__ __forceinline__ cplx cmk(double x, double y) { return make_double2(x, y); }
 static __device__ __forceinline__ cplx cadd(cplx a, cplx b) { return make_double2(a.x + b.x, a.y + b.y); }
 static __device__ __forceinline__ cplx csub(cplx a, cplx b) { return make_double2(a.x - b.x, a.y - b.y); }
@@ -134,6 +141,7 @@ struct RedScratch {
 // loads).
 template <int NV>
 static __device__ __forceinline__ void block_sum_n(double (&x)[NV], RedScratch& rs) {
+  ASSUME_SHARED(&rs);
   const int lane = ltid() & 31, wid = ltid() >> 5;
   if (NV == 16) {
     warp_sum_multi<NV>(x);
@@ -176,6 +184,7 @@ static __device__ __forceinline__ double block_sum(double v, RedScratch& rs) {
 }
 
 static __device__ __forceinline__ double block_max(double v, RedScratch& rs) {
+  ASSUME_SHARED(&rs);
   const int lane = ltid() & 31, wid = ltid() >> 5;
   v = warp_max(v);
   if (lane == 0) rs.v[wid] = v;

@@ -126,6 +126,7 @@ template <int GBK, class Prov, class Epi>
 static __device__ __forceinline__ void gemm_core(const Prov& pv, int M, int N, bool conjA, bool conjB, Epi epi,
                                                  GemmSmem& sm) {
   constexpr int GSTAGES = GROWS / GBK;
+  ASSUME_SHARED(&sm);
   const int tid = ltid();
   const int lane = tid & 31, wid = tid >> 5;
   const int wm = wid & 1, wn = wid >> 1;  // 2 x NW/2 warps

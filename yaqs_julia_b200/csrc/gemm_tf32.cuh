@@ -120,6 +120,7 @@ static __device__ __forceinline__ void store_c(cplx* c, float re, float im, bool
 template <bool CA, bool CB, class TC>
 static __device__ __noinline__ void cta_gemm_tf32_t(const GemmArgsF g, GemmSmemF& sm) {
   ProfScope prof_scope_(PF_GEMM);
+  ASSUME_SHARED(&sm);
   const int tid = ltid();
   const int lane = tid & 31, wid = tid >> 5;
   const int wm = wid & 1, wn = wid >> 1;  // 2 x 4 warps

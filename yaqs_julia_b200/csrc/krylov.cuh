@@ -104,6 +104,7 @@ template <class T>
 static __device__ __noinline__ void dev_wapply(const T* in, T* out, const WMat W,
                                         const WApplyGeom g, WApplySmem& ws) {
   ProfScope prof_scope_(PF_WAPPLY);
+  ASSUME_SHARED(&ws);
   T* sin = reinterpret_cast<T*>(&ws.in[0]);
   const int cap = (int)(WAPPLY_IN_CPLX * sizeof(cplx) / sizeof(T));
   const int PT = W.ni * NT <= cap ? NT : (W.ni * (NT / 2) <= cap ? NT / 2 : NT / 4);
@@ -445,6 +446,7 @@ struct KrylovCfg {
 // from a table filled once.
 static __device__ __noinline__ void dev_tridiag_expm(int m, double dt, KrySmem& ks) {
   ProfScope prof_scope_(PF_TRIDIAG);
+  ASSUME_SHARED(&ks);
   if (ltid() >= 32) return;
   const int j = ltid();
   const bool on = j < m;
@@ -709,6 +711,7 @@ static __device__ __forceinline__ void small_heff(const HeffOp& h, const SmallPl
 // the general path's threads, warps and block add them.
 static __device__ __noinline__ double small_dots(const cplx* sQ, int nfit, const cplx* Q, long long qs, const cplx* w,
                                                  int n, int k, KrySmem& ks) {
+  ASSUME_SHARED(&ks);
   const int lane = ltid() & 31, wid = ltid() >> 5;
 #pragma unroll 1
   for (int j = wid; j <= k; j += NW) {  // j = k: the norm
@@ -746,6 +749,7 @@ static __device__ __noinline__ double small_dots(const cplx* sQ, int nfit, const
 // dev_expm_krylov for a solve that fits small_plan.
 static __device__ __noinline__ int dev_expm_small(const HeffOp& h, const SmallPlan& p, cplx* x, double dt,
                                                   const KrylovCfg& kc, cplx* Q, long long qs, EngineSmem& sm) {
+  ASSUME_SHARED(&sm);
   cplx* buf = reinterpret_cast<cplx*>(&sm.u);
   cplx* sQ = buf + p.oQ;
   KrySmem& ks = sm.k;
@@ -841,6 +845,7 @@ static __device__ __noinline__ int dev_expm_small(const HeffOp& h, const SmallPl
 // values a thread keep 16 loads in flight.  CTA-collective.
 static __device__ __noinline__ double predicted_dots(const cplx* Q, long long qs, const cplx* w, int n, int k,
                                                      double sigma, double beta, EngineSmem& sm) {
+  ASSUME_SHARED(&sm);
   const int tid = ltid(), lane = tid & 31, wid = tid >> 5;
   const cplx* q0 = Q + qs * (k - 1);
   const cplx* q1 = k > 1 ? q0 - qs : q0;
@@ -901,6 +906,7 @@ static __device__ __noinline__ double predicted_dots(const cplx* Q, long long qs
 // With out32 the result is also stored in FP32.
 static __device__ __noinline__ void combine_pass(const cplx* Q, long long qs, const cplx* w, cplx* out, int n, int k,
                                                  double s, EngineSmem& sm, cflt* out32 = nullptr) {
+  ASSUME_SHARED(&sm);
   const cplx* h = sm.k.h;
 #pragma unroll 1
   for (int i0 = ltid(); i0 < n; i0 += 2 * NT) {

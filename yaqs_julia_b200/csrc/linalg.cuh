@@ -243,6 +243,8 @@ static __device__ __forceinline__ void dev_qr_extract_r(const cplx* H, int m, in
 template <int CH, int CG>
 static __device__ __noinline__ void qr_apply(cplx* X, int ld, int c0, int c1, const cplx* V, int m, int ja, int jb,
                                              bool ascending, int ident, const cplx* tau) {
+  ASSUME_SHARED(V);
+  ASSUME_SHARED(tau);
   constexpr int NV = 2 * CG;
   constexpr int SH = NV == 2 ? 4 : NV == 4 ? 3 : NV == 8 ? 2 : 1;  // lane of value v: v << SH
   const int lane = ltid() & 31, wid = ltid() >> 5;
@@ -309,6 +311,8 @@ static __device__ __noinline__ void qr_apply(cplx* X, int ld, int c0, int c1, co
 // (pe - ja) in shared memory, ld m) with the columns up to pe updated.
 template <int CH>
 static __device__ __noinline__ void qr_panel(cplx* V, int m, int ja, int jb, int pe, double null_abs, cplx* tau) {
+  ASSUME_SHARED(V);
+  ASSUME_SHARED(tau);
   const int lane = ltid() & 31, wid = ltid() >> 5;
   cplx v[CH];
   double diag = 0.0;
@@ -642,6 +646,7 @@ static __device__ __forceinline__ bool jacobi_params(double al, double be, doubl
 template <class PairFn>
 static __device__ __forceinline__ void smem_rotate_round(cplx* sb, int ld, int q, int rows, int npairs, PairFn pairs,
                                                   double tol, int* rot) {
+  ASSUME_SHARED(sb);
   const int hl = ltid() & 15, hw = ltid() >> 4;
   const unsigned mask = (ltid() & 16) ? 0xffff0000u : 0x0000ffffu;
   for (int k = hw; k < npairs; k += NT / 16) {
@@ -687,6 +692,7 @@ static __device__ __forceinline__ void smem_rotate_round(cplx* sb, int ld, int q
 template <int LP, class PairFn>
 static __device__ __forceinline__ void smem_rotate_short(cplx* sb, int ld, int q, int npairs, PairFn pairs, double tol2,
                                                          int* rot) {
+  ASSUME_SHARED(sb);
   const int hl = ltid() & (LP - 1), grp = ltid() / LP;
   const int base = (ltid() & 31) & ~(LP - 1);
   const unsigned mask = ((LP == 32 ? 0u : (1u << (LP & 31))) - 1u) << base;

@@ -57,6 +57,9 @@ template <int MODE>
 static __device__ __noinline__ bool ts_pass(const HeffOp& h, const TsSide& side, const cplx* loc, const cplx* x,
                                             cplx* y, TcSmem& raw, TcState& st) {
   ProfScope prof_scope_(PF_GEMM);
+  ASSUME_SHARED(&raw);
+  ASSUME_SHARED(&side);
+  ASSUME_SHARED(loc);
   TsSmem& s = reinterpret_cast<TsSmem&>(raw);
   const int tid = ltid(), lane = tid & 31, wid = tid >> 5;
   const int chil = h.chil, D = h.D, chir = h.chir;
