@@ -31,6 +31,21 @@ def test_saturated_sweeps_match_oracle(oracle, chi, tdvp):
     assert np.array_equal(got.max_bond, chi_ref)
 
 
+@pytest.mark.parametrize("chi", [33, 70])
+def test_entropy_of_wide_bonds_matches_oracle(oracle, chi):
+    """Singular values of 2 chi x chi centre tensors: 66 rows take 16 lanes a
+    pair, 140 rows a whole warp."""
+    L = 15
+    obs = [api.Observable("S7", None, 7, kind="entropy"), api.Observable("S8", None, 8, kind="entropy")]
+    cfg = api.TimeEvolutionConfig(obs, 0.0, dt=0.05, num_traj=1, max_bond_dim=chi, order=1)
+    nm = api.NoiseModel([{"name": "pauli_z", "sites": [1], "strength": 0.1}], L)
+    d = api.Descriptors(api.random_mps(L, chi, seed=1), api.init_ising(L, 1.0, 0.5), cfg, nm, seed=3,
+                        tdvp_mode=api.TDVP_MODES["1site"])
+    ref, _, _ = oracle.analog_run(d)
+    got = api.run_descriptors(d)
+    assert np.abs(got.trajectories - ref).max() <= 1e-10 * np.abs(ref).max()
+
+
 @pytest.mark.parametrize("threads", ["128", "256"])
 def test_circuit_bonds_match_oracle(oracle, threads, monkeypatch):
     monkeypatch.setenv("YAQS_DIGITAL_THREADS", threads)

@@ -31,9 +31,13 @@ struct LinalgSmem {
 // Householder QR
 // ---------------------------------------------------------------------------
 // Factor H (m x n, col-major, ld m) in place: R in the upper triangle,
-// reflector vectors below, scalars in ls.tau.  CTA-collective.
-static __device__ __noinline__ void dev_qr_factor(cplx* H, int m, int n, LinalgSmem& ls, RedScratch& rs) {
+// reflector vectors below, scalars in ls.tau.  SHARED: H lies in shared
+// memory.  CTA-collective.
+template <bool SHARED>
+static __device__ __noinline__ void dev_qr_factor_at(cplx* H, int m, int n, LinalgSmem& ls, RedScratch& rs) {
   ProfScope prof_scope_(PF_QR);
+  if (SHARED) ASSUME_SHARED(H);
+  ASSUME_SHARED(&ls);
   const int tid = ltid(), lane = tid & 31, wid = tid >> 5;
   const int kq = min(m, n);
   double fro2 = cta_norm2(H, (long long)m * n, rs);
@@ -131,9 +135,17 @@ static __device__ __noinline__ void dev_qr_factor(cplx* H, int m, int n, LinalgS
   }
 }
 
-// Q (m x kq) of a factored H.  CTA-collective.
-static __device__ __noinline__ void dev_qr_formq(const cplx* H, int m, int n, cplx* Q, LinalgSmem& ls) {
+static __device__ __forceinline__ void dev_qr_factor(cplx* H, int m, int n, LinalgSmem& ls, RedScratch& rs) {
+  dev_qr_factor_at<false>(H, m, n, ls, rs);
+}
+
+// Q (m x kq) of a factored H; SHARED: both in shared memory.  CTA-collective.
+template <bool SHARED>
+static __device__ __noinline__ void dev_qr_formq_at(const cplx* H, int m, int n, cplx* Q, LinalgSmem& ls) {
   ProfScope prof_scope_(PF_QRQ);
+  if (SHARED) ASSUME_SHARED(H);
+  if (SHARED) ASSUME_SHARED(Q);
+  ASSUME_SHARED(&ls);
   const int tid = ltid(), lane = tid & 31, wid = tid >> 5;
   const int kq = min(m, n);
   for (int e = tid; e < m * kq; e += NT) {
@@ -208,6 +220,10 @@ static __device__ __noinline__ void dev_qr_formq(const cplx* H, int m, int n, cp
     }
     cta_sync();
   }
+}
+
+static __device__ __forceinline__ void dev_qr_formq(const cplx* H, int m, int n, cplx* Q, LinalgSmem& ls) {
+  dev_qr_formq_at<false>(H, m, n, Q, ls);
 }
 
 // R (kq x n) of a factored H into Rout (ld kq), zero below the diagonal.
@@ -527,8 +543,14 @@ static __device__ __forceinline__ void dev_qr_thin(int m, int n, Load load, cplx
   cta_sync();  // the shared buffer's last readers are done
   for (int e = ltid(); e < m * n; e += NT) h[e] = load(e);
   cta_sync();
-  dev_qr_factor(h, m, n, ls, rs);
-  dev_qr_formq(h, m, n, q, ls);
+  if (h == sb)
+    dev_qr_factor_at<true>(h, m, n, ls, rs);
+  else
+    dev_qr_factor_at<false>(h, m, n, ls, rs);
+  if (h == sb && q != Qg)
+    dev_qr_formq_at<true>(h, m, n, q, ls);
+  else
+    dev_qr_formq_at<false>(h, m, n, q, ls);
   dev_qr_extract_r(h, m, n, Rout);
   for (int e = ltid(); e < m * k; e += NT) store_q(e, q);
   cta_sync();
@@ -663,12 +685,23 @@ static __device__ __forceinline__ void smem_rotate_round(cplx* sb, int ld, int q
       gx += x.x * y.x + x.y * y.y;
       gy += x.x * y.y - x.y * y.x;
     }
-#pragma unroll
-    for (int o = 8; o > 0; o >>= 1) {
-      al += __shfl_xor_sync(mask, al, o);
-      be += __shfl_xor_sync(mask, be, o);
-      gx += __shfl_xor_sync(mask, gx, o);
-      gy += __shfl_xor_sync(mask, gy, o);
+    {  // the four trees over 16 lanes with the values halved twice: same pairs, 9 shuffles instead of 16
+      const int base = (ltid() & 31) & 16;
+      bool up = (hl & 8) != 0;
+      double k0 = up ? gx : al, k1 = up ? gy : be;
+      const double g0 = up ? al : gx, g1 = up ? be : gy;
+      k0 += __shfl_xor_sync(mask, g0, 8);
+      k1 += __shfl_xor_sync(mask, g1, 8);
+      up = (hl & 4) != 0;
+      double v = up ? k1 : k0;
+      const double g = up ? k0 : k1;
+      v += __shfl_xor_sync(mask, g, 4);
+      v += __shfl_xor_sync(mask, v, 2);
+      v += __shfl_xor_sync(mask, v, 1);
+      al = __shfl_sync(mask, v, base);
+      be = __shfl_sync(mask, v, base + 4);
+      gx = __shfl_sync(mask, v, base + 8);
+      gy = __shfl_sync(mask, v, base + 12);
     }
     double c;
     cplx se, sec;
@@ -683,81 +716,123 @@ static __device__ __forceinline__ void smem_rotate_round(cplx* sb, int ld, int q
   cta_sync();
 }
 
-// The same round with LP lanes a pair, the four sums reduced together and the
-// rotation from two reciprocal square roots: with R = sqrt(d^2 + 4 |g|^2),
-//   cos^2 = (1 + |d| / R) / 2,  sin / |g| = 1 / (R cos)
-// instead of a chain of rsqrt, sqrt, division and rsqrt.  A round is one
-// dependent chain of loads, shuffles and these, so its length is its cost.
-// For the runs that may reorder sums.
-template <int LP, class PairFn>
-static __device__ __forceinline__ void smem_rotate_short(cplx* sb, int ld, int q, int npairs, PairFn pairs, double tol2,
-                                                         int* rot) {
-  ASSUME_SHARED(sb);
+// All rounds of one diagonal block (cross = false: n0 columns, round-robin
+// over be2 places) or of one pair of blocks (cross: columns kk < n0 against
+// joff + (kk + t) mod b for t = 0 .. b-1), LP lanes a pair, RPL rows a lane.
+// For the runs that may reorder sums.  A round is one dependent chain, so its
+// length is its cost: both columns are loaded at once and stay in registers
+// for the update, the four sums are reduced together, and the rotation comes
+// from two reciprocal square roots: with R = sqrt(d^2 + 4 |g|^2),
+//   cos^2 = (1 + |d| / R) / 2,  sin / |g| = 1 / (R cos),
+// instead of a chain of rsqrt, sqrt, division and rsqrt.
+template <int LP, int RPL>
+static __device__ __noinline__ void jacobi_rounds(cplx* cols, int ld, int q, bool cross, int b, int n0, int n1, int joff,
+                                                  double tol2, int* rot) {
+  ASSUME_SHARED(cols);
   const int hl = ltid() & (LP - 1), grp = ltid() / LP;
   const int base = (ltid() & 31) & ~(LP - 1);
-  const unsigned mask = ((LP == 32 ? 0u : (1u << (LP & 31))) - 1u) << base;
+  const unsigned mask = LP == 32 ? 0xffffffffu : ((1u << (LP & 31)) - 1u) << base;
+  const int be2 = b + (b & 1);
+  const int rounds = cross ? b : be2 - 1, npairs = cross ? b : be2 / 2;
 #pragma unroll 1
-  for (int k = grp; k < npairs; k += NT / LP) {
-    int i, j;
-    pairs(k, i, j);
-    if (i < 0 || j < 0) continue;
-    cplx* bi = sb + ld * i;
-    cplx* bj = sb + ld * j;
-    double d4[4] = {0.0, 0.0, 0.0, 0.0};  // |b_i|^2, |b_j|^2, b_i^H b_j
-#pragma unroll 2
-    for (int r = hl; r < q; r += LP) {
-      const cplx x = bi[r], y = bj[r];
-      d4[0] = fma(x.x, x.x, fma(x.y, x.y, d4[0]));
-      d4[1] = fma(y.x, y.x, fma(y.y, y.y, d4[1]));
-      d4[2] = fma(x.x, y.x, fma(x.y, y.y, d4[2]));
-      d4[3] = fma(x.x, y.y, fma(-x.y, y.x, d4[3]));
-    }
-    {  // butterfly over the pair's lanes, halving the values twice
-      bool up = (hl & (LP / 2)) != 0;
-#pragma unroll
-      for (int e = 0; e < 2; ++e) {
-        const double keep = up ? d4[e + 2] : d4[e], give = up ? d4[e] : d4[e + 2];
-        d4[e] = keep + __shfl_xor_sync(mask, give, LP / 2);
+  for (int t = 0; t < rounds; ++t) {
+#pragma unroll 1
+    for (int k = grp; k < npairs; k += NT / LP) {
+      int i, j;
+      if (cross) {
+        i = k;
+        j = k + t < b ? k + t : k + t - b;
+        if (i >= n0 || j >= n1) continue;
+        j += joff;
+      } else {
+        // place p holds column ((p - 1 - t) mod (be2 - 1)) + 1, place 0 column 0
+        const int tb = be2 - 1 - k;
+        int x = k == 0 ? 0 : k - t, y = tb == 0 ? 0 : tb - t;
+        if (k != 0 && x < 1) x += be2 - 1;
+        if (tb != 0 && y < 1) y += be2 - 1;
+        i = min(x, y);
+        j = max(x, y);
+        if (j >= n0) continue;
       }
-      up = (hl & (LP / 4)) != 0;
-      const double keep = up ? d4[1] : d4[0], give = up ? d4[0] : d4[1];
-      d4[0] = keep + __shfl_xor_sync(mask, give, LP / 4);
+      cplx* bi = cols + ld * i;
+      cplx* bj = cols + ld * j;
+      cplx x[RPL], y[RPL];
 #pragma unroll
-      for (int o = LP / 8; o > 0; o >>= 1) d4[0] += __shfl_xor_sync(mask, d4[0], o);
+      for (int u = 0; u < RPL; ++u) {
+        const int r = hl + LP * u;
+        x[u] = r < q ? bi[r] : make_double2(0.0, 0.0);
+        y[u] = r < q ? bj[r] : make_double2(0.0, 0.0);
+      }
+      double d4[4] = {0.0, 0.0, 0.0, 0.0};  // |b_i|^2, |b_j|^2, b_i^H b_j
+#pragma unroll
+      for (int u = 0; u < RPL; ++u) {
+        d4[0] = fma(x[u].x, x[u].x, fma(x[u].y, x[u].y, d4[0]));
+        d4[1] = fma(y[u].x, y[u].x, fma(y[u].y, y[u].y, d4[1]));
+        d4[2] = fma(x[u].x, y[u].x, fma(x[u].y, y[u].y, d4[2]));
+        d4[3] = fma(x[u].x, y[u].y, fma(-x[u].y, y[u].x, d4[3]));
+      }
+      {  // butterfly over the pair's lanes, halving the values twice
+        bool up = (hl & (LP / 2)) != 0;
+#pragma unroll
+        for (int e = 0; e < 2; ++e) {
+          const double keep = up ? d4[e + 2] : d4[e], give = up ? d4[e] : d4[e + 2];
+          d4[e] = keep + __shfl_xor_sync(mask, give, LP / 2);
+        }
+        up = (hl & (LP / 4)) != 0;
+        const double keep = up ? d4[1] : d4[0], give = up ? d4[0] : d4[1];
+        d4[0] = keep + __shfl_xor_sync(mask, give, LP / 4);
+#pragma unroll
+        for (int o = LP / 8; o > 0; o >>= 1) d4[0] += __shfl_xor_sync(mask, d4[0], o);
+      }
+      const double al = __shfl_sync(mask, d4[0], base), be = __shfl_sync(mask, d4[0], base + LP / 4);
+      const double gx = __shfl_sync(mask, d4[0], base + LP / 2), gy = __shfl_sync(mask, d4[0], base + 3 * LP / 4);
+      const double g2 = fma(gx, gx, gy * gy);
+      if (!(g2 > tol2 * (al * be))) continue;
+      if (hl == 0) *rot = 1;  // any rotation keeps the sweeps going
+      const double d = be - al;
+      const double h = rsqrt(fma(d, d, 4.0 * g2));
+      const double c2 = fma(0.5 * fabs(d), h, 0.5);
+      const double rc = rsqrt(c2);
+      const double c = c2 * rc, f = d < 0.0 ? -h * rc : h * rc;
+      const cplx se = make_double2(f * gx, f * gy);
+#pragma unroll
+      for (int u = 0; u < RPL; ++u) {
+        const int r = hl + LP * u;
+        if (r < q) {
+          const cplx a = x[u], e = y[u];
+          // b_i <- c b_i - conj(se) b_j,  b_j <- se b_i + c b_j
+          bi[r] = make_double2(fma(c, a.x, fma(-se.x, e.x, -se.y * e.y)), fma(c, a.y, fma(-se.x, e.y, se.y * e.x)));
+          bj[r] = make_double2(fma(c, e.x, fma(se.x, a.x, -se.y * a.y)), fma(c, e.y, fma(se.x, a.y, se.y * a.x)));
+        }
+      }
     }
-    const double al = __shfl_sync(mask, d4[0], base), be = __shfl_sync(mask, d4[0], base + LP / 4);
-    const double gx = __shfl_sync(mask, d4[0], base + LP / 2), gy = __shfl_sync(mask, d4[0], base + 3 * LP / 4);
-    const double g2 = fma(gx, gx, gy * gy);
-    if (!(g2 > tol2 * (al * be))) continue;
-    if (hl == 0) *rot = 1;  // any rotation keeps the sweeps going
-    const double d = be - al;
-    const double h = rsqrt(fma(d, d, 4.0 * g2));
-    const double c2 = fma(0.5 * fabs(d), h, 0.5);
-    const double rc = rsqrt(c2);
-    const double c = c2 * rc, f = d < 0.0 ? -h * rc : h * rc;
-    const cplx se = make_double2(f * gx, f * gy);
-#pragma unroll 2
-    for (int r = hl; r < q; r += LP) {
-      const cplx x = bi[r], y = bj[r];
-      // b_i <- c b_i - conj(se) b_j,  b_j <- se b_i + c b_j
-      bi[r] = make_double2(fma(c, x.x, fma(-se.x, y.x, -se.y * y.y)), fma(c, x.y, fma(-se.x, y.y, se.y * y.x)));
-      bj[r] = make_double2(fma(c, y.x, fma(se.x, x.x, -se.y * x.y)), fma(c, y.y, fma(se.x, x.y, se.y * x.x)));
-    }
+    cta_sync();
   }
-  cta_sync();
 }
 
-// One round of a sweep in the form the run takes; a pair gets 16 lanes where
-// the round's pairs leave that many, else 8.
-template <class PairFn>
-static __device__ __forceinline__ void rotate_round(cplx* sb, int ld, int q, int npairs, PairFn pairs, double tol,
-                                                    LinalgSmem& ls, bool blocked) {
-  if (!blocked)
-    smem_rotate_round(sb, ld, q, q, npairs, pairs, tol, &ls.rot_count);
-  else if (npairs * 16 <= NT)
-    smem_rotate_short<16>(sb, ld, q, npairs, pairs, tol * tol, &ls.rot_count);
+// A pair gets 16 lanes where a round's pairs leave that many, else 8, and at
+// least as many as hold its rows in registers; q <= 256 (SVD_MAX_COLS).
+template <int LP>
+static __device__ __forceinline__ void jacobi_block_lp(cplx* cols, int ld, int q, bool cross, int b, int n0, int n1,
+                                                       int joff, double tol2, int* rot) {
+  if (q <= LP)
+    jacobi_rounds<LP, 1>(cols, ld, q, cross, b, n0, n1, joff, tol2, rot);
+  else if (q <= 2 * LP)
+    jacobi_rounds<LP, 2>(cols, ld, q, cross, b, n0, n1, joff, tol2, rot);
+  else if (q <= 4 * LP)
+    jacobi_rounds<LP, 4>(cols, ld, q, cross, b, n0, n1, joff, tol2, rot);
   else
-    smem_rotate_short<8>(sb, ld, q, npairs, pairs, tol * tol, &ls.rot_count);
+    jacobi_rounds<LP, 8>(cols, ld, q, cross, b, n0, n1, joff, tol2, rot);
+}
+static __device__ __forceinline__ void jacobi_block(cplx* cols, int ld, int q, bool cross, int b, int n0, int n1,
+                                                    int joff, double tol, int* rot) {
+  const int npairs = cross ? b : (b + 1) / 2;
+  if (q > 128)  // up to 256 rows
+    jacobi_rounds<32, 8>(cols, ld, q, cross, b, n0, n1, joff, tol * tol, rot);
+  else if (npairs * 16 <= NT || q > 64)
+    jacobi_block_lp<16>(cols, ld, q, cross, b, n0, n1, joff, tol * tol, rot);
+  else
+    jacobi_block_lp<8>(cols, ld, q, cross, b, n0, n1, joff, tol * tol, rot);
 }
 
 // Stage columns [c0, c0+nc0) and [c1, c1+nc1) of B into sb (ld = q), or
@@ -823,8 +898,10 @@ static __device__ __noinline__ SvdResult dev_svd(const cplx* M, int m, int n, in
     cta_sync();
     if (panel)
       dev_qr_factor_panel(H, mm, nn, sb, ls, rs);
+    else if (h_shared)
+      dev_qr_factor_at<true>(H, mm, nn, ls, rs);
     else
-      dev_qr_factor(H, mm, nn, ls, rs);
+      dev_qr_factor_at<false>(H, mm, nn, ls, rs);
   }
   // B = R^H (nn x k): B[r, c] = conj(R[c, r]) for c <= r
   cplx* B0 = both ? sb : w.B;
@@ -851,8 +928,9 @@ static __device__ __noinline__ SvdResult dev_svd(const cplx* M, int m, int n, in
       const int c0 = I * b, nc = min(b, p - c0);
       if (!resident) svd_stage(sb, ld, w, q, c0, nc, 0, 0, false);
       cplx* cols = resident ? sb + ld * c0 : sb;
-      for (int round = 0; round < be2 - 1; ++round) {
-        rotate_round(cols, ld, q, be2 / 2,
+      if (blocked) jacobi_block(cols, ld, q, false, b, nc, 0, 0, tol, &ls.rot_count);
+      for (int round = 0; !blocked && round < be2 - 1; ++round) {
+        smem_rotate_round(cols, ld, q, q, be2 / 2,
                      [&](int pr, int& i, int& j) {
                        // round-robin: place t holds column ((t - 1 - round) mod (be2 - 1)) + 1, place 0 column 0
                        const int ta = pr, tb = be2 - 1 - pr;
@@ -863,7 +941,7 @@ static __device__ __noinline__ SvdResult dev_svd(const cplx* M, int m, int n, in
                        j = max(a, c);
                        if (j >= nc) i = j = -1;
                      },
-                     tol, ls, blocked);
+                     tol, &ls.rot_count);
       }
       if (!resident) svd_stage(sb, ld, w, q, c0, nc, 0, 0, true);
     }
@@ -878,8 +956,9 @@ static __device__ __noinline__ SvdResult dev_svd(const cplx* M, int m, int n, in
         if (!resident) svd_stage(sb, ld, w, q, c0, n0, c1, n1, false);
         cplx* cols = resident ? sb + ld * c0 : sb;
         const int joff = resident ? c1 - c0 : n0;
-        for (int t = 0; t < b; ++t) {
-          rotate_round(cols, ld, q, b,
+        if (blocked) jacobi_block(cols, ld, q, true, b, n0, n1, joff, tol, &ls.rot_count);
+        for (int t = 0; !blocked && t < b; ++t) {
+          smem_rotate_round(cols, ld, q, q, b,
                        [&](int kk, int& i, int& j) {
                          const int jj = kk + t < b ? kk + t : kk + t - b;
                          if (kk >= n0 || jj >= n1) {
@@ -889,7 +968,7 @@ static __device__ __noinline__ SvdResult dev_svd(const cplx* M, int m, int n, in
                            j = joff + jj;
                          }
                        },
-                       tol, ls, blocked);
+                       tol, &ls.rot_count);
         }
         if (!resident) svd_stage(sb, ld, w, q, c0, n0, c1, n1, true);
       }
