@@ -1861,7 +1861,7 @@ int digital_begin(yaqs_ctx* ctx, const yaqs_mps_desc* psi0, const yaqs_gate_desc
             for (int k = 0; k < 2; ++k) v += std::conj(cload(q.matrix, k + 2 * i)) * cload(q.matrix, k + 2 * j);
             dev = std::max(dev, std::abs(v));
           }
-        if (!(dev < 1e-12)) P.canonical = 0;
+        if (!(dev < 1e-14)) P.canonical = 0;
       }
       if (by_tdvp(q)) {
         // construct_window_mpo (DigitalTJM.jl:192-236): coeff g(s1) on the
