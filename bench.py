@@ -58,14 +58,14 @@ sys.path.insert(0, ROOT)
 from yaqs_julia_b200 import _abi as A  # noqa: E402
 from yaqs_julia_b200 import api  # noqa: E402
 
-# the same for the digital workload: (L, trajectories, timed layers) -> bytes
-DIG_TIMED_TRAFFIC = {(40, 512, 57): 4.458638080e9 + 15.767363584e9}
+# the same for the digital workload: (L, trajectories, timed layers) -> bytes;
+# empty: no capture of the current kernels
+DIG_TIMED_TRAFFIC = {}
 
 METRIC = "TJM trajectory-steps/s (L=30 Heisenberg, chi=64, 1024 trajectories) vs plain FP64 GPU"
 # DRAM read + write bytes per trajectory-step of the trajectory kernel, from
 # one small-case ncu capture per configuration: (precision, tdvp, L, chi) -> bytes
-TRAFFIC_PER_TRAJ_STEP = {("mixed", "dynamic", 30, 64): 276.942e9 / 148 + 189.476e9 / 148,
-                         ("fp64", "dynamic", 30, 64): 438.298e9 / 148 + 252.204e9 / 148}
+TRAFFIC_PER_TRAJ_STEP = {}  # no capture of the current kernels
 TDVP_NAMES = {"dynamic": A.YAQS_TDVP_DYNAMIC, "2site": A.YAQS_TDVP_2SITE, "1site": A.YAQS_TDVP_1SITE}
 TDVP = [A.YAQS_TDVP_DYNAMIC]  # set from --tdvp
 TDVP_DESC = {"dynamic": "1-site TDVP with 2-site growth (local dynamic TDVP)", "2site": "2-site TDVP",

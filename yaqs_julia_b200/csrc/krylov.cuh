@@ -640,8 +640,9 @@ static __device__ __forceinline__ bool small_plan(const HeffOp& h, SmallPlan& p)
   return cap > off && p.nfit >= SMALL_MIN_VECS;
 }
 
-// C(M x N) = A B on 8 x 8 blocks dealt to the warps: fa(row, k) and fb(k, col)
-// give the operands inside the matrix, C (m,n) at C[m + n M].
+// C(M x N) = A B on 8 x 8 blocks dealt to the warps, C (m,n) at C[m + n M].
+// fa(row, k) starts a row's walk at k; its () gives the value there and then
+// moves on by four.  fb(k, col) gives B inside the matrix.
 template <class FA, class FB>
 static __device__ __forceinline__ void small_gemm(int M, int N, int K, FA fa, FB fb, cplx* C) {
   const int lane = ltid() & 31, wid = ltid() >> 5;
@@ -651,12 +652,12 @@ static __device__ __forceinline__ void small_gemm(int M, int N, int K, FA fa, FB
   for (int q = wid; q < mb * nb; q += NW) {
     const int nq = q / mb, row = (q - nq * mb) * 8 + gq, n0 = nq * 8;
     const bool rm = row < M, rn = n0 + gq < N;
-    auto arow = fa(row);
+    auto arow = fa(row, tq);
     double cr[2] = {0.0, 0.0}, ci[2] = {0.0, 0.0};
 #pragma unroll 1
     for (int k = tq; k - tq < K; k += 4) {
       cplx a = make_double2(0.0, 0.0), b = make_double2(0.0, 0.0);
-      if (rm && k < K) a = arow(k);
+      if (rm && k < K) a = arow();
       if (rn && k < K) b = fb(k, n0 + gq);
       dmma884(cr[0], cr[1], a.x, b.x);
       dmma884(ci[0], ci[1], a.x, b.y);
@@ -680,7 +681,15 @@ static __device__ __forceinline__ void small_heff(const HeffOp& h, const SmallPl
   const int chil = h.chil, D = h.D, chir = h.chir, wl = h.wl, wr = h.wr;
   cplx* T1 = buf + p.oT1;
   const int ml = chil * wl;
-  small_gemm(ml, D * chir, chil, [&](int row) { return [=](int k) { return buf[row + k * ml]; }; },
+  small_gemm(ml, D * chir, chil,
+             [&](int row, int k) {
+               const cplx* at = buf + row + k * ml;
+               return [=]() mutable {
+                 const cplx v = *at;
+                 at += 4 * ml;
+                 return v;
+               };
+             },
              [&](int k, int n) { return x[k + n * chil]; }, T1);
   cta_sync();
   const cplx* R = buf + p.oR;
@@ -689,16 +698,23 @@ static __device__ __forceinline__ void small_heff(const HeffOp& h, const SmallPl
   const int* col = rowp + h.W.no + 1;
   const bool ident = h.W.ident != 0;
   small_gemm(chil * D, chir, wr * chir,
-             [&](int row) {
+             [&](int row, int k) {
+               // T2[a, p', m', c] = sum W[(p', m'), (m, p)] T1[a, m, p, c], k = m' + wr c;
+               // ident: T2[a, k] = T1[a + chil k]
                const int pp = row / chil, a = row - pp * chil;
-               return [=](int k) {
-                 if (ident) return T1[a + k * chil];
-                 // T2[a, p', m', c] = sum W[(p', m'), (m, p)] T1[a, m, p, c], k = m' + wr c
-                 const int c = k / wr, o = pp + D * (k - c * wr);
-                 const cplx* in = T1 + a + c * ml * D;
+               int c = k / wr, mp = k - c * wr;
+               const cplx* in = T1 + a + (ident ? k * chil : c * ml * D);
+               return [=]() mutable {
+                 if (ident) {
+                   const cplx v = *in;
+                   in += 4 * chil;
+                   return v;
+                 }
+                 const int o = pp + D * mp;
                  cplx acc = make_double2(0.0, 0.0);
 #pragma unroll 1
                  for (int z = rowp[o]; z < rowp[o + 1]; ++z) wfma(acc, val[z], in[col[z] * chil]);
+                 for (mp += 4; mp >= wr; mp -= wr) in += ml * D;
                  return acc;
                };
              },
