@@ -765,8 +765,8 @@ def run_ours(args):
                     "frac": achieved / tc_peak,
                     "peak_source": f"half the {peaks['source']} dense bf16 rate (MEASURED_PEAKS.json): the rate of "
                                    "the tcgen05 kind::tf32 MMAs the mixed products issue",
-                    "achieved_counts": "H_eff product flops only, 8 per complex MAC (the tensor pipe executes 9 "
-                                       "TF32 MMAs per 4 real MACs: 3-product complex form x 3xTF32 split)"}
+                    "achieved_counts": "H_eff product flops only, 8 per complex MAC (the tensor pipe executes 12 "
+                                       "TF32 MMAs per complex product: four real ones x 3xTF32 split)"}
         else:
             roof = {"bound": "tensor", "achieved": achieved, "peak": pk.value, "unit": "TFLOP/s",
                     "frac": achieved / pk.value if pk.value else None,
