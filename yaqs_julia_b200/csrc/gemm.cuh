@@ -18,10 +18,6 @@
 // wn + NW/2 j), so a tile that is only partly inside the matrix still spreads
 // over all warps; blocks outside it issue no MMA and stage no data.
 // Conjugation is applied when a slice is read from shared memory.
-//
-// A product may be a sum over segments, C = sum_s coef_s A_s B_s, that share
-// one output tile in registers (the effective Hamiltonian in krylov.cuh): the
-// K slices of all segments form one stream through the ring.
 #pragma once
 #include "common.cuh"
 
@@ -96,44 +92,36 @@ static __device__ __forceinline__ void dmma884(double& d0, double& d1, double a,
                : "d"(a), "d"(b));
 }
 
-// One segment of a product: A (m,k) at A[m am + k ak], B (k,n) at
-// B[k bk + n bn], the product scaled by the provider's coef(s) unless unit(s).
-struct GemmSeg {
-  const cplx* A;
-  const cplx* B;
-  int am, ak, bk, bn;  // element offsets inside one operand stay far below 2^31
-  int K;
-};
-
 static __device__ __forceinline__ double flip_sign(double x, unsigned mask) {
   return __hiloint2double(__double2hiint(x) ^ (int)mask, __double2loint(x));
 }
 
-// C(M x N) = sum over the provider's segments; pv.nseg segments, pv.get(s, seg)
-// fills segment s, epi(mm, nn, value) stores one element.  CTA-collective;
-// ends with a cta_sync() so C is visible to all.
+// CTA-collective; ends with a cta_sync() so C is visible to all.
 //
 // Complex products run on the FP64 tensor cores (mma.sync m8n8k4): an 8 x 8
 // block accumulates re and im with four real MMAs per four k.  Bound: the
 // FP64 pipe, 64 FMA per clock and SM (0.23 TFLOP/s of an SM's share); a block
 // step of four MMAs takes 16 clocks of it and 8 of shared memory.  Against the
 // two-stage 16-deep slices with two barriers each, which multiplied whole
-// 64 x 64 tiles of mostly padding for small operands, the analog run on L = 30,
-// chi 64, FP64 (260 trajectories, 2 time indices) went from 1588 to 1453 ms,
-// L = 16 at chi 128 from 600 to 550 ms and L = 6 at chi 16 from 528 to 446 ms,
-// with the same bits.
-template <int GBK, class Prov, class Epi>
-static __device__ __forceinline__ void gemm_core(const Prov& pv, int M, int N, bool conjA, bool conjB, Epi epi,
-                                                 GemmSmem& sm) {
+// 64 x 64 tiles of mostly padding for small operands, L = 16 at chi 128 went
+// from 600 to 550 ms and L = 6 at chi 16 from 528 to 446 ms, with the same
+// bits.
+template <int GBK>
+static __device__ __noinline__ void cta_gemm_k(const GemmArgs g, GemmSmem& sm) {
+  ProfScope prof_scope_(PF_GEMM);
   constexpr int GSTAGES = GROWS / GBK;
   ASSUME_SHARED(&sm);
   const int tid = ltid();
   const int lane = tid & 31, wid = tid >> 5;
   const int wm = wid & 1, wn = wid >> 1;  // 2 x NW/2 warps
   const int gq = lane >> 2, tq = lane & 3;
-  const unsigned sgA = conjA ? 0x80000000u : 0u, sgB = conjB ? 0x80000000u : 0u;
-  int nslice = 0;
-  for (int s = 0; s < pv.nseg; ++s) nslice += (pv.K(s) + GBK - 1) / GBK;
+  const unsigned sgA = g.conjA ? 0x80000000u : 0u, sgB = g.conjB ? 0x80000000u : 0u;
+  const bool a_m_fast = (g.am == 1) || (g.ak != 1);
+  const bool b_n_fast = (g.bn == 1) || (g.bk != 1);
+  // element offsets inside one operand stay far below 2^31
+  const int am = (int)g.am, ak = (int)g.ak, bk = (int)g.bk, bn = (int)g.bn;
+  const int M = g.M, N = g.N, K = g.K;
+  const int nslice = (K + GBK - 1) / GBK;
   for (int tm = 0; tm < M; tm += GBM) {
     for (int tn = 0; tn < N; tn += GBN_EFF) {
       const int mrem = min(GBM, M - tm), nrem = min(GBN_EFF, N - tn);
@@ -146,54 +134,41 @@ static __device__ __forceinline__ void gemm_core(const Prov& pv, int M, int N, b
           cr[i][j][0] = cr[i][j][1] = 0.0;
           ci[i][j][0] = ci[i][j][1] = 0.0;
         }
-      GemmSeg o;
-      int is = 0, ik = 0;  // segment and k of the next slice to stage
-      pv.get(0, o);
-      auto issue = [&](int buf) {
-        if (is < pv.nseg) {
-          const bool a_m_fast = (o.am == 1) || (o.ak != 1);
-          const bool b_n_fast = (o.bn == 1) || (o.bk != 1);
+      auto issue = [&](int t, int buf) {  // slice t into stage buf; empty past the end
+        const int k0 = t * GBK;
+        if (t < nslice) {
 #pragma unroll
           for (int e = 0; e < GBM * GBK / NT; ++e) {
             const int idx = tid + NT * e;
             const int mi = a_m_fast ? (idx & (GBM - 1)) : (idx / GBK);
             const int ki = a_m_fast ? (idx / GBM) : (idx & (GBK - 1));
-            const int ka = ik + ki;
-            const bool va = mi < mrem && ka < o.K;
-            if (mi < mlim)
-              cp_async16(&sm.As[buf * GBK + ki][mi], o.A + (va ? (tm + mi) * o.am + ka * o.ak : 0), va);
+            const int ka = k0 + ki;
+            const bool va = mi < mrem && ka < K;
+            if (mi < mlim) cp_async16(&sm.As[buf * GBK + ki][mi], g.A + (va ? (tm + mi) * am + ka * ak : 0), va);
           }
 #pragma unroll
           for (int e = 0; e < GBN_EFF * GBK / NT; ++e) {
             const int idx = tid + NT * e;
             const int ni = b_n_fast ? (idx & (GBN_EFF - 1)) : (idx / GBK);
             const int kj = b_n_fast ? (idx / GBN_EFF) : (idx & (GBK - 1));
-            const int kb = ik + kj;
-            const bool vb = ni < nrem && kb < o.K;
-            if (ni < nlim)
-              cp_async16(&sm.Bs[buf * GBK + kj][ni], o.B + (vb ? kb * o.bk + (tn + ni) * o.bn : 0), vb);
-          }
-          ik += GBK;
-          if (ik >= o.K) {
-            ik = 0;
-            if (++is < pv.nseg) pv.get(is, o);
+            const int kb = k0 + kj;
+            const bool vb = ni < nrem && kb < K;
+            if (ni < nlim) cp_async16(&sm.Bs[buf * GBK + kj][ni], g.B + (vb ? kb * bk + (tn + ni) * bn : 0), vb);
           }
         }
         cp_async_commit();
       };
       cta_sync();  // the ring's last readers (the tile before) are done
 #pragma unroll 1
-      for (int p = 0; p < GSTAGES - 1; ++p) issue(p);
-      int cs = 0, ck = 0, cK = pv.K(0);
+      for (int p = 0; p < GSTAGES - 1; ++p) issue(p, p);
       for (int t = 0; t < nslice; ++t) {
         cp_async_wait<GSTAGES - 2>();  // slice t has landed (this thread's part)
-        cta_sync();            // everybody's part; slice t - 1 is consumed
-        issue((t + GSTAGES - 1) % GSTAGES);
+        cta_sync();                    // everybody's part; slice t - 1 is consumed
+        issue(t + GSTAGES - 1, (t + GSTAGES - 1) % GSTAGES);
         const int buf = t % GSTAGES;
-        const bool unit = pv.unit(cs);
 #pragma unroll
         for (int k4 = 0; k4 < GBK; k4 += 4) {
-          if (ck + k4 >= cK) break;
+          if (t * GBK + k4 >= K) break;
           double ar[4], ai[4], br[2], bi[2];
 #pragma unroll
           for (int j = 0; j < 2; ++j) {
@@ -202,12 +177,6 @@ static __device__ __forceinline__ void gemm_core(const Prov& pv, int M, int N, b
               const cplx b = sm.Bs[buf * GBK + k4 + tq][n0 + gq];
               br[j] = b.x;
               bi[j] = flip_sign(b.y, sgB);
-              if (!unit) {
-                const cplx f = pv.coef(cs);
-                const double x = br[j], y = bi[j];
-                br[j] = f.x * x - f.y * y;
-                bi[j] = f.x * y + f.y * x;
-              }
             }
           }
 #pragma unroll
@@ -238,11 +207,6 @@ static __device__ __forceinline__ void gemm_core(const Prov& pv, int M, int N, b
             }
           }
         }
-        ck += GBK;
-        if (ck >= cK) {
-          ck = 0;
-          if (++cs < pv.nseg) cK = pv.K(cs);
-        }
       }
 #pragma unroll
       for (int i = 0; i < 4; ++i) {
@@ -253,43 +217,16 @@ static __device__ __forceinline__ void gemm_core(const Prov& pv, int M, int N, b
 #pragma unroll
           for (int h = 0; h < 2; ++h) {
             const int nn = tn + (wn + (NW / 2) * j) * 8 + 2 * tq + h;
-            if (nn < N) epi(mm, nn, make_double2(cr[i][j][h], ci[i][j][h]));
+            if (nn >= N) continue;
+            cplx* c = g.C + (mm * (int)g.cm + nn * (int)g.cn);
+            cplx v = make_double2(cr[i][j][h], ci[i][j][h]);
+            if (g.accumulate) v = cadd(v, *c);
+            *c = v;
           }
       }
     }
   }
   cta_sync();
-}
-
-// The plain product: one segment.
-struct OneSeg {
-  const GemmArgs& g;
-  int nseg;
-  __device__ __forceinline__ int K(int) const { return g.K; }
-  __device__ __forceinline__ bool unit(int) const { return true; }
-  __device__ __forceinline__ cplx coef(int) const { return make_double2(1.0, 0.0); }
-  __device__ __forceinline__ void get(int, GemmSeg& o) const {
-    o.A = g.A;
-    o.B = g.B;
-    o.am = (int)g.am;
-    o.ak = (int)g.ak;
-    o.bk = (int)g.bk;
-    o.bn = (int)g.bn;
-    o.K = g.K;
-  }
-};
-
-template <int GBK>
-static __device__ __noinline__ void cta_gemm_k(const GemmArgs g, GemmSmem& sm) {
-  ProfScope prof_scope_(PF_GEMM);
-  const OneSeg pv{g, 1};
-  gemm_core<GBK>(pv, g.M, g.N, g.conjA, g.conjB,
-                 [&](int mm, int nn, cplx v) {
-                   cplx* c = g.C + (mm * (int)g.cm + nn * (int)g.cn);
-                   if (g.accumulate) v = cadd(v, *c);
-                   *c = v;
-                 },
-                 sm);
 }
 
 // A product of a few 8 x 8 blocks and a short sum, straight from global memory:

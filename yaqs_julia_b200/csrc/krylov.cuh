@@ -26,18 +26,12 @@
 // running-sum form gives them next to isometric sites.  With those blocks
 // taken out the product is, per output physical index p',
 //   y_{p'} = sum_s coef_s A_s B_s + sum_p loc[p', p] x_p
-// over segments L_m x_p (side 0, the term ends on the left), x_p R_m' (side
-// 1, it starts there) and (L_m x)_p R_m' (side 2, it passes through; the
-// products T1 = L_m x for m in [t1m, t1m + nt1) are formed first).
-#define HEFF_MAX_SEGS 64
-struct HSeg {
-  int side, m, p;  // p: physical index of the source
-  int g;           // side 2: row block of T1
-  cplx coef;
-};
-// The same terms by environment block for the tensor-core product (tsgemm.cuh):
-// block b multiplies channel m[b] with, per output index p', coef * (slice
-// src of x, or of row block t1 of T1 where t1 >= 0); src < 0: no term.
+// over terms L_m x_p (the term ends on the left), x_p R_m' (it starts there)
+// and (L_m x)_p R_m' (it passes through; the products T1 = L_m x for m in
+// [t1m, t1m + nt1) are formed first).  The mixed form takes it (tsgemm.cuh),
+// with the terms gathered by environment block: block b multiplies channel
+// m[b] with, per output index p', coef * (slice src of x, or of row block t1
+// of T1 where t1 >= 0); src < 0: no term.
 #define TS_MAX_BLOCKS 8
 struct TsSide {
   int nb;
@@ -46,13 +40,11 @@ struct TsSide {
   float2 coef[TS_MAX_BLOCKS][4];
 };
 struct HPlan {
-  int ts_ok;  // one term at most per block and p', at least one block on each side
   TsSide left, right;
   int il, ir;  // channels that have to be the identity
-  int t1m, nt1, nseg, has_loc;
-  int off[5];     // segments of p' are off[p'] .. off[p' + 1] - 1
-  cplx loc[16];   // [p' + D p]
-  const HSeg* seg;
+  int t1m, nt1, has_loc;
+  int nleft, nright;  // terms on each side
+  cplx loc[16];       // [p' + D p]
 };
 
 // Sparse MPO matrix M[o, i] in CSR form (rows are outputs).
@@ -157,7 +149,7 @@ static __device__ __noinline__ void dev_wapply(const T* in, T* out, const WMat W
 
 struct HeffOp {
   int blocked = 0;  // the run may reorder sums
-  const HPlan* plan = nullptr;  // set when both identity channels were found in the environments
+  const HPlan* plan = nullptr;  // mixed form: set when both identity channels were found in the environments
   const cplx* L;  // (chil, wl, chil)
   const cplx* R;  // (chir, wr, chir)
   WMat W;         // rows p'+D m', cols m + wl p
@@ -211,8 +203,6 @@ struct EngineSmem {
 #if YAQS_TC
   TsSide ts[2];  // left and right blocks of the solve's plan
   cplx loc[16];  // and its local term
-#else
-  HSeg hseg[HEFF_MAX_SEGS];  // segments of the solve's plan
 #endif
   EngineSmemU u;
 };
@@ -283,69 +273,6 @@ static __device__ void dev_heff_tc(const HeffOp& h, const cplx* x, cplx* y, Engi
 }
 #endif
 
-#if !YAQS_TC
-// One output block of the structured product as a segmented GEMM.
-struct HeffProv {
-  const HeffOp& h;
-  const HSeg* seg;
-  const cplx* x;
-  int nseg;
-  __device__ __forceinline__ int K(int s) const { return seg[s].side == 0 ? h.chil : h.chir; }
-  __device__ __forceinline__ bool unit(int s) const { return seg[s].coef.x == 1.0 && seg[s].coef.y == 0.0; }
-  __device__ __forceinline__ cplx coef(int s) const { return seg[s].coef; }
-  __device__ __forceinline__ void get(int s, GemmSeg& o) const {
-    const HSeg& q = seg[s];
-    o.am = 1;
-    if (q.side == 0) {
-      o.A = h.L + h.chil * q.m;
-      o.ak = h.chil * h.wl;
-      o.B = x + h.chil * q.p;
-      o.bk = 1;
-      o.bn = h.chil * h.D;
-      o.K = h.chil;
-    } else {
-      const int ld = q.side == 1 ? h.chil : h.chil * h.plan->nt1;
-      o.A = q.side == 1 ? x + h.chil * q.p : h.T1 + h.chil * q.g + ld * q.p;
-      o.ak = ld * h.D;
-      o.B = h.R + h.chir * q.m;
-      o.bk = h.chir * h.wr;
-      o.bn = 1;
-      o.K = h.chir;
-    }
-  }
-};
-
-// y = H_eff x by the plan of h (its segments in sm.hseg).  A Heisenberg site
-// multiplies 8 blocks of chi^3 instead of 10 and neither stores nor maps the
-// (w chi) x (D chi) intermediates: the K slices of all segments run through
-// one ring into one accumulator tile.
-static __device__ __noinline__ void heff_block(const HeffOp& h, const cplx* x, int pp, cplx* y, EngineSmem& sm) {
-  ProfScope prof_scope_(PF_GEMM);
-  const HPlan& pl = *h.plan;
-  const HeffProv pv{h, sm.hseg + pl.off[pp], x, pl.off[pp + 1] - pl.off[pp]};
-  const int ld = h.chil * h.D;
-  const bool loc = pl.has_loc != 0;
-  gemm_core<16>(pv, h.chil, h.chir, false, false,
-            [&](int mm, int nn, cplx v) {
-              const int e = mm + nn * ld;
-              if (loc)
-                for (int p = 0; p < h.D; ++p) cfma(v, pl.loc[pp + h.D * p], x[e + h.chil * p]);
-              y[e + h.chil * pp] = v;
-            },
-            sm.u.gw.g);
-}
-
-static __device__ __forceinline__ void heff_structured(const HeffOp& h, const cplx* x, cplx* y, EngineSmem& sm) {
-  const HPlan& pl = *h.plan;
-  if (pl.nt1 > 0)
-    cta_gemm(gemm_args(h.chil * pl.nt1, h.D * h.chir, h.chil, h.L + h.chil * pl.t1m, 1, h.chil * h.wl, x, 1, h.chil,
-                       h.T1, 1, h.chil * pl.nt1),
-             sm.u.gw.g);
-  for (int pp = 0; pp < h.D; ++pp) heff_block(h, x, pp, y, sm);
-}
-
-#endif
-
 // y = H_eff x.  CTA-collective.  In the mixed form x is rounded to FP32, the
 // three contractions run in FP32 (tensor cores for the two GEMMs) and y is
 // written back in FP64.
@@ -354,12 +281,6 @@ static __device__ __noinline__ void dev_heff(const HeffOp& h, const cplx* x, cpl
 #if YAQS_TC
   if (h.tc) {
     dev_heff_tc(h, x, y, sm);
-    return;
-  }
-#endif
-#if !YAQS_TC
-  if (h.plan && !h.mixed) {
-    heff_structured(h, x, y, sm);
     return;
   }
 #endif
@@ -422,11 +343,9 @@ static __device__ __forceinline__ double heff_flops(int chil, int wl, int D, int
 
 // Floating-point operations of one product in the form it takes.
 static __device__ __forceinline__ double heff_work(const HeffOp& h) {
-  if (!h.plan || (h.mixed && !h.tc)) return heff_flops(h.chil, h.wl, h.D, h.chir, h.wr);
+  if (!h.plan || !h.tc) return heff_flops(h.chil, h.wl, h.D, h.chir, h.wr);
   const double l = h.chil, r = h.chir;
-  double f = l * l * h.plan->nt1 * h.D * r;
-  for (int s = 0; s < h.plan->nseg; ++s) f += h.plan->seg[s].side == 0 ? l * l * r : l * r * r;
-  return 8.0 * f;
+  return 8.0 * (l * l * h.plan->nt1 * h.D * r + h.plan->nleft * l * l * r + h.plan->nright * l * r * r);
 }
 
 struct KrylovCfg {
@@ -608,9 +527,8 @@ static __device__ double lanczos_subtract(const cplx* Q, long long qs, cplx* w, 
 // in code that runs a few dozen times, a solve waits for instruction fetches
 // before it waits for anything else.
 // Every sum is formed in the general path's order (four-deep MMA steps from
-// k = 0, the same reduction trees), so both give the same bits: where a
-// 2-site sweep truncates between equal Schmidt values, rounding decides, and
-// a chain must not change its records by crossing this limit.
+// k = 0, the same reduction trees), so both give the same bits, which FP64
+// analog runs need (DevParams::blocked).
 // SMALL_N is one value per thread; wider solves fill the tiles of the general
 // path.  Measured with the sweep on L = 6 Ising, chi 16, 200 trajectories, 51
 // time indices: 445 ms with the general path alone, 180 ms with this one.

@@ -88,7 +88,7 @@ struct DevParams {
   // idx are the indices that belong to site i, ascending.
   const int *p0_off, *p0_idx, *p1_off, *p1_idx, *ob_off, *ob_idx;
   int canonical;   // recorded states are in mixed canonical form around their centre
-  int blocked;     // panel QR and short Jacobi rounds (LinalgSmem::blocked)
+  int blocked;     // may reorder sums (circuits, mixed): panel QR, short Jacobi rounds, predicted projections
   int scalar_all;  // every process is a scalar dissipator (pauli_name)
   int has_lr;      // some process is long-range
   const cplx* psi0;  // arena layout, compact tensors
@@ -505,23 +505,16 @@ static __device__ HeffOp make_heff(Ctx& c, int l, int D, int r, int bl, int br, 
   h.mixed = c.P.mixed;
   h.blocked = c.P.blocked;
   const bool tc = c.P.tc && !(c.P.tune && c.P.tune[tune_index(l, D, r)] == 1);
-  if (W.plan && c.sm.id_left[bl] == W.plan->il + 1 && c.sm.id_right[br] == W.plan->ir + 1) {
 #if YAQS_TC
-    if (tc && W.plan->ts_ok) {
-      h.plan = W.plan;
-      const int* src = reinterpret_cast<const int*>(&W.plan->left);
-      int* dst = reinterpret_cast<int*>(c.sm.e.ts);
-      for (int e = ltid(); e < (int)(2 * sizeof(TsSide) / sizeof(int)); e += NT) dst[e] = src[e];
-      if (ltid() < 16) c.sm.e.loc[ltid()] = W.plan->loc[ltid()];
-    }
-#else
-    if (!c.P.mixed) {
-      h.plan = W.plan;
-      for (int e = ltid(); e < W.plan->nseg; e += NT) c.sm.e.hseg[e] = W.plan->seg[e];
-    }
-#endif
+  if (tc && W.plan && c.sm.id_left[bl] == W.plan->il + 1 && c.sm.id_right[br] == W.plan->ir + 1) {
+    h.plan = W.plan;
+    const int* src = reinterpret_cast<const int*>(&W.plan->left);
+    int* dst = reinterpret_cast<int*>(c.sm.e.ts);
+    for (int e = ltid(); e < (int)(2 * sizeof(TsSide) / sizeof(int)); e += NT) dst[e] = src[e];
+    if (ltid() < 16) c.sm.e.loc[ltid()] = W.plan->loc[ltid()];
     cta_sync();
   }
+#endif
   h.T1f = reinterpret_cast<cflt*>(c.ws + c.P.lay.T1f);
   h.xf = reinterpret_cast<cflt*>(c.ws + c.P.lay.xf);
   SmallPlan sp;
