@@ -416,18 +416,30 @@ static __device__ __noinline__ void dev_tridiag_expm(int m, double dt, KrySmem& 
   if (on) ks.y[j] = v;
 }
 
-// v - c a, its roundings spelled out so that every path subtracts a basis
-// vector with the same bits.
+// The roundings of the sums that FP64 analog runs keep (DevParams::blocked),
+// spelled out: where a product meets a sum the compiler fuses one or the other
+// factor as the code around it falls, and the last bit follows.
+// v - c a
 static __device__ __forceinline__ cplx csub_mul(cplx v, cplx c, cplx a) {
   return make_double2(__dsub_rn(v.x, __fma_rn(c.x, a.x, -__dmul_rn(c.y, a.y))),
                       __dsub_rn(v.y, __fma_rn(c.y, a.x, __dmul_rn(c.x, a.y))));
 }
+// conj(a) b
+static __device__ __forceinline__ cplx cmulc_rn(cplx a, cplx b) {
+  return make_double2(__fma_rn(a.x, b.x, __dmul_rn(a.y, b.y)), __fma_rn(a.x, b.y, -__dmul_rn(a.y, b.x)));
+}
+// |a|^2
+static __device__ __forceinline__ double cabs2_rn(cplx a) { return __fma_rn(a.x, a.x, __dmul_rn(a.y, a.y)); }
 
 // h_j = <q_j, w> (j < k) into ks.h and |w|^2 in the same pass over w: the
 // first group takes seven vectors and the norm, later groups eight.  Each
 // thread takes two elements per iteration so that up to 18 independent
-// loads are in flight (the pass is bound by memory latency).
-static __device__ double lanczos_dots(const cplx* Q, long long qs, const cplx* w, long long n, int k, EngineSmem& sm) {
+// loads are in flight (the pass is bound by memory latency).  Out of line, like
+// basis_combine: inlined into the solver the loads of a group spill (L = 30,
+// chi 64: 1631 against 1513 ms; 2-site, L = 16, chi 64: 279 against 266).
+static __device__ __noinline__ double lanczos_dots(const cplx* Q, long long qs, const cplx* w, int n, int k,
+                                                   EngineSmem& sm) {
+  ASSUME_SHARED(&sm);
   const int tid = ltid();
   double nw2 = 0.0;
   for (int j0 = 0, first = 1; j0 < k || first; first = 0) {
@@ -435,23 +447,25 @@ static __device__ double lanczos_dots(const cplx* Q, long long qs, const cplx* w
     double d[16];
 #pragma unroll
     for (int e = 0; e < 16; ++e) d[e] = 0.0;
-    for (long long i0 = tid; i0 < n; i0 += 2 * NT) {
-      const long long i1 = i0 + NT;
-      const bool two = i1 < n;
+#pragma unroll 1
+    for (int i0 = tid; i0 < n; i0 += 2 * NT) {
+      const bool two = i0 + NT < n;
+      const int i1 = two ? i0 + NT : i0;
       const cplx w0 = w[i0];
       const cplx w1 = two ? w[i1] : make_double2(0.0, 0.0);
       cplx a0[8], a1[8];
 #pragma unroll
       for (int e = 0; e < 8; ++e) {
         const bool live = e < G && j0 + e < k;
-        a0[e] = live ? Q[qs * (j0 + e) + i0] : make_double2(0.0, 0.0);
-        a1[e] = (live && two) ? Q[qs * (j0 + e) + i1] : make_double2(0.0, 0.0);
+        const cplx* q = Q + qs * (j0 + e);
+        a0[e] = live ? q[i0] : make_double2(0.0, 0.0);
+        a1[e] = live ? q[i1] : make_double2(0.0, 0.0);
       }
-      if (first) d[15] += cabs2(w0) + cabs2(w1);
+      if (first) d[15] += cabs2_rn(w0) + __fma_rn(w1.y, w1.y, __dmul_rn(w1.x, w1.x));
 #pragma unroll
       for (int e = 0; e < 8; ++e) {
         if (e == 7 && first) continue;
-        const cplx p = cadd(cmulc(a0[e], w0), cmulc(a1[e], w1));
+        const cplx p = cadd(cmulc_rn(a0[e], w0), cmulc_rn(a1[e], w1));
         d[2 * e] += p.x;
         d[2 * e + 1] += p.y;
       }
@@ -465,52 +479,50 @@ static __device__ double lanczos_dots(const cplx* Q, long long qs, const cplx* w
   return nw2;
 }
 
-// out_i = s (w_i - sum_{j<k} c_j q_j[i]) for i < n (w null: w_i = 0; out may
-// be w), c in shared memory; returns the CTA sum of |out_i|^2 when norm.
+// out_i = s (w_i - sum_{j<k} h_j q_j[i]) for i < n (w null: w_i = 0; out may
+// be w), h in ks.h; returns the CTA sum of |out_i|^2 when norm.
 // Basis vectors go in groups of eight, two elements per thread, so the loads
 // of a group are in flight together.  CTA-collective.
-static __device__ double basis_combine(const cplx* Q, long long qs, const cplx* w, cplx* out, long long n, int k,
-                                       const cplx* c, double s, bool norm, EngineSmem& sm) {
+static __device__ __noinline__ double basis_combine(const cplx* Q, long long qs, const cplx* w, cplx* out, int n,
+                                                    int k, double s, bool norm, EngineSmem& sm) {
+  ASSUME_SHARED(&sm);
   double part = 0.0;
-  for (long long i0 = ltid(); i0 < n; i0 += 2 * NT) {
-    const long long i1 = i0 + NT;
-    const bool two = i1 < n;
+#pragma unroll 1
+  for (int i0 = ltid(); i0 < n; i0 += 2 * NT) {
+    const bool two = i0 + NT < n;
+    const int i1 = two ? i0 + NT : i0;
     cplx v0 = w ? w[i0] : make_double2(0.0, 0.0);
-    cplx v1 = (w && two) ? w[i1] : make_double2(0.0, 0.0);
+    cplx v1 = w ? w[i1] : make_double2(0.0, 0.0);
+#pragma unroll 1
     for (int j0 = 0; j0 < k; j0 += 8) {
       cplx a0[8], a1[8];
 #pragma unroll
       for (int e = 0; e < 8; ++e) {
         const bool live = j0 + e < k;
-        a0[e] = live ? Q[qs * (j0 + e) + i0] : make_double2(0.0, 0.0);
-        a1[e] = (live && two) ? Q[qs * (j0 + e) + i1] : make_double2(0.0, 0.0);
+        const cplx* q = Q + qs * (j0 + e);
+        a0[e] = live ? q[i0] : make_double2(0.0, 0.0);
+        a1[e] = live ? q[i1] : make_double2(0.0, 0.0);
       }
 #pragma unroll
       for (int e = 0; e < 8; ++e) {
         if (j0 + e < k) {
-          const cplx ce = c[j0 + e];
+          const cplx ce = sm.k.h[j0 + e];
           v0 = csub_mul(v0, ce, a0[e]);
           v1 = csub_mul(v1, ce, a1[e]);
         }
       }
     }
     v0 = cscale(v0, s);
-    v1 = cscale(v1, s);
+    v1 = two ? cscale(v1, s) : make_double2(0.0, 0.0);
     out[i0] = v0;
     if (two) out[i1] = v1;
-    part += cabs2(v0) + cabs2(v1);
+    part += cabs2_rn(v0) + cabs2_rn(v1);
   }
   if (!norm) {
     cta_sync();
     return 0.0;
   }
   return block_sum(part, sm.r);
-}
-
-// w <- w - sum_j h_j q_j (j < k); with norm, returns |w|^2 after the update.
-static __device__ double lanczos_subtract(const cplx* Q, long long qs, cplx* w, long long n, int k, EngineSmem& sm,
-                                          bool norm) {
-  return basis_combine(Q, qs, w, w, n, k, sm.k.h, 1.0, norm, sm);
 }
 
 // ---------------------------------------------------------------------------
@@ -660,11 +672,11 @@ static __device__ __noinline__ double small_dots(const cplx* sQ, int nfit, const
         if (i < n) {
           const cplx w0 = w[i];
           if (j < k) {
-            const cplx v = cmulc(q[i], w0);
+            const cplx v = cmulc_rn(q[i], w0);
             d[2 * u] = v.x;
             d[2 * u + 1] = v.y;
           } else {
-            d[2 * u] = cabs2(w0);
+            d[2 * u] = cabs2_rn(w0);
           }
         }
       }
@@ -714,7 +726,7 @@ static __device__ __noinline__ int dev_expm_small(const HeffOp& h, const SmallPl
       for (int j = 0; j < k; ++j) v = csub_mul(v, ks.h[j], j < nfit ? sQ[j * n + i] : Q[qs * j + i]);
       v = cscale(v, s);
       out[i] = v;
-      part += cabs2(v);
+      part += cabs2_rn(v);
     }
     return part;
   };
@@ -950,11 +962,11 @@ static __device__ __noinline__ int dev_expm_krylov(const HeffOp& h, cplx* x, dou
   if (small_plan(h, sp)) return dev_expm_small(h, sp, x, dt, kc, Q, qs, sm);
   if (h.blocked) return dev_expm_predicted(h, x, dt, kc, Q, qs, sm);
   const int tid = ltid();
-  const long long n = (long long)h.chil * h.D * h.chir;
+  const int n = h.chil * h.D * h.chir;
   const double beta0 = sqrt(cta_norm2(x, n, sm.r));
   if (beta0 == 0.0) return 0;
   const double tau = fabs(dt);
-  for (long long i = tid; i < n; i += NT) Q[i] = cscale(x[i], 1.0 / beta0);
+  for (int i = tid; i < n; i += NT) Q[i] = cscale(x[i], 1.0 / beta0);
   cta_sync();
   double bound = 1.0;
   int m = 0;
@@ -979,10 +991,10 @@ static __device__ __noinline__ int dev_expm_krylov(const HeffOp& h, cplx* x, dou
     if (accept) {
       b_k = sqrt(r2);
     } else {
-      lanczos_subtract(Q, qs, w, n, k, sm, false);
+      basis_combine(Q, qs, w, w, n, k, 1.0, false, sm);
       lanczos_dots(Q, qs, w, n, k, sm);
       a_k += sm.k.h[k - 1].x;
-      b_k = sqrt(lanczos_subtract(Q, qs, w, n, k, sm, true));
+      b_k = sqrt(basis_combine(Q, qs, w, w, n, k, 1.0, true, sm));
     }
     if (tid == 0) sm.k.alpha[k - 1] = a_k;
     m = k;
@@ -993,9 +1005,9 @@ static __device__ __noinline__ int dev_expm_krylov(const HeffOp& h, cplx* x, dou
     if (tid == 0) sm.k.beta[k - 1] = b_k;
     const double inv = 1.0 / b_k;
     if (accept) {
-      basis_combine(Q, qs, w, w, n, k, sm.k.h, inv, false, sm);
+      basis_combine(Q, qs, w, w, n, k, inv, false, sm);
     } else {
-      for (long long i = tid; i < n; i += NT) w[i] = cscale(w[i], inv);
+      for (int i = tid; i < n; i += NT) w[i] = cscale(w[i], inv);
       cta_sync();
     }
   }
@@ -1004,6 +1016,6 @@ static __device__ __noinline__ int dev_expm_krylov(const HeffOp& h, cplx* x, dou
   cta_sync();
   if (tid < m) sm.k.h[tid] = make_double2(-sm.k.y[tid].x, -sm.k.y[tid].y);  // x = beta0 sum_j y_j q_j
   cta_sync();
-  basis_combine(Q, qs, nullptr, x, n, m, sm.k.h, beta0, false, sm);
+  basis_combine(Q, qs, nullptr, x, n, m, beta0, false, sm);
   return mv;
 }
