@@ -5,6 +5,7 @@
 // broadcast through shared memory so control flow stays uniform.
 #pragma once
 #include <cuda_runtime.h>
+#include <math.h>
 #include <stdint.h>
 
 // Threads of one trajectory program: 256, or 128 in the small-program
@@ -92,6 +93,14 @@ static __device__ __forceinline__ void cfmac(cplx& c, cplx a, cplx b) {
   c.x = fma(a.y, b.y, c.x);
   c.y = fma(a.x, b.y, c.y);
   c.y = fma(-a.y, b.x, c.y);
+}
+
+// Deviation of one value from `diag` (1 on the diagonal, 0 off it) by its
+// larger part; infinite when either part is not a number, which fmax and a
+// comparison of the larger part alone would pass over.
+static __host__ __device__ __forceinline__ double identity_dev(cplx v, double diag) {
+  const double d = fabs(v.x - diag), e = fabs(v.y);
+  return d + e == d + e ? fmax(d, e) : INFINITY;
 }
 
 static __device__ __forceinline__ double warp_sum(double v) {

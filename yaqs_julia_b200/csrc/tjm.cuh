@@ -362,11 +362,8 @@ static __device__ __noinline__ void note_identity(Ctx& c, cplx* E, int dim, int 
   if (c.P.blocked && idc >= 0) {
     double dev = 0.0;
     for (int k = ltid() >> 5; k < dim; k += NW)
-      for (int a = ltid() & 31; a < dim; a += 32) {
-        const cplx v = E[a + dim * (idc + w * k)];
-        const double d = fmax(fabs(v.x - (a == k ? 1.0 : 0.0)), fabs(v.y));
-        dev = d > dev || d != d ? (d != d ? INFINITY : d) : dev;
-      }
+      for (int a = ltid() & 31; a < dim; a += 32)
+        dev = fmax(dev, identity_dev(E[a + dim * (idc + w * k)], a == k ? 1.0 : 0.0));
     found = block_max(dev, c.sm.e.r) <= (c.P.mixed ? 2e-5 : 1e-12);
     if (found)
       for (int k = ltid() >> 5; k < dim; k += NW)
