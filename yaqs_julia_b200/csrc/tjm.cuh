@@ -1295,6 +1295,27 @@ static __device__ __noinline__ bool local_by_envs(Ctx& c, const DState& s, int c
   return true;
 }
 
+// Largest deviation of the state from mixed canonical form around its centre:
+// of A^H A = 1 over the sites left of it and A A^H = 1 over those right of it.
+// CTA-collective.
+static __device__ __noinline__ double canonical_defect(Ctx& c, const DState& s) {
+  cplx* G = c.ws + c.P.lay.tA;
+  const int oc = *s.oc;
+  double dev = 0.0;
+  for (int i = 0; i < c.P.L; ++i) {
+    if (i == oc) continue;
+    const int l = s.chi[i], r = s.chi[i + 1], d = i < oc ? r : l;
+    const cplx* A = site_ptr(c, s, i);
+    if (i < oc)
+      cta_gemm(gemm_args(r, r, 2 * l, A, 2 * l, 1, A, 1, 2 * l, G, 1, r, true, false), c.sm.e.u.gw.g);
+    else
+      cta_gemm(gemm_args(l, l, 2 * r, A, 1, l, A, l, 1, G, 1, l, false, true), c.sm.e.u.gw.g);
+    for (int e = ltid(); e < d * d; e += NT) dev = fmax(dev, identity_dev(G[e], e / d == e % d ? 1.0 : 0.0));
+    cta_sync();
+  }
+  return block_max(dev, c.sm.e.r);
+}
+
 static __device__ __noinline__ void evaluate(Ctx& c, const DState& s, int col) {
   ProfScope prof_scope_(PF_EVAL);
   const int ncols = c.P.ncols;
