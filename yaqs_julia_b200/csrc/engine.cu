@@ -1535,6 +1535,9 @@ int yaqs_run_restore(yaqs_run* run, int32_t traj, const int32_t* chi, int32_t oc
                            cudaMemcpyHostToDevice));
   CUDA_TRY(ctx, cudaMemcpy(run->P.phi_oc + traj, &oc, sizeof(int32_t), cudaMemcpyHostToDevice));
   CUDA_TRY(ctx, cudaMemcpy(run->P.rng_pos + traj, &d, sizeof(long long), cudaMemcpyHostToDevice));
+  // a copy from pageable memory may return before it has landed, and the run's
+  // stream does not wait for the legacy one
+  CUDA_TRY(ctx, cudaStreamSynchronize(0));
   return YAQS_OK;
 }
 
@@ -1551,6 +1554,7 @@ int yaqs_run_seek(yaqs_run* run, int32_t position) {
   CUDA_TRY(ctx, cudaMemset(run->P.queue + position, 0, (size_t)(np - position) * sizeof(int)));
   std::vector<int> done(run->P.num_traj, position - 1);
   CUDA_TRY(ctx, cudaMemcpy(run->P.done, done.data(), done.size() * sizeof(int), cudaMemcpyHostToDevice));
+  CUDA_TRY(ctx, cudaStreamSynchronize(0));  // the run's stream does not wait for the legacy one
   run->next = position;
   return YAQS_OK;
 }
