@@ -236,9 +236,15 @@ int set_err(yaqs_ctx* ctx, int code, const std::string& msg) {
 struct DevMem {
   cudaMemPool_t pool = nullptr;  // the context's pool, null for cudaMalloc
   std::vector<void*> ptrs, pooled;
+  int device = 0;  // of the pooled blocks: their frees go to its legacy stream
   ~DevMem() {
     for (void* p : ptrs) cudaFree(p);
+    if (pooled.empty()) return;
+    int caller = 0;
+    cudaGetDevice(&caller);
+    if (caller != device) cudaSetDevice(device);
     for (void* p : pooled) cudaFreeAsync(p, 0);
+    if (caller != device) cudaSetDevice(caller);
   }
   template <class T>
   cudaError_t alloc(T** p, size_t count) {
@@ -246,6 +252,7 @@ struct DevMem {
     const size_t bytes = std::max<size_t>(count, 1) * sizeof(T);
     if (pool && bytes <= POOL_BLOCK_BYTES) {
       if (cudaMallocFromPoolAsync(&q, bytes, pool, 0) == cudaSuccess) {
+        cudaGetDevice(&device);
         pooled.push_back(q);
         *p = reinterpret_cast<T*>(q);
         return cudaSuccess;
@@ -824,7 +831,6 @@ struct yaqs_run {
   double* d_flops = nullptr;
   unsigned long long* d_prof = nullptr;
   ~yaqs_run() {
-    if (ctx) cudaSetDevice(ctx->device);  // pooled memory is freed on its device's stream
     if (d_prof) {
       unsigned long long* z = nullptr;
       cudaMemcpyToSymbol(g_prof, &z, sizeof(z));
