@@ -190,7 +190,14 @@ typedef struct {
 
 /* ---- context ---- */
 int yaqs_ctx_create(int32_t device, yaqs_ctx** out);
+/* Finish the runs and destroy the servers of a context before it. */
 int yaqs_ctx_destroy(yaqs_ctx* ctx);
+/*
+ * A context keeps freed device memory of its runs for the next one (blocks up
+ * to 768 MB, 1.75 GB in all), and so does a server; these give back what is
+ * held and not in use.  A run that does not fit gets it back by itself.
+ */
+void yaqs_ctx_trim(yaqs_ctx* ctx);
 const char* yaqs_last_error(const yaqs_ctx* ctx);
 const char* yaqs_version(void);
 
@@ -438,6 +445,7 @@ int yaqs_server_take(yaqs_server* srv, int64_t id, double* traj_out, double* mea
                      yaqs_run_stats* stats, double* times_s);
 const char* yaqs_server_last_error(yaqs_server* srv);
 int yaqs_server_stats_get(yaqs_server* srv, yaqs_server_stats* out);
+void yaqs_server_trim(yaqs_server* srv); /* see yaqs_ctx_trim */
 /* Fails whatever is still queued or running and frees the server. */
 int yaqs_server_destroy(yaqs_server* srv);
 

@@ -33,6 +33,8 @@ def lib():
         L.yaqs_last_error.argtypes = [C.c_void_p]
         L.yaqs_ctx_create.argtypes = [C.c_int32, P(C.c_void_p)]
         L.yaqs_ctx_destroy.argtypes = [C.c_void_p]
+        L.yaqs_ctx_trim.argtypes = [C.c_void_p]
+        L.yaqs_ctx_trim.restype = None
         L.yaqs_analog_run.argtypes = [C.c_void_p, P(A.MpsDesc), P(A.MpoDesc), P(A.NoiseDesc), P(A.ObsDesc),
                                       C.c_int32, P(A.TevConfig), P(A.RngDesc), A.DPTR, A.DPTR, P(C.c_int32),
                                       P(A.RunStats)]
@@ -70,6 +72,8 @@ def lib():
         L.yaqs_server_last_error.argtypes = [C.c_void_p]
         L.yaqs_server_last_error.restype = C.c_char_p
         L.yaqs_server_stats_get.argtypes = [C.c_void_p, P(A.ServerStats)]
+        L.yaqs_server_trim.argtypes = [C.c_void_p]
+        L.yaqs_server_trim.restype = None
         L.yaqs_server_destroy.argtypes = [C.c_void_p]
         L.yaqs_fp64_peak.argtypes = [C.c_void_p, P(C.c_double)]
         L.yaqs_autotune_results.argtypes = [C.c_void_p, A.DPTR, C.c_int32, P(C.c_int32)]
@@ -102,6 +106,10 @@ class Context:
     def check(self, st):
         if st != A.YAQS_OK:
             raise EngineError(st, self._lib.yaqs_last_error(self.handle).decode())
+
+    def trim(self):
+        """Give back the device memory held for the next run (yaqs_ctx_trim)."""
+        self._lib.yaqs_ctx_trim(self.handle)
 
     def close(self):
         if self.handle:

@@ -1335,6 +1335,10 @@ class Server:
         self._check_static(self._lib.yaqs_server_stats_get(self.handle, C.byref(s)))
         return s.as_dict()
 
+    def trim(self):
+        """Give back the device memory held for the next request (yaqs_server_trim)."""
+        self._lib.yaqs_server_trim(self.handle)
+
     def close(self):
         if getattr(self, "handle", None):
             self._lib.yaqs_server_destroy(self.handle)

@@ -206,6 +206,13 @@ cudaMemPool_t make_pool(int device) {
   return pool;
 }
 
+// Gives back what the pool holds without using it; frees under way land first.
+// The pool's device has to be current.
+cudaError_t trim_pool(cudaMemPool_t pool) {
+  const cudaError_t e = cudaStreamSynchronize(0);
+  return e == cudaSuccess ? cudaMemPoolTrimTo(pool, 0) : e;
+}
+
 // Bytes the pool holds without using them: as good as free to this context.
 size_t pool_idle(const yaqs_ctx* ctx) {
   unsigned long long held = 0, used = 0;
@@ -260,6 +267,11 @@ struct DevMem {
       cudaGetLastError();
     }
     cudaError_t e = cudaMalloc(&q, bytes);
+    if (e == cudaErrorMemoryAllocation && pool) {  // what the pool holds idle counted as free
+      cudaGetLastError();
+      trim_pool(pool);
+      e = cudaMalloc(&q, bytes);
+    }
     if (e == cudaSuccess) {
       ptrs.push_back(q);
       *p = reinterpret_cast<T*>(q);
@@ -1142,6 +1154,12 @@ int yaqs_ctx_create(int32_t device, yaqs_ctx** out) {
 int yaqs_ctx_destroy(yaqs_ctx* ctx) {
   delete ctx;
   return YAQS_OK;
+}
+
+void yaqs_ctx_trim(yaqs_ctx* ctx) {
+  if (!ctx || !ctx->pool) return;
+  std::lock_guard<std::mutex> lk(ctx->mu);
+  if (cudaSetDevice(ctx->device) != cudaSuccess || trim_pool(ctx->pool) != cudaSuccess) cudaGetLastError();
 }
 
 const char* yaqs_last_error(const yaqs_ctx* ctx) { return ctx ? ctx->err.c_str() : g_static_err.c_str(); }

@@ -548,6 +548,10 @@ int yaqs_server_stats_get(yaqs_server* srv, yaqs_server_stats* out) {
   return YAQS_OK;
 }
 
+void yaqs_server_trim(yaqs_server* srv) {
+  if (srv) yaqs_ctx_trim(&srv->ictx);
+}
+
 int yaqs_server_destroy(yaqs_server* srv) {
   if (!srv) return YAQS_OK;
   {
