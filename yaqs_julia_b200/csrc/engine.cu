@@ -1167,18 +1167,23 @@ const char* yaqs_last_error(const yaqs_ctx* ctx) { return ctx ? ctx->err.c_str()
 // Autotuner of the mixed H_eff products: per shape bucket (tune_index) the
 // tcgen05 form or the mma.sync form, whichever a launch over every slot of
 // the run applying H_eff to synthetic operands of that shape finishes first
-// (mma.sync only when it is more than 5 % faster).  Choices are measured
-// once per (device, chi_l, D, chi_r, w_l, w_r) and kept for the process, so
-// every run of a shape uses the same form and a run's results do not depend
-// on when it was tuned.  YAQS_AUTOTUNE=0 keeps tcgen05 everywhere.
+// (mma.sync only when it is more than 5 % faster).  Choices are measured once
+// per device, shape and what the tcgen05 form does there (the structured
+// product with its block counts where the MPO has a plan, the general one
+// elsewhere) and kept for the process, so every run of a kind uses the same
+// form and a run's results do not depend on what ran before it.  Solves that
+// run in shared memory take neither form; their entry is fixed.
+// YAQS_AUTOTUNE=0 keeps tcgen05 everywhere.
 struct TuneRecord {
   unsigned char form;
   float us_tc, us_mma;
 };
 static std::mutex g_tune_mu;
-static std::map<std::array<int, 6>, TuneRecord> g_tune_cache;
+static std::map<std::array<int, 10>, TuneRecord> g_tune_cache;
 
-static int autotune_products(yaqs_ctx* ctx, yaqs_run* run, const std::vector<int>& cap, const std::vector<int>& w) {
+// all: the run's maps in the order append_mpo_wmats and the bonds give them.
+static int autotune_products(yaqs_ctx* ctx, yaqs_run* run, const std::vector<int>& cap, const std::vector<int>& w,
+                             const std::vector<HostWMat>& all) {
   const char* env = getenv("YAQS_AUTOTUNE");
   if (env && env[0] == '0') return YAQS_OK;
   DevParams& P = run->P;
@@ -1202,7 +1207,13 @@ static int autotune_products(yaqs_ctx* ctx, yaqs_run* run, const std::vector<int
   std::lock_guard<std::mutex> lk(g_tune_mu);
   for (const auto& kv : buckets) {
     const Shape& sh = kv.second;
-    const std::array<int, 6> key{ctx->device, sh.l, sh.D, sh.r, w[sh.bl], w[sh.br]};
+    const HostWMat& W = sh.D == 1 ? all[4 * L - 1 + sh.bl] : sh.D == 2 ? all[sh.site] : all[L + sh.site];
+    const HPlan none{}, &pl = W.planned ? W.plan : none;
+    const std::array<int, 10> key{ctx->device, sh.l,           sh.D,   sh.r,       w[sh.bl],
+                                  w[sh.br],    (int)W.planned, pl.nt1, pl.left.nb, pl.right.nb};
+    SmallPlan sp;
+    const bool small =
+        small_layout(sh.l, sh.D, sh.r, w[sh.bl], w[sh.br], W.ident, W.no, (int)W.val.size(), sp);
     auto it = g_tune_cache.find(key);
     if (it == g_tune_cache.end()) {
       TuneRecord rec{0, 0.f, 0.f};
@@ -1210,7 +1221,7 @@ static int autotune_products(yaqs_ctx* ctx, yaqs_run* run, const std::vector<int
       CUDA_TRY(ctx, tc_tune_time(P, run->slots, d_mma, sh.bl, sh.br, sh.l, sh.D, sh.r, sh.site, 4, &rec.us_mma));
       rec.us_tc *= 250.f;  // ms for 4 products -> us per product
       rec.us_mma *= 250.f;
-      rec.form = rec.us_mma < 0.95f * rec.us_tc ? 1 : 0;
+      rec.form = !small && rec.us_mma < 0.95f * rec.us_tc ? 1 : 0;
       it = g_tune_cache.emplace(key, rec).first;
     }
     table[kv.first] = it->second.form;
@@ -1435,7 +1446,7 @@ static int analog_begin_impl(yaqs_ctx* ctx, const yaqs_mps_desc* psi0, const yaq
   P.wm_bond = d_views + L + (L - 1) + L + L;
 
   if (use_tc) {
-    st = autotune_products(ctx, run, cap, w);
+    st = autotune_products(ctx, run, cap, w, all);
     if (st != YAQS_OK) return st;
   }
   run->launches.push_back(0);

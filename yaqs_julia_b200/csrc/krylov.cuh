@@ -552,22 +552,26 @@ struct SmallPlan {
   int nfit;                     // Krylov vectors held in the buffer
 };
 
-static __device__ __forceinline__ bool small_plan(const HeffOp& h, SmallPlan& p) {
-  const int n = h.chil * h.D * h.chir;
+static __host__ __device__ __forceinline__ bool small_layout(int chil, int D, int chir, int wl, int wr, int ident,
+                                                             int no, int nnz, SmallPlan& p) {
+  const int n = chil * D * chir;
   if (n > SMALL_N) return false;
   const int cap = (int)(sizeof(EngineSmemU) / sizeof(cplx));
-  int off = h.chil * h.wl * h.chil;
+  int off = chil * wl * chil;
   p.oR = off;
-  off += h.chir * h.wr * h.chir;
+  off += chir * wr * chir;
   p.oT1 = off;
-  off += h.chil * h.wl * h.D * h.chir;
+  off += chil * wl * D * chir;
   p.oVal = off;
-  off += h.W.ident ? 0 : h.W.nnz;
+  off += ident ? 0 : nnz;
   p.oIdx = off;  // row pointers, then columns
-  off += h.W.ident ? 0 : (h.W.no + 1 + h.W.nnz + 3) / 4;
+  off += ident ? 0 : (no + 1 + nnz + 3) / 4;
   p.oQ = off;
   p.nfit = (cap - off) / n;
   return cap > off && p.nfit >= SMALL_MIN_VECS;
+}
+static __device__ __forceinline__ bool small_plan(const HeffOp& h, SmallPlan& p) {
+  return small_layout(h.chil, h.D, h.chir, h.wl, h.wr, h.W.ident, h.W.no, h.W.nnz, p);
 }
 
 // C(M x N) = A B on 8 x 8 blocks dealt to the warps, C (m,n) at C[m + n M].
