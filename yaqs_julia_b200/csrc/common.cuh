@@ -62,9 +62,13 @@ struct ProfScope {
 
 // Routines that are not inlined see shared memory through plain pointers and
 // would load it as generic memory, slower and on the global scoreboard; this
-// tells the compiler where a pointer points.  For routines whose pointer is
-// always shared; dev_svd, which picks between the staging buffer and global
-// memory, came out wrong with it and takes plain pointers.
+// tells the compiler where a pointer points.  Only for a pointer that is
+// always shared, in a routine that is not inlined and picks no address between
+// that memory and global memory: given the hint, dev_svd, which does, came out
+// wrong although the hint was true.  It and dev_expm_small leave the work on
+// shared memory alone to routines of their own (kept_rounds, jacobi_rounds,
+// small_heff).  The reductions below are inlined and hint their own scratch,
+// which no routine mixes with other memory.
 #define ASSUME_SHARED(p) __builtin_assume(__isShared((const void*)(p)))
 
 static __device__ __forceinline__ cplx cmk(double x, double y) { return make_double2(x, y); }

@@ -610,8 +610,9 @@ static __device__ __forceinline__ void small_gemm(int M, int N, int K, FA fa, FB
 // map is applied while the second product loads its left operand: every
 // value is loaded by one block column only (chir <= 8) or a few, and T2 and
 // its barriers go away.
-static __device__ __forceinline__ void small_heff(const HeffOp& h, const SmallPlan& p, cplx* buf, const cplx* x,
-                                                  cplx* w) {
+static __device__ __noinline__ void small_heff(const HeffOp& h, const SmallPlan& p, cplx* buf, const cplx* x,
+                                               cplx* w) {
+  ASSUME_SHARED(buf);
   const int chil = h.chil, D = h.D, chir = h.chir, wl = h.wl, wr = h.wr;
   cplx* T1 = buf + p.oT1;
   const int ml = chil * wl;
@@ -696,10 +697,11 @@ static __device__ __noinline__ double small_dots(const cplx* sQ, int nfit, const
   return ks.h[k].x;
 }
 
-// dev_expm_krylov for a solve that fits small_plan.
+// dev_expm_krylov for a solve that fits small_plan.  Its vectors lie in the
+// buffer or, past the first nfit, in global memory, so it is told nothing of
+// where sm points; the routines that read the buffer alone are.
 static __device__ __noinline__ int dev_expm_small(const HeffOp& h, const SmallPlan& p, cplx* x, double dt,
                                                   const KrylovCfg& kc, cplx* Q, long long qs, EngineSmem& sm) {
-  ASSUME_SHARED(&sm);
   cplx* buf = reinterpret_cast<cplx*>(&sm.u);
   cplx* sQ = buf + p.oQ;
   KrySmem& ks = sm.k;

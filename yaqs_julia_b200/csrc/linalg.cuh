@@ -659,65 +659,89 @@ static __device__ __forceinline__ bool jacobi_params(double al, double be, doubl
   return true;
 }
 
-// One Jacobi rotation pass over disjoint column pairs held in shared memory
-// (columns c of the stacked [B; X] block at sb + c*ld).  pairs(k) gives the
-// k-th pair as (i, j) local column indices, -1 to skip.  Each half-warp
-// takes one pair.
-template <class PairFn>
-static __device__ __forceinline__ void smem_rotate_round(cplx* sb, int ld, int q, int rows, int npairs, PairFn pairs,
-                                                  double tol, int* rot) {
-  ASSUME_SHARED(sb);
-  const int hl = ltid() & 15, hw = ltid() >> 4;
-  const unsigned mask = (ltid() & 16) ? 0xffff0000u : 0x0000ffffu;
-  for (int k = hw; k < npairs; k += NT / 16) {
-    int i, j;
-    pairs(k, i, j);
-    if (i < 0 || j < 0) continue;
-    cplx* bi = sb + (long long)ld * i;
-    cplx* bj = sb + (long long)ld * j;
-    double al = 0.0, be = 0.0, gx = 0.0, gy = 0.0;
-    for (int r = hl; r < q; r += 16) {
-      cplx x = bi[r], y = bj[r];
-      al += cabs2(x);
-      be += cabs2(y);
-      gx += x.x * y.x + x.y * y.y;
-      gy += x.x * y.y - x.y * y.x;
-    }
-    {  // the four trees over 16 lanes with the values halved twice: same pairs, 9 shuffles instead of 16
-      const int base = (ltid() & 31) & 16;
-      bool up = (hl & 8) != 0;
-      double k0 = up ? gx : al, k1 = up ? gy : be;
-      const double g0 = up ? al : gx, g1 = up ? be : gy;
-      k0 += __shfl_xor_sync(mask, g0, 8);
-      k1 += __shfl_xor_sync(mask, g1, 8);
-      up = (hl & 4) != 0;
-      double v = up ? k1 : k0;
-      const double g = up ? k0 : k1;
-      v += __shfl_xor_sync(mask, g, 4);
-      v += __shfl_xor_sync(mask, v, 2);
-      v += __shfl_xor_sync(mask, v, 1);
-      al = __shfl_sync(mask, v, base);
-      be = __shfl_sync(mask, v, base + 4);
-      gx = __shfl_sync(mask, v, base + 8);
-      gy = __shfl_sync(mask, v, base + 12);
-    }
-    double c;
-    cplx se, sec;
-    if (!jacobi_params(al, be, gx, gy, tol, c, se, sec)) continue;
-    if (hl == 0) atomicAdd(rot, 1);
-    for (int r = hl; r < rows; r += 16) {
-      cplx x = bi[r], y = bj[r];
-      bi[r] = csub(cscale(x, c), cmul(sec, y));
-      bj[r] = cadd(cmul(se, x), cscale(y, c));
-    }
+// Pair k of round t of such a block as columns i < j; false when it has none.
+static __device__ __forceinline__ bool block_pair(bool cross, int b, int n0, int n1, int joff, int t, int k, int& i,
+                                                  int& j) {
+  if (cross) {
+    i = k;
+    j = k + t < b ? k + t : k + t - b;
+    if (i >= n0 || j >= n1) return false;
+    j += joff;
+    return true;
   }
-  cta_sync();
+  // place p holds column ((p - 1 - t) mod (be2 - 1)) + 1, place 0 column 0
+  const int be2 = b + (b & 1), tb = be2 - 1 - k;
+  int x = k == 0 ? 0 : k - t, y = tb == 0 ? 0 : tb - t;
+  if (k != 0 && x < 1) x += be2 - 1;
+  if (tb != 0 && y < 1) y += be2 - 1;
+  i = min(x, y);
+  j = max(x, y);
+  return j < n0;
 }
 
-// All rounds of one diagonal block (cross = false: n0 columns, round-robin
-// over be2 places) or of one pair of blocks (cross: columns kk < n0 against
-// joff + (kk + t) mod b for t = 0 .. b-1), LP lanes a pair, RPL rows a lane.
-// For the runs that may reorder sums.  A round is one dependent chain, so its
+// All rounds of one diagonal block (cross = false: n0 columns, round-robin over
+// be2 places) or of one pair of blocks (cross: columns kk < n0 against
+// joff + (kk + t) mod b for t = 0 .. b-1) of columns held in shared memory, for
+// the runs that keep the order of their sums.  Each half-warp takes one pair a
+// round.  Out of line and with the columns as its only data pointer: it is told
+// that they are shared memory, which its caller, choosing between the staging
+// buffer and global memory elsewhere, must not be.
+static __device__ __noinline__ void kept_rounds(cplx* cols, int ld, int q, bool cross, int b, int n0, int n1, int joff,
+                                                double tol, int* rot) {
+  ASSUME_SHARED(cols);
+  const int hl = ltid() & 15, hw = ltid() >> 4;
+  const unsigned mask = (ltid() & 16) ? 0xffff0000u : 0x0000ffffu;
+  const int be2 = b + (b & 1);
+  const int rounds = cross ? b : be2 - 1, npairs = cross ? b : be2 / 2;
+#pragma unroll 1
+  for (int t = 0; t < rounds; ++t) {
+#pragma unroll 1
+    for (int k = hw; k < npairs; k += NT / 16) {
+      int i, j;
+      if (!block_pair(cross, b, n0, n1, joff, t, k, i, j)) continue;
+      cplx* bi = cols + ld * i;
+      cplx* bj = cols + ld * j;
+      double al = 0.0, be = 0.0, gx = 0.0, gy = 0.0;
+      for (int r = hl; r < q; r += 16) {
+        cplx x = bi[r], y = bj[r];
+        al += cabs2(x);
+        be += cabs2(y);
+        gx += x.x * y.x + x.y * y.y;
+        gy += x.x * y.y - x.y * y.x;
+      }
+      {  // the four trees over 16 lanes with the values halved twice: same pairs, 9 shuffles instead of 16
+        const int base = (ltid() & 31) & 16;
+        bool up = (hl & 8) != 0;
+        double k0 = up ? gx : al, k1 = up ? gy : be;
+        const double g0 = up ? al : gx, g1 = up ? be : gy;
+        k0 += __shfl_xor_sync(mask, g0, 8);
+        k1 += __shfl_xor_sync(mask, g1, 8);
+        up = (hl & 4) != 0;
+        double v = up ? k1 : k0;
+        const double g = up ? k0 : k1;
+        v += __shfl_xor_sync(mask, g, 4);
+        v += __shfl_xor_sync(mask, v, 2);
+        v += __shfl_xor_sync(mask, v, 1);
+        al = __shfl_sync(mask, v, base);
+        be = __shfl_sync(mask, v, base + 4);
+        gx = __shfl_sync(mask, v, base + 8);
+        gy = __shfl_sync(mask, v, base + 12);
+      }
+      double c;
+      cplx se, sec;
+      if (!jacobi_params(al, be, gx, gy, tol, c, se, sec)) continue;
+      if (hl == 0) *rot = 1;  // any rotation keeps the sweeps going
+      for (int r = hl; r < q; r += 16) {
+        cplx x = bi[r], y = bj[r];
+        bi[r] = csub(cscale(x, c), cmul(sec, y));
+        bj[r] = cadd(cmul(se, x), cscale(y, c));
+      }
+    }
+    cta_sync();
+  }
+}
+
+// The same for the runs that may reorder sums, LP lanes a pair, RPL rows a lane.  A round is one dependent chain, so its
 // length is its cost: both columns are loaded at once and stay in registers
 // for the update, the four sums are reduced together, and the rotation comes
 // from two reciprocal square roots: with R = sqrt(d^2 + 4 |g|^2),
@@ -737,21 +761,7 @@ static __device__ __noinline__ void jacobi_rounds(cplx* cols, int ld, int q, boo
 #pragma unroll 1
     for (int k = grp; k < npairs; k += NT / LP) {
       int i, j;
-      if (cross) {
-        i = k;
-        j = k + t < b ? k + t : k + t - b;
-        if (i >= n0 || j >= n1) continue;
-        j += joff;
-      } else {
-        // place p holds column ((p - 1 - t) mod (be2 - 1)) + 1, place 0 column 0
-        const int tb = be2 - 1 - k;
-        int x = k == 0 ? 0 : k - t, y = tb == 0 ? 0 : tb - t;
-        if (k != 0 && x < 1) x += be2 - 1;
-        if (tb != 0 && y < 1) y += be2 - 1;
-        i = min(x, y);
-        j = max(x, y);
-        if (j >= n0) continue;
-      }
+      if (!block_pair(cross, b, n0, n1, joff, t, k, i, j)) continue;
       cplx* bi = cols + ld * i;
       cplx* bj = cols + ld * j;
       cplx x[RPL], y[RPL];
@@ -918,7 +928,6 @@ static __device__ __noinline__ SvdResult dev_svd(const cplx* M, int m, int n, in
   const int b = svd_block_size(q, p);
   const int nb = (p + b - 1) / b;
   const int nbe = nb + (nb & 1);
-  const int be2 = b + (b & 1);
   for (int sweep = 0; sweep < JACOBI_MAX_SWEEPS; ++sweep) {
     if (tid == 0) ls.rot_count = 0;
     cta_sync();
@@ -926,21 +935,10 @@ static __device__ __noinline__ SvdResult dev_svd(const cplx* M, int m, int n, in
       const int c0 = I * b, nc = min(b, p - c0);
       if (!resident) svd_stage(sb, ld, w, q, c0, nc, 0, 0, false);
       cplx* cols = resident ? sb + ld * c0 : sb;
-      if (blocked) jacobi_block(cols, ld, q, false, b, nc, 0, 0, tol, &ls.rot_count);
-      for (int round = 0; !blocked && round < be2 - 1; ++round) {
-        smem_rotate_round(cols, ld, q, q, be2 / 2,
-                     [&](int pr, int& i, int& j) {
-                       // round-robin: place t holds column ((t - 1 - round) mod (be2 - 1)) + 1, place 0 column 0
-                       const int ta = pr, tb = be2 - 1 - pr;
-                       int a = ta == 0 ? 0 : ta - round, c = tb == 0 ? 0 : tb - round;
-                       if (ta != 0 && a < 1) a += be2 - 1;
-                       if (tb != 0 && c < 1) c += be2 - 1;
-                       i = min(a, c);
-                       j = max(a, c);
-                       if (j >= nc) i = j = -1;
-                     },
-                     tol, &ls.rot_count);
-      }
+      if (blocked)
+        jacobi_block(cols, ld, q, false, b, nc, 0, 0, tol, &ls.rot_count);
+      else
+        kept_rounds(cols, ld, q, false, b, nc, 0, 0, tol, &ls.rot_count);
       if (!resident) svd_stage(sb, ld, w, q, c0, nc, 0, 0, true);
     }
     for (int round = 0; round < nbe - 1; ++round) {
@@ -954,20 +952,10 @@ static __device__ __noinline__ SvdResult dev_svd(const cplx* M, int m, int n, in
         if (!resident) svd_stage(sb, ld, w, q, c0, n0, c1, n1, false);
         cplx* cols = resident ? sb + ld * c0 : sb;
         const int joff = resident ? c1 - c0 : n0;
-        if (blocked) jacobi_block(cols, ld, q, true, b, n0, n1, joff, tol, &ls.rot_count);
-        for (int t = 0; !blocked && t < b; ++t) {
-          smem_rotate_round(cols, ld, q, q, b,
-                       [&](int kk, int& i, int& j) {
-                         const int jj = kk + t < b ? kk + t : kk + t - b;
-                         if (kk >= n0 || jj >= n1) {
-                           i = j = -1;
-                         } else {
-                           i = kk;
-                           j = joff + jj;
-                         }
-                       },
-                       tol, &ls.rot_count);
-        }
+        if (blocked)
+          jacobi_block(cols, ld, q, true, b, n0, n1, joff, tol, &ls.rot_count);
+        else
+          kept_rounds(cols, ld, q, true, b, n0, n1, joff, tol, &ls.rot_count);
         if (!resident) svd_stage(sb, ld, w, q, c0, n0, c1, n1, true);
       }
     }
