@@ -5,10 +5,10 @@ non-unitary jump, after growth from a product state, in a chain with a
 symmetry), a one-site or dynamic sweep follows those directions, and another
 order of the sums moves the records by 1e-9 to 1e-5.  golden/kept_order.json
 holds the records of the general path (plain products, column QR, projections
-on the whole basis) on a B200 for four such problems; keeping its order gives
-the same states bit for bit, so only the records' own contractions may round
-differently.  Bound: 1e-12, about 100 roundings of a contraction over 128
-values.
+on the whole basis, full environments) on a B200 for four such problems; its
+order gives the same states.  Bound: 1e-12, about 100 roundings of a
+contraction over 128 values.  A fifth problem has records that a symmetry makes
+zero: they are nothing but rounding and are equal only if every sum is.
 """
 import json
 import os
@@ -61,6 +61,12 @@ def _problem(name):
     if name == "padded_start":
         return _desc(api.MPS(10, state="Neel", pad=16), api.init_general_hamiltonian(10, 1, 1, 1, 0, 0, 0.5),
                      _procs("lowering", range(1, 11)), 6, 4, 16, "1site", seed=3)
+    if name == "zero_by_symmetry":
+        L = 3
+        obs = [api.Observable(f"Z{i}", api.Z, i) for i in range(1, L + 1)]
+        cfg = api.TimeEvolutionConfig(obs, 0.8, dt=0.1, num_traj=8, max_bond_dim=16, order=1)
+        return api.Descriptors(api.MPS(L, state="x+"), api.init_ising(L, 1.0, 0.7), cfg,
+                               api.NoiseModel(_procs("pauli_z", range(1, L + 1)), L), seed=4)
     psi, H = _evolved_xy()
     return _desc(psi, H, _procs("pauli_z", range(1, 13)), 12, 4, 16, "1site", seed=2)
 
@@ -68,11 +74,22 @@ def _problem(name):
 NAMES = ["jump_right_of_the_middle", "dynamic_from_a_product", "padded_start", "evolved_symmetric_start"]
 
 
+def _golden(name):
+    return np.array(json.load(open(GOLDEN))[name])
+
+
 @pytest.mark.parametrize("name", NAMES)
 def test_records_of_the_general_path(name):
     res = api.run_descriptors(_problem(name))
-    ref = np.array(json.load(open(GOLDEN))[name])
+    ref = _golden(name)
     assert res.trajectories.shape == ref.shape
     assert np.abs(res.trajectories - ref).max() <= 1e-12
     if name == "jump_right_of_the_middle":
         assert res.stats["jumps"] >= 2
+
+
+def test_records_of_pure_rounding():
+    res = api.run_descriptors(_problem("zero_by_symmetry"))
+    ref = _golden("zero_by_symmetry")
+    assert 0 < np.abs(ref).max() < 1e-14
+    assert np.array_equal(res.trajectories, ref)

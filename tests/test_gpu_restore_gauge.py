@@ -1,14 +1,16 @@
 """Restoring checkpoints: the look at the restored gauge (needs a B200).
 
-A restored trajectory in another gauge takes the run's records off the
-canonical form; restoring a canonical one brings them back, bit for bit; and
-the look costs no more than the copies beside it.
+Mixed runs and circuits read records from the canonical form.  A restored
+trajectory in another gauge takes the run's records off it; restoring a
+canonical one brings them back, bit for bit; and the look costs no more than
+the copies beside it.
 """
 import time
 
 import numpy as np
 import pytest
 
+from yaqs_julia_b200 import _abi as A
 from yaqs_julia_b200 import api
 
 pytestmark = pytest.mark.gpu
@@ -20,7 +22,8 @@ def _desc(L, chi, nt, steps, start):
     nm = api.NoiseModel([{"name": "pauli_z", "sites": [i], "strength": 0.2} for i in range(1, L + 1)], L)
     psi = api.random_mps(L, chi, seed=2) if start == "random" else api.MPS(L, state="Neel")
     return api.Descriptors(psi, api.init_general_hamiltonian(L, 1, 1, 1, 0, 0, 0.4), cfg, nm, seed=6,
-                           tdvp_mode=api.TDVP_MODES["1site" if start == "random" else "2site"])
+                           tdvp_mode=api.TDVP_MODES["1site" if start == "random" else "2site"],
+                           precision=A.YAQS_PREC_MIXED)
 
 
 def _skew(psi, b):

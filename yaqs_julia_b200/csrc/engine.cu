@@ -38,8 +38,7 @@ __global__ void __launch_bounds__(NT, 2) tjm_step_kernel(const DevParams P, int 
 
 // Digital TJM: position 0 prepares every trajectory, position l >= 1 applies
 // layer l-1 of the circuit (run_digital_tjm, DigitalTJM.jl:363-450).
-__global__ void __launch_bounds__(NT, 2) digital_step_kernel(const DevParams P,
-                                                             const DigParams D, int first,
+__global__ void __launch_bounds__(NT, 2) digital_step_kernel(const DevParams P, const DigParams D, int first,
                                                              int count) {
   extern __shared__ __align__(16) unsigned char smraw[];
   CtaSmem& sm = *reinterpret_cast<CtaSmem*>(align_smem_1024(smraw));
@@ -930,8 +929,10 @@ static int setup_run(yaqs_ctx* ctx, yaqs_run* run, const std::vector<int>& cap, 
     }
     // sweeps, splits and normalisations leave canonical states; what may not:
     // long-range jumps, non-unitary 1-qubit gates (digital_begin) and states
-    // put in from outside (yaqs_run_restore, looked over by check_restored)
-    P.canonical = P.has_lr ? 0 : 1;
+    // put in from outside (yaqs_run_restore, looked over by check_restored).
+    // FP64 analog records keep their sums' order like the sweeps: a record
+    // that a symmetry makes zero is nothing but its rounding.
+    P.canonical = P.has_lr || !P.blocked ? 0 : 1;
   }
 
   // initial state arena (compact tensors at the site slots)
