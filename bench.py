@@ -58,14 +58,11 @@ sys.path.insert(0, ROOT)
 from yaqs_julia_b200 import _abi as A  # noqa: E402
 from yaqs_julia_b200 import api  # noqa: E402
 
-# the same for the digital workload: (L, trajectories, timed layers) -> bytes;
-# empty: no capture of the current kernels
-DIG_TIMED_TRAFFIC = {}
-
 METRIC = "TJM trajectory-steps/s (L=30 Heisenberg, chi=64, 1024 trajectories) vs plain FP64 GPU"
 # DRAM read + write bytes per trajectory-step of the trajectory kernel, from
 # one small-case ncu capture per configuration: (precision, tdvp, L, chi) -> bytes
-TRAFFIC_PER_TRAJ_STEP = {}  # no capture of the current kernels
+TRAFFIC_PER_TRAJ_STEP = {("mixed", "dynamic", 30, 64): (199.835e9 + 104.335e9) / 148,
+                         ("fp64", "dynamic", 30, 64): (427.882e9 + 242.090e9) / 148}
 TDVP_NAMES = {"dynamic": A.YAQS_TDVP_DYNAMIC, "2site": A.YAQS_TDVP_2SITE, "1site": A.YAQS_TDVP_1SITE}
 TDVP = [A.YAQS_TDVP_DYNAMIC]  # set from --tdvp
 TDVP_DESC = {"dynamic": "1-site TDVP with 2-site growth (local dynamic TDVP)", "2site": "2-site TDVP",
@@ -436,10 +433,7 @@ def run_digital(args):
                 "gpu_launches": 1,  # one digital_step_kernel launch covers the timed layers
                 "roofline": {"bound": "tensor", "achieved": achieved, "peak": pk.value, "unit": "TFLOP/s",
                              "frac": achieved / pk.value if pk.value else None,
-                             "traffic": DIG_TIMED_TRAFFIC.get((L, nt, K)),
-                             "traffic_source": "ncu dram__bytes_read.sum + dram__bytes_write.sum of the timed "
-                                               "launch (profiles/digital_step_kernel_L40_ising_512traj.md); "
-                                               "null for configurations not captured",
+                             "traffic": None,  # not captured; the working set stays in L2
                              "kernel": "digital_step_kernel",
                              "peak_source": "measured FP64 DFMA probe (yaqs_fp64_peak) in this run",
                              "achieved_counts": "nominal TEBD work: theta merge GEMM + 4x4 gate + SVD as "
@@ -778,8 +772,8 @@ def run_ours(args):
                      "traffic_source": "DRAM read+write bytes per trajectory-step from a one-launch ncu capture of "
                                        "148 trajectories of the same configuration (profiles/tjm_step_kernels_L30_"
                                        "chi64_148traj_traffic.md), scaled by the trajectory-steps of the timed launch "
-                                       "(a lower bound: the full run keeps twice the slots in L2); null when not "
-                                       "captured",
+                                       "(a lower bound: the full run keeps twice the slots in L2)"
+                     if tt else None,
                      "traffic_gbs": tt / (main["dev_ms"] / 1e3) / 1e9 if tt else None,
                      "hbm_frac": tt / (main["dev_ms"] / 1e3) / 1e9 / peaks["hbm_gbs"] if tt else None})
         line = {"metric": METRIC, "value": value, "unit": UNIT, "n_gpus": ws, "steps": K,

@@ -15,8 +15,7 @@
 #include "program.cuh"
 #include "engine_dg.h"
 
-__global__ void __launch_bounds__(NT, 3) digital_step_kernel_dg(const DevParams P,
-                                                             const DigParams D, int first,
+__global__ void __launch_bounds__(NT, 3) digital_step_kernel_dg(const DevParams P, const DigParams D, int first,
                                                                 int count) {
   extern __shared__ __align__(16) unsigned char smraw[];
   CtaSmem& sm = *reinterpret_cast<CtaSmem*>(align_smem_1024(smraw));

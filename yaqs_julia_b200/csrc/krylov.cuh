@@ -4,12 +4,18 @@
 //   T1[a,m,p,c]   = sum_k L[a,m,k] x[k,p,c]                    (GEMM)
 //   T2[a,p',m',c] = sum_{m,p} W[m,p',p,m'] T1[a,m,p,c]         (sparse MPO apply)
 //   y[a,p',b]     = sum_{m',c} T2[a,p',m',c] R[b,m',c]         (GEMM)
+// In mixed runs next to isometric sites the identity channels are taken out
+// (HPlan, tsgemm.cuh).
+//
 // dev_expm_krylov restates expm_krylov (Algorithms.jl:144-187) / KrylovKit
 // exponentiate: Lanczos with classical Gram-Schmidt against the whole basis,
 // refined by a second pass when the first kept less than 1/sqrt(2) of the
 // norm (DGKS), stopping at krylov_dim, at breakdown (beta <= |dt| tol), or
 // once prod(beta_i |dt|)/k! <= exit_tol; the small tridiagonal exponential
-// is taken on one warp by Taylor series over substeps of norm <= 1/2.
+// is taken on one warp by Taylor series over substeps of norm <= 1/2.  Three
+// forms: the general one, dev_expm_small (at most 256 values, in shared memory,
+// the same bits), and dev_expm_predicted for circuits and mixed runs, which
+// projects what the three-term recurrence leaves.
 #pragma once
 #include "common.cuh"
 #include "gemm_tf32.cuh"
