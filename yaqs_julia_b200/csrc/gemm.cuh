@@ -8,22 +8,23 @@
 // written as one such GEMM over the reference's column-major layouts.
 //
 // Tiling: 64 x GBN_EFF output tiles (64 x 64 for a 256-thread program, 64 x
-// 32 for a 128-thread one), K slices staged in shared memory by cp.async
-// through a ring (one barrier per slice, zero-filled outside the matrix): two
-// stages of 16 for long sums, where the work of a slice has to outweigh its
-// barrier (L = 30, chi 64, FP64: 1158 ms against 1246 with 8-deep slices),
-// four of 8 for sums shorter than 32, which 16-deep ones would pad (digital
-// L = 40: 766 against 799 ms).  The 8 x 8 blocks of a tile are dealt to the warps in
-// rows and columns (warp (wm, wn) owns block rows wm + 2 i and block columns
-// wn + NW/2 j), so a tile that is only partly inside the matrix still spreads
-// over all warps; blocks outside it issue no MMA and stage no data.
+// 32 for a 128-thread one), K slices of 16 staged in shared memory by cp.async
+// through a ring of two (one barrier per slice, zero-filled outside the
+// matrix): the work of a slice has to outweigh its barrier (L = 30, chi 64,
+// FP64: 1525 ms against 1799 with a ring of four 8-deep slices; sums shorter
+// than 32 take as long either way).  The 8 x 8 blocks of a tile are dealt to the
+// warps in rows and columns (warp (wm, wn) owns block rows wm + 2 i and block
+// columns wn + NW/2 j), so a tile that is only partly inside the matrix still
+// spreads over all warps; blocks outside it issue no MMA and stage no data.
 // Conjugation is applied when a slice is read from shared memory.
 #pragma once
 #include "common.cuh"
 
 #define GBM 64
 #define GBN 64
-#define GROWS 32  // k rows in the ring: stages x slice depth
+#define GBK 16
+#define GSTAGES 2
+#define GROWS (GSTAGES * GBK)  // k rows in the ring
 // Output columns of one CTA tile: the warps form a 2 x NW/2 grid.
 #define GBN_EFF (16 * (NW / 2))
 static_assert(NW % 2 == 0 && GBN_EFF <= GBN, "the GEMM needs an even warp count of at most 8");
@@ -106,10 +107,8 @@ static __device__ __forceinline__ double flip_sign(double x, unsigned mask) {
 // 64 x 64 tiles of mostly padding for small operands, L = 16 at chi 128 went
 // from 600 to 550 ms and L = 6 at chi 16 from 528 to 446 ms, with the same
 // bits.
-template <int GBK>
-static __device__ __noinline__ void cta_gemm_k(const GemmArgs g, GemmSmem& sm) {
+static __device__ __noinline__ void cta_gemm_tiled(const GemmArgs g, GemmSmem& sm) {
   ProfScope prof_scope_(PF_GEMM);
-  constexpr int GSTAGES = GROWS / GBK;
   ASSUME_SHARED(&sm);
   const int tid = ltid();
   const int lane = tid & 31, wid = tid >> 5;
@@ -285,8 +284,6 @@ static __device__ __noinline__ void cta_gemm_direct(const GemmArgs g) {
 static __device__ __forceinline__ void cta_gemm(const GemmArgs g, GemmSmem& sm) {
   if (g.K <= GDIRECT_K && ((g.M + 7) >> 3) * ((g.N + 7) >> 3) <= 2 * NW)
     cta_gemm_direct(g);
-  else if (g.K >= 32)
-    cta_gemm_k<16>(g, sm);
   else
-    cta_gemm_k<8>(g, sm);
+    cta_gemm_tiled(g, sm);
 }
