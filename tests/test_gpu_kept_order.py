@@ -1,14 +1,15 @@
-"""FP64 analog runs keep the order of their sums (needs a B200).
+"""FP64 TDVP sweeps keep the order of their sums (needs a B200).
 
 Where a bond's basis holds directions that rounding decides (after a
 non-unitary jump, after growth from a product state, in a chain with a
-symmetry), a one-site or dynamic sweep follows those directions, and another
-order of the sums moves the records by 1e-9 to 1e-5.  golden/kept_order.json
-holds the records of the general path (plain products, column QR, projections
-on the whole basis, full environments) on a B200 for four such problems; its
-order gives the same states.  Bound: 1e-12, about 100 roundings of a
-contraction over 128 values.  A fifth problem has records that a symmetry makes
-zero: they are nothing but rounding and are equal only if every sum is.
+symmetry), a sweep follows those directions, and another order of the sums
+moves the records by 1e-9 to 1e-4.  golden/kept_order.json holds the records
+of the general path (plain products, column QR, projections on the whole
+basis, full environments) on a B200 for five such problems, one of them a
+circuit of TDVP windows; its order gives the same states.  Bound: 1e-12, about
+100 roundings of a contraction over 128 values.  One more problem has records
+that a symmetry makes zero: they are nothing but rounding and are equal only
+if every sum is.
 """
 import json
 import os
@@ -67,11 +68,29 @@ def _problem(name):
         cfg = api.TimeEvolutionConfig(obs, 0.8, dt=0.1, num_traj=8, max_bond_dim=16, order=1)
         return api.Descriptors(api.MPS(L, state="x+"), api.init_ising(L, 1.0, 0.7), cfg,
                                api.NoiseModel(_procs("pauli_z", range(1, L + 1)), L), seed=4)
+    if name == "tdvp_windows":
+        L, c = 12, api.DigitalCircuit(12)
+        for _ in range(5):
+            for i in list(range(1, L, 2)) + list(range(2, L, 2)):
+                c.add_gate(api.RzzGate(0.1), [i, i + 1])
+            for i in range(1, L + 1):
+                c.add_gate(api.Rx(0.1), [i])
+            c.add_gate(api.Barrier(), [])
+        obs = [api.Observable(f"{n}{i}", op, i) for i in range(1, L + 1) for n, op in (("Z", api.Z), ("X", api.X))]
+        cfg = api.TimeEvolutionConfig(obs, 4.0, dt=1.0, num_traj=12, max_bond_dim=64, truncation_threshold=1e-6)
+        nm = api.NoiseModel([{"name": n, "sites": [i], "strength": 0.01} for i in range(1, L + 1)
+                             for n in ("pauli_x", "pauli_y", "pauli_z")], L)
+        return api.CircuitDescriptors(api.MPS(L, state="x+"), c, cfg, nm, seed=4, local_method="tdvp",
+                                      long_range_method="tdvp")
     psi, H = _evolved_xy()
     return _desc(psi, H, _procs("pauli_z", range(1, 13)), 12, 4, 16, "1site", seed=2)
 
 
-NAMES = ["jump_right_of_the_middle", "dynamic_from_a_product", "padded_start", "evolved_symmetric_start"]
+NAMES = ["jump_right_of_the_middle", "dynamic_from_a_product", "padded_start", "evolved_symmetric_start", "tdvp_windows"]
+
+
+def _run(d):
+    return (api.run_circuit_descriptors if isinstance(d, api.CircuitDescriptors) else api.run_descriptors)(d)
 
 
 def _golden(name):
@@ -80,7 +99,7 @@ def _golden(name):
 
 @pytest.mark.parametrize("name", NAMES)
 def test_records_of_the_general_path(name):
-    res = api.run_descriptors(_problem(name))
+    res = _run(_problem(name))
     ref = _golden(name)
     assert res.trajectories.shape == ref.shape
     assert np.abs(res.trajectories - ref).max() <= 1e-12
@@ -89,7 +108,7 @@ def test_records_of_the_general_path(name):
 
 
 def test_records_of_pure_rounding():
-    res = api.run_descriptors(_problem("zero_by_symmetry"))
+    res = _run(_problem("zero_by_symmetry"))
     ref = _golden("zero_by_symmetry")
     assert 0 < np.abs(ref).max() < 1e-14
     assert np.array_equal(res.trajectories, ref)

@@ -13,9 +13,9 @@
 // norm (DGKS), stopping at krylov_dim, at breakdown (beta <= |dt| tol), or
 // once prod(beta_i |dt|)/k! <= exit_tol; the small tridiagonal exponential
 // is taken on one warp by Taylor series over substeps of norm <= 1/2.  Three
-// forms: the general one, dev_expm_small (at most 256 values, in shared memory,
-// the same bits), and dev_expm_predicted for circuits and mixed runs, which
-// projects what the three-term recurrence leaves.
+// forms: the general one, dev_expm_small (at most one value a thread, in shared
+// memory, the same bits), and dev_expm_predicted for mixed runs, which projects
+// what the three-term recurrence leaves.
 #pragma once
 #include "common.cuh"
 #include "gemm_tf32.cuh"
@@ -422,7 +422,7 @@ static __device__ __noinline__ void dev_tridiag_expm(int m, double dt, KrySmem& 
   if (on) ks.y[j] = v;
 }
 
-// The roundings of the sums that FP64 analog runs keep (DevParams::blocked),
+// The roundings of the sums that FP64 sweeps keep (DevParams::blocked),
 // spelled out: where a product meets a sum the compiler fuses one or the other
 // factor as the code around it falls, and the last bit follows.
 // v - c a
@@ -546,11 +546,11 @@ static __device__ __noinline__ double basis_combine(const cplx* Q, long long qs,
 // before it waits for anything else.
 // Every sum is formed in the general path's order (four-deep MMA steps from
 // k = 0, the same reduction trees), so both give the same bits, which FP64
-// analog runs need (DevParams::blocked).
-// SMALL_N is one value per thread; wider solves fill the tiles of the general
-// path.  Measured with the sweep on L = 6 Ising, chi 16, 200 trajectories, 51
+// sweeps need (DevParams::blocked).
+// SMALL_N is one value per thread, up to which the general path adds a thread's
+// values in this order too; wider solves fill its tiles.  Measured with the sweep on L = 6 Ising, chi 16, 200 trajectories, 51
 // time indices: 445 ms with the general path alone, 180 ms with this one.
-#define SMALL_N 256
+#define SMALL_N NT
 #define SMALL_MIN_VECS 4  // Krylov vectors that have to fit beside the operands
 
 struct SmallPlan {

@@ -246,7 +246,7 @@ static __device__ __forceinline__ void dev_qr_extract_r(const cplx* H, int m, in
 // loaded once a panel into the registers of one warp, which applies all
 // reflectors of the panel to it without a barrier.  Q is formed the same way
 // from the last panel to the first.  The sums run in another order than the
-// column loop's, so it serves circuits and mixed runs (DevParams::blocked).
+// column loop's, so it serves TEBD circuits and mixed runs (DevParams::blocked).
 #define QR_PANEL 16
 #define QR_PANEL_MAX_ROWS 256
 

@@ -88,7 +88,7 @@ struct DevParams {
   // idx are the indices that belong to site i, ascending.
   const int *p0_off, *p0_idx, *p1_off, *p1_idx, *ob_off, *ob_idx;
   int canonical;   // 1-site records are read from the mixed canonical form around the centre
-  int blocked;     // may reorder sums (circuits, mixed): panel QR, short Jacobi rounds, predicted projections
+  int blocked;     // may reorder sums (TEBD, mixed): panel QR, short Jacobi rounds, predicted projections
   int scalar_all;  // every process is a scalar dissipator (pauli_name)
   int has_lr;      // some process is long-range
   const cplx* psi0;  // arena layout, compact tensors
